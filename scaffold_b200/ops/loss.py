@@ -29,7 +29,8 @@ from . import _lib
 _P = C.c_void_p
 _lib.register("sb_loss_blocks", [C.c_longlong], C.c_int)
 _lib.register("sb_loss_sums", [_P, _P, C.c_int, _P, _P, _P, C.c_int, C.c_longlong, C.c_int, C.c_int, C.c_int, _P, _P])
-_lib.register("sb_loss_grad", [_P, _P, C.c_int, _P, _P, _P, _P, C.c_int, C.c_longlong, C.c_int, C.c_int, _P, _P])
+_lib.register("sb_loss_head", [_P, C.c_int, C.c_int, _P, _P, _P, _P, _P])
+_lib.register("sb_loss_grad", [_P, _P, C.c_int, _P, _P, _P, _P, _P, C.c_int, C.c_longlong, C.c_int, C.c_int, _P, _P])
 
 FUSED_MAX_CLASSES = 32  # widest head of csrc/loss.cu (LOSS_MAXC); wider heads take the PyTorch formula
 
@@ -131,41 +132,30 @@ class _FusedLossFn(torch.autograd.Function):
         if spatial is not None and spatial.size > 1:
             spatial.all_reduce_sum(sums)
         n = sums.shape[0]
-        P, Q, I = sums[:, :c], sums[:, c:2 * c], sums[:, 2 * c:3 * c]
-        num, den = sums[:, 3 * c].sum(), sums[:, 3 * c + 1].sum()
-        den = den.clamp_min(torch.finfo(torch.float32).eps)
-        inter2, sets = 2.0 * I, P + Q
-        empty = sets == 0
-        U = torch.where(empty, inter2, sets)
-        dice = (inter2 + EPS) / (U + EPS)
-        fg = dice[:, 1:].mean()
-        ce = num / den
-        # d loss / d p_c(v) = alpha * [y = c] + beta  (foreground classes only)
-        m = float(n * (c - 1))
-        alpha = -2.0 / (m * (U + EPS))
-        beta = (inter2 + EPS) / (m * (U + EPS) ** 2)
-        alpha = torch.where(empty, torch.zeros_like(alpha), alpha)
-        beta = torch.where(empty, torch.zeros_like(beta), beta)
-        alpha[:, 0] = 0
-        beta[:, 0] = 0
-        ctx.save_for_backward(logits_vm, labels, torch.stack([alpha, beta], 1).contiguous(), den.reshape(1))
+        dev = sums.device
+        out = torch.empty(3, dtype=torch.float32, device=dev)  # loss, ce, fg
+        coef = torch.empty((n, 2, c), dtype=torch.float32, device=dev)
+        den = torch.empty(1, dtype=torch.float32, device=dev)
+        _lib.check(_lib.lib().sb_loss_head(sums.data_ptr(), n, c, None, out.data_ptr(), coef.data_ptr(),
+                                           den.data_ptr(), _lib.stream_ptr()), "sb_loss_head")
+        ctx.save_for_backward(logits_vm, labels, coef, den)
         ctx.cw, ctx.c = cw, c
         ctx.mark_non_differentiable(labels)
-        return ce + (1.0 - fg), ce, fg
+        return out[0], out[1], out[2]
 
     @staticmethod
     def backward(ctx, g, _gce, _gfg):
         logits_vm, labels, coef, den = ctx.saved_tensors
         n, d, h, w, cp = logits_vm.shape
-        coef = (coef * g).contiguous()
-        kce = (g / den).reshape(1).float().contiguous()
+        g = g.float().contiguous()
         dl = torch.empty_like(logits_vm)
         lab = labels if labels.dtype in _LABEL_KIND else labels.long()
         lab = lab.contiguous()
         _lib.check(_lib.lib().sb_loss_grad(logits_vm.data_ptr(), lab.data_ptr(), _LABEL_KIND[lab.dtype],
-                                           _lib.ptr(ctx.cw), coef.data_ptr(), kce.data_ptr(), dl.data_ptr(), n,
-                                           d * h * w, ctx.c, cp, _lib.status_tensor(logits_vm.device).data_ptr(),
-                                           _lib.stream_ptr()), "sb_loss_grad")
+                                           _lib.ptr(ctx.cw), coef.data_ptr(), g.data_ptr(), den.data_ptr(),
+                                           dl.data_ptr(), n, d * h * w, ctx.c, cp,
+                                           _lib.status_tensor(logits_vm.device).data_ptr(), _lib.stream_ptr()),
+                   "sb_loss_grad")
         return dl, None, None, None, None
 
 
@@ -183,8 +173,10 @@ def hard_dice_fused(logits_vm: torch.Tensor, labels: torch.Tensor, n_classes: in
     sums = _sums(logits_vm.contiguous(), labels, c, None, True)
     if spatial is not None and spatial.size > 1:
         spatial.all_reduce_sum(sums)
-    P, Q, I = sums[:, :c], sums[:, c:2 * c], sums[:, 2 * c:3 * c]
-    return dice_from_sums(2.0 * I, P + Q)
+    dice = torch.empty((sums.shape[0], c), dtype=torch.float32, device=sums.device)
+    _lib.check(_lib.lib().sb_loss_head(sums.data_ptr(), sums.shape[0], c, dice.data_ptr(), None, None, None,
+                                       _lib.stream_ptr()), "sb_loss_head")
+    return dice
 
 
 def hard_dice_reference(logits: torch.Tensor, labels: torch.Tensor, n_classes: int, spatial=None) -> torch.Tensor:
