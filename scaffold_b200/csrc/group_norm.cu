@@ -88,40 +88,69 @@ __device__ __forceinline__ void chan_merge(float& n_a, float& mean_a, float& m2_
 }
 
 
-// One warp collapses the `nsplit` partials of (n, g) with a fixed merge tree (lane-strided, then xor
-// shuffles merging the lower lane first): the separate finalize kernel and the last-block tail of the
-// statistics kernel run exactly this, so both give the same bits. Loads bypass L1 (the partials may
-// have been written by other SMs during this launch).
+// Pooled (count, mean, M2) of a set of partials as three plain sums in double: count, count * mean and
+// M2 + count * mean^2. No division stands in the chain (Chan's merge has one per partial), the loads of a thread are
+// independent, and double leaves nothing of the cancellation in M2 = S2 - S1^2 / count at fp32.
+struct StatSums {
+  double n, s1, s2;
+};
+__device__ __forceinline__ void stat_add(StatSums& a, float n, float mean, float m2) {
+  const double nm = (double)n * (double)mean;
+  a.n += (double)n;
+  a.s1 += nm;
+  a.s2 += (double)m2 + nm * (double)mean;
+}
+__device__ __forceinline__ void stat_store(float* dst, const StatSums& a) {
+  const double mean = a.n > 0.0 ? a.s1 / a.n : 0.0;
+  const double m2 = a.s2 - a.s1 * mean;
+  dst[0] = (float)a.n;
+  dst[1] = (float)mean;
+  dst[2] = (float)(m2 > 0.0 ? m2 : 0.0);
+}
+// The sums of partials first, first + step, ... of (n, g) (`base`: partial 0), eight partials in flight. Loads bypass
+// L1 (the partials may have been written by other SMs during this launch).
+__device__ __forceinline__ StatSums stat_walk(const float* __restrict__ base, int G, int first, int step, int nsplit) {
+  StatSums a{0.0, 0.0, 0.0};
+  int s = first;
+  for (; s + 7 * step < nsplit; s += 8 * step) {
+    float e[8][3];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const float* q = base + (long long)(s + u * step) * G * 3;
+      e[u][0] = __ldcg(q); e[u][1] = __ldcg(q + 1); e[u][2] = __ldcg(q + 2);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) stat_add(a, e[u][0], e[u][1], e[u][2]);
+  }
+  for (; s < nsplit; s += step) {
+    const float* q = base + (long long)s * G * 3;
+    stat_add(a, __ldcg(q), __ldcg(q + 1), __ldcg(q + 2));
+  }
+  return a;
+}
+__device__ __forceinline__ StatSums stat_warp_sum(StatSums a) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a.n += __shfl_xor_sync(0xffffffffu, a.n, o);
+    a.s1 += __shfl_xor_sync(0xffffffffu, a.s1, o);
+    a.s2 += __shfl_xor_sync(0xffffffffu, a.s2, o);
+  }
+  return a;
+}
+
+// One warp collapses the `nsplit` partials of (n, g) in a fixed order (lane-strided, then xor shuffles): the separate
+// finalize kernel and the last-block tail of the statistics kernel run exactly this, so both give the same bits.
+// 592 partials, kernel time: 13 us as a chain of Chan merges (one L2 latency and one division each).
 __device__ __forceinline__ void stats_collapse_warp(const float* __restrict__ part, float* __restrict__ fin, int G,
                                                     int nsplit, int n, int g, int lane) {
-  float gn = 0.f, gm = 0.f, g2 = 0.f;
-  for (int s = lane; s < nsplit; s += 32) {
-    const float* e = part + (((long long)n * nsplit + s) * G + g) * 3;
-    chan_merge(gn, gm, g2, __ldcg(e), __ldcg(e + 1), __ldcg(e + 2));
-  }
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const float on = __shfl_xor_sync(0xffffffffu, gn, o);
-    const float om = __shfl_xor_sync(0xffffffffu, gm, o);
-    const float o2 = __shfl_xor_sync(0xffffffffu, g2, o);
-    // merge (lower lane, higher lane) in that order on both sides: bitwise identical results
-    if (lane & o) {
-      float an = on, am = om, a2 = o2;
-      chan_merge(an, am, a2, gn, gm, g2);
-      gn = an; gm = am; g2 = a2;
-    } else {
-      chan_merge(gn, gm, g2, on, om, o2);
-    }
-  }
-  if (lane == 0) {
-    float* dst = fin + ((long long)n * G + g) * 3;
-    dst[0] = gn; dst[1] = gm; dst[2] = g2;
-  }
+  const StatSums a = stat_warp_sum(stat_walk(part + ((long long)n * nsplit * G + g) * 3, G, lane, 32, nsplit));
+  if (lane == 0) stat_store(fin + ((long long)n * G + g) * 3, a);
 }
 
 __device__ __forceinline__ void bwd_collapse_warp(const float* __restrict__ part, float* __restrict__ fin, int C,
                                                   int nsplit, int n, int c, int lane) {
   float a = 0.f, b = 0.f;
+#pragma unroll 8
   for (int s = lane; s < nsplit; s += 32) {
     const float2 e = __ldcg(reinterpret_cast<const float2*>(part + (((long long)n * nsplit + s) * C + c) * 2));
     a += e.x;
@@ -530,45 +559,39 @@ __global__ void __launch_bounds__(GN_THREADS) gn_stats_finalize_kernel(const flo
 }
 
 // The same collapse for MANY partials per (n, g) (the per-warp partials a convolution's epilogue leaves: up to
-// 16K per sample): one block per (n, g); thread t merges partials t, t + 256, ... in order, then a fixed
-// shared-memory tree merges the 256 results (lower index first), so the result is deterministic.
-__global__ void __launch_bounds__(GN_THREADS) gn_stats_finalize_wide_kernel(const float* __restrict__ part,
-                                                                            float* __restrict__ fin, int N, int G,
-                                                                            int nsplit) {
-  __shared__ float s_n[GN_THREADS], s_m[GN_THREADS], s_2[GN_THREADS];
-  const int n = blockIdx.x / G, g = blockIdx.x % G;
-  float gn = 0.f, gm = 0.f, g2 = 0.f;
-  const float* base = part + ((long long)n * nsplit * G + g) * 3;
-  int s = threadIdx.x;
-  // four independent loads in flight per thread; merged in index order
-  for (; s + 3 * GN_THREADS < nsplit; s += 4 * GN_THREADS) {
-    float e[4][3];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const float* q = base + (long long)(s + u * GN_THREADS) * G * 3;
-      e[u][0] = q[0]; e[u][1] = q[1]; e[u][2] = q[2];
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) chan_merge(gn, gm, g2, e[u][0], e[u][1], e[u][2]);
-  }
-  for (; s < nsplit; s += GN_THREADS) {
-    const float* q = base + (long long)s * G * 3;
-    chan_merge(gn, gm, g2, q[0], q[1], q[2]);
-  }
-  s_n[threadIdx.x] = gn; s_m[threadIdx.x] = gm; s_2[threadIdx.x] = g2;
+// 16K per sample). Bound: L2 latency and the sectors around 12-byte entries, so a cluster of eight CTAs shares one
+// (n, g): thread t of CTA r adds the partials r * 256 + t, + 2048, ..., each CTA adds its warps in order, and CTA 0
+// reads the eight sums over distributed shared memory in rank order. 16K partials of 2 x 8 groups, call: 17.9 us with
+// one CTA per (n, g), 10.4 us (the cost of the call itself) with the cluster.
+constexpr int GN_WIDE_CLUSTER = 8;
+__global__ void __cluster_dims__(GN_WIDE_CLUSTER, 1, 1) __launch_bounds__(GN_THREADS)
+    gn_stats_finalize_wide_kernel(const float* __restrict__ part, float* __restrict__ fin, int N, int G, int nsplit) {
+  __shared__ double s_w[GN_THREADS / 32][3];
+  __shared__ double s_cta[3];
+  const int out = blockIdx.x / GN_WIDE_CLUSTER, rank = blockIdx.x % GN_WIDE_CLUSTER;
+  const int n = out / G, g = out % G, warp = threadIdx.x >> 5;
+  const StatSums a = stat_warp_sum(stat_walk(part + ((long long)n * nsplit * G + g) * 3, G,
+                                             rank * GN_THREADS + threadIdx.x, GN_WIDE_CLUSTER * GN_THREADS, nsplit));
+  if ((threadIdx.x & 31) == 0) { s_w[warp][0] = a.n; s_w[warp][1] = a.s1; s_w[warp][2] = a.s2; }
   __syncthreads();
-  for (int o = GN_THREADS / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      float an = s_n[threadIdx.x], am = s_m[threadIdx.x], a2 = s_2[threadIdx.x];
-      chan_merge(an, am, a2, s_n[threadIdx.x + o], s_m[threadIdx.x + o], s_2[threadIdx.x + o]);
-      s_n[threadIdx.x] = an; s_m[threadIdx.x] = am; s_2[threadIdx.x] = a2;
+  if (threadIdx.x < 3) {
+    double t = 0.0;
+    for (int w = 0; w < GN_THREADS / 32; ++w) t += s_w[w][threadIdx.x];
+    s_cta[threadIdx.x] = t;
+  }
+  __syncthreads();
+  cluster_sync_all();
+  if (rank == 0 && threadIdx.x == 0) {
+    StatSums t{0.0, 0.0, 0.0};
+    for (int r = 0; r < GN_WIDE_CLUSTER; ++r) {
+      t.n += ld_cluster_f64(&s_cta[0], r);
+      t.s1 += ld_cluster_f64(&s_cta[1], r);
+      t.s2 += ld_cluster_f64(&s_cta[2], r);
     }
-    __syncthreads();
+    stat_store(fin + ((long long)n * G + g) * 3, t);
   }
-  if (threadIdx.x == 0) {
-    float* dst = fin + ((long long)n * G + g) * 3;
-    dst[0] = s_n[0]; dst[1] = s_m[0]; dst[2] = s_2[0];
-  }
+  __syncthreads();
+  cluster_sync_all();  // no CTA leaves while its shared memory is still being read
 }
 
 __global__ void __launch_bounds__(GN_THREADS) gn_bwd_finalize_kernel(const float* __restrict__ part,
@@ -649,15 +672,23 @@ using namespace sb;
 // 1 when the kernels cover GroupNorm over C channels in G groups, else 0 (callers then take another path)
 extern "C" int sb_gn_supported(int C, int G) { return gn_channels_ok(C, G) ? 1 : 0; }
 
-extern "C" int sb_gn_nsplit(int N, long long S, int C) {
+// Splits of a sample's voxels, at least `rows` rows of voxels (one per thread) in each.
+static int gn_nsplit(int N, long long S, int C, int rows) {
   if (N < 1 || S < 1 || C < 8 || C / 8 > GN_THREADS) return 1;  // unsupported shapes are refused by the launchers
-  const int vpb = GN_THREADS / (C / 8);
-  long long maxs = (S + vpb - 1) / vpb;  // at least one row of voxels per split
+  const long long step = (long long)rows * (GN_THREADS / (C / 8));
+  const long long maxs = (S + step - 1) / step;
   long long want = (148LL * 4 + N - 1) / N;
   long long s = want < maxs ? want : maxs;
   if (s > 1024) s = 1024;
   return (int)(s < 1 ? 1 : s);
 }
+
+extern "C" int sb_gn_nsplit(int N, long long S, int C) { return gn_nsplit(N, S, C, 1); }
+
+// Splits of the backward sums (never more than sb_gn_nsplit). Their partials have 2 C floats per split, so with one
+// row of voxels per split a small wide tensor (512 voxels of 1024 channels) would write and read back twice its own
+// bytes; four rows keep them below a quarter of the two tensors that the pass reads.
+extern "C" int sb_gn_bwd_nsplit(int N, long long S, int C) { return gn_nsplit(N, S, C, 4); }
 
 extern "C" int sb_gn_stats(const SbGnArgs* a, cudaStream_t stream) {
   GnParams p;
@@ -734,8 +765,8 @@ extern "C" int sb_gn_share(const float* fin, long long count, void* const* dst, 
 // fin: [N][G][3] (stats) / [N][C][2] (bwd) -- the single-split form the apply / dx kernels merge
 extern "C" int sb_gn_stats_finalize(const float* part, float* fin, int N, int G, int nsplit, cudaStream_t stream) {
   const int warps = N * G;
-  if (nsplit > 1024) {  // a warp per output would walk hundreds of partials per lane: a block per output instead
-    gn_stats_finalize_wide_kernel<<<warps, GN_THREADS, 0, stream>>>(part, fin, N, G, nsplit);
+  if (nsplit > 1024) {  // a warp per output would walk more than 32 partials per lane: a cluster per output instead
+    gn_stats_finalize_wide_kernel<<<warps * GN_WIDE_CLUSTER, GN_THREADS, 0, stream>>>(part, fin, N, G, nsplit);
     sb_count_launch(1);
     return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
   }

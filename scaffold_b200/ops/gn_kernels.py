@@ -16,6 +16,7 @@ import torch
 from . import _lib
 
 _lib.register("sb_gn_nsplit", [C.c_int, C.c_longlong, C.c_int], C.c_int)
+_lib.register("sb_gn_bwd_nsplit", [C.c_int, C.c_longlong, C.c_int], C.c_int)
 _lib.register("sb_gn_supported", [C.c_int, C.c_int], C.c_int)
 
 
@@ -153,11 +154,12 @@ def gn_forward(x, w, b, groups: int, eps: float = 1e-5, relu: bool = True, fin: 
 def gn_bwd_partial(dy, x, w, b, mean, rstd, groups, eps, relu, part: Optional[torch.Tensor] = None,
                    fin: Optional[torch.Tensor] = None):
     """Backward pass 1: this rank's per-(n, channel) sums ``[N*C*2]`` (what peers exchange)."""
-    a = _base(x, w, b, groups, eps, relu, 1)
+    a = _base(x, w, b, groups, eps, relu, 1,
+              nsplit=_lib.lib().sb_gn_bwd_nsplit(x.shape[0], x.shape[1] * x.shape[2] * x.shape[3], x.shape[4]))
     a.dy = dy.data_ptr()
     a.mean, a.rstd = mean.data_ptr(), rstd.data_ptr()
     if part is None:
-        part = torch.empty(partial_numel_bwd(x), dtype=torch.float32, device=x.device)
+        part = torch.empty(a.N * a.nsplit * a.C * 2, dtype=torch.float32, device=x.device)
     a.part = part.data_ptr()
     a.n_parts = 1
     a.parts[0] = part.data_ptr()

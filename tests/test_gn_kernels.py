@@ -129,3 +129,23 @@ def test_last_block_collapse_equals_the_separate_finalize_launch(shape, groups, 
     again = gk.gn_stats(x, w, b, groups, 1e-5, True)
     torch.cuda.synchronize()
     assert torch.equal(again, outs[0][0])
+
+
+@pytest.mark.parametrize("nsplit", [1, 31, 592, 1024, 1025, 2049, 16384])
+def test_finalize_pools_partials_like_fp64(nsplit):
+    """Both collapse kernels (a warp per output up to 1024 partials, a cluster of eight CTAs beyond), empty partials and
+    a mean of a hundred standard deviations included."""
+    from scaffold_b200.ops import gn_kernels as gk
+    g = torch.Generator(device="cuda").manual_seed(nsplit)
+    part = torch.empty((2, nsplit, 8, 3), device="cuda")
+    part[..., 0] = torch.randint(0, 3, (2, nsplit, 1), generator=g, device="cuda") * 512.0
+    part[:, 0, :, 0] = 512.0
+    part[..., 1] = 100.0 + torch.randn((2, nsplit, 8), generator=g, device="cuda")
+    part[..., 2] = torch.rand((2, nsplit, 8), generator=g, device="cuda") * 512.0
+    got = gk.gn_finalize(part.reshape(-1), 2, 8, nsplit).view(2, 8, 3).double()
+    n, m, m2 = part.double().unbind(-1)
+    tot = n.sum(1)
+    mean = (n * m).sum(1) / tot
+    ref = torch.stack([tot, mean, (m2 + n * (m - mean[:, None]) ** 2).sum(1)], -1)
+    # sums in double, results rounded once to fp32: 2^-24, doubled for the subtraction in M2
+    torch.testing.assert_close(got, ref, rtol=2 ** -22, atol=1e-3)
