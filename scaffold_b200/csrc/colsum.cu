@@ -55,29 +55,33 @@ __global__ void __launch_bounds__(CS_THREADS) colsum_partial_kernel(const __nv_b
 
 // one warp per channel: lanes take the partials b = lane, lane + 32, ... in order, then a fixed shuffle tree
 __global__ void __launch_bounds__(CS_THREADS) colsum_final_kernel(const float* __restrict__ part, int nblocks, int C,
-                                                                  float* __restrict__ out, int n_out) {
+                                                                  float* __restrict__ out, int n_out, int accumulate) {
   const int ch = blockIdx.x * (CS_THREADS / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (ch >= n_out) return;
   float s = 0.f;
+#pragma unroll 8
   for (int b = lane; b < nblocks; b += 32) s += part[(long long)b * C + ch];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) out[ch] = s;
+  if (lane == 0) out[ch] = accumulate ? out[ch] + s : s;
 }
 
 }  // namespace sb
 
-// x bf16 [M, C] (C a multiple of 8, at most 2048), out fp32 [n_out] (n_out <= C), work fp32 [sb_colsum_blocks() * C]
+// x bf16 [M, C] (C a multiple of 8, at most 2048), out fp32 [n_out] (n_out <= C; added to when `accumulate`),
+// work fp32 [sb_colsum_blocks() * C]
 extern "C" int sb_colsum_blocks(void) { return 592; }
-extern "C" int sb_colsum(const void* x, long long M, int C, float* out, int n_out, float* work, cudaStream_t stream) {
+extern "C" int sb_colsum(const void* x, long long M, int C, float* out, int n_out, float* work, int accumulate,
+                         cudaStream_t stream) {
   if (C % 8 != 0 || C / 8 > sb::CS_THREADS || n_out > C || M <= 0) return SB_ERR_SHAPE;
   const int rpb = sb::CS_THREADS / (C / 8);
   long long want = (M + rpb - 1) / rpb;
   const int nblocks = (int)(want < 592 ? want : 592);
   sb::colsum_partial_kernel<<<nblocks, sb::CS_THREADS, 0, stream>>>((const __nv_bfloat16*)x, M, C, work);
   const int cpb = sb::CS_THREADS / 32;
-  sb::colsum_final_kernel<<<(n_out + cpb - 1) / cpb, sb::CS_THREADS, 0, stream>>>(work, nblocks, C, out, n_out);
+  sb::colsum_final_kernel<<<(n_out + cpb - 1) / cpb, sb::CS_THREADS, 0, stream>>>(work, nblocks, C, out, n_out,
+                                                                                         accumulate);
   sb_count_launch(2);
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }

@@ -51,6 +51,7 @@ struct GnParams {
   int nsplit;
   float eps;
   int relu;
+  int accumulate;     // add to dw / db
   float group_elems;  // elements per (n, g) over ALL shards = S_total * C/G
   const uint32_t* wait_flags;  // optional: peers' "statistics landed" flags (local memory)
   uint32_t wait_epoch;
@@ -493,8 +494,8 @@ __global__ void __launch_bounds__(GN_THREADS) gn_bwd_dx_kernel(const GnParams p)
           b += base[(long long)s * p.C * 2 + 1];
         }
       }
-      p.db[ch] = a;
-      p.dw[ch] = b;
+      p.db[ch] = p.accumulate ? p.db[ch] + a : a;
+      p.dw[ch] = p.accumulate ? p.dw[ch] + b : b;
     }
   }
   const int tpv = p.C / 8;
@@ -632,6 +633,7 @@ static int gn_fill(const SbGnArgs* a, GnParams& p) {
   p.nsplit = a->nsplit;
   p.eps = a->eps;
   p.relu = a->relu;
+  p.accumulate = a->accumulate;
   p.group_elems = (float)((double)a->S_total * cg);
   p.wait_flags = a->wait_flags;
   p.wait_epoch = a->wait_epoch;

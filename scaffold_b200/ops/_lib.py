@@ -152,12 +152,13 @@ _SIGNATURES = {
     "sb_pack_conv3_batch": ([_P, C.c_int, C.c_longlong, _P], C.c_int),
     "sb_stage_input": ([_P, C.c_int, C.c_int, C.c_int, C.c_longlong, _P, C.c_int, _P], C.c_int),
     "sb_colsum_blocks": ([], C.c_int),
-    "sb_colsum": ([_P, C.c_longlong, C.c_int, _P, C.c_int, _P, _P], C.c_int),
+    "sb_colsum": ([_P, C.c_longlong, C.c_int, _P, C.c_int, _P, C.c_int, _P], C.c_int),
     "sb_convT_fwd": ([C.POINTER(SbConvTArgs), _P], C.c_int),
     "sb_convT_dgrad": ([C.POINTER(SbConvTArgs), _P], C.c_int),
     "sb_conv_wgrad": ([C.POINTER(SbWgradArgs), _P], C.c_int),
     "sb_conv_wgrad_workspace": ([C.POINTER(SbWgradArgs)], C.c_longlong),
     "sb_launch_count": ([], C.c_longlong),
+    "sb_count_launch": ([C.c_int], None),
 }
 
 

@@ -27,56 +27,92 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import conv_kernels as ck
-from .layout import direct_grad_target, from_vm, notify_grad_written, to_vm, use_cuda_kernels, weights_epoch
+from .layout import (EPOCH_CELL_ATTR, direct_grad_target, from_vm, notify_grad_written, to_vm, use_cuda_kernels,
+                     weights_epoch)
 
 
 # A/B switch: "0" keeps the GroupNorm statistics in their own pass instead of the convolution's epilogue
 _GN_FROM_EPILOGUE = os.environ.get("SCAFFOLD_GN_FROM_EPILOGUE", "1") != "0"
 
 _PACK_REGISTRY: "weakref.WeakSet[_PackCache]" = weakref.WeakSet()
-_PACK_PLAN = {"key": None, "table": None, "n": 0, "tiles": 0, "members": []}
+_PACK_GENERATION = [0]  # counts the layouts that layers have asked for: a packing table built before is out of date
 
 
-def repack_all() -> int:
-    """Refresh every 3x3x3 operand copy that any layer has asked for so far, in ONE kernel launch.
-
-    The optimizer calls this right after it updated the weights, so the next forward pass finds all
-    packs fresh instead of launching one packing kernel per layer (role of the weight repack that
-    the update kernel owes the convolutions). Returns the number of layers covered; layers that have
-    not run yet, or whose weight is a non-contiguous view, keep packing lazily on first use.
-    """
-    from . import _lib
+def _pack_members(cell) -> list:
     members = []
     for cache in list(_PACK_REGISTRY):
         w = cache._w_ref() if cache._w_ref is not None else None
-        if w is None or not w.is_cuda or not w.is_contiguous() or w.dtype != torch.float32:
+        if w is None or not w.is_cuda or not w.is_contiguous() or w.dtype != torch.float32 \
+                or getattr(w, EPOCH_CELL_ATTR, None) is not cell:
             continue
         for sig in sorted({k[1] for k in cache._asked}):
             names = sorted(nm for nm, s_ in cache._asked if s_ == sig)
             bufs = {nm: cache._bufs.get((nm, sig, w.device)) for nm in names}
             if any(b is None for b in bufs.values()):
                 continue
-            members.append((cache, w, sig, cache._real[sig], bufs))
-    if not members:
+            members.append((weakref.ref(cache), weakref.ref(w), w.data_ptr(), sig, cache._tap_swap, bufs))
+    return members
+
+
+def repack_all(flat) -> int:
+    """Refresh every 3x3x3 operand copy that any layer has asked for so far of the parameters of ``flat`` (a
+    ``FlatBuffers``), in ONE kernel launch.
+
+    The optimizer calls this right after it updated the weights, so the next forward pass finds all
+    packs fresh instead of launching one packing kernel per layer (role of the weight repack that
+    the update kernel owes the convolutions). Other models' layers are left alone: their weights did not change.
+    The job table is kept with the parameters and rebuilt when a layer asks for a new layout or a weight has moved.
+    Returns the number of layers covered; layers that have not run yet, or whose weight is a non-contiguous view,
+    keep packing lazily on first use.
+    """
+    from . import _lib
+    plan = flat.pack_plan
+    live = None
+    if plan.get("generation") == _PACK_GENERATION[0]:
+        live = [(c(), w()) for c, w, *_ in plan["members"]]
+        if any(c is None or w is None or w.data_ptr() != m[2] or c._tap_swap != m[4]
+               for (c, w), m in zip(live, plan["members"])):
+            live = None
+    if live is None:
+        members = _pack_members(flat.epoch_cell)
+        plan.update(generation=_PACK_GENERATION[0], members=members, tiles=0)
+        live = [(c(), w()) for c, w, *_ in members]
+        if members:
+            jobs = (_lib.SbPackJob * len(members))()
+            for j, ((cache, w), (_, _, _, sig, swap, bufs)) in enumerate(zip(live, members)):
+                ck.fill_pack_args(jobs[j].a, w, sig, cache._real[sig], bufs, swap)
+            plan["tiles"] = int(_lib.lib().sb_pack_conv3_plan(jobs, len(members)))
+            if plan["tiles"] < 1:
+                plan.clear()
+                raise _lib.NativeError("sb_pack_conv3_plan refused the packing table")
+            host = torch.frombuffer(bytearray(bytes(jobs)), dtype=torch.uint8)
+            plan["table"] = host.to(live[0][1].device)
+    if not live:
         return 0
-    key = tuple((id(c), w.data_ptr(), sig, c._tap_swap, tuple((n, b.data_ptr()) for n, b in sorted(bufs.items())))
-                for c, w, sig, _, bufs in members)
-    plan = _PACK_PLAN
-    if plan["key"] != key:
-        jobs = (_lib.SbPackJob * len(members))()
-        for j, (_, w, sig, real_c, bufs) in enumerate(members):
-            ck.fill_pack_args(jobs[j].a, w, sig, real_c, bufs, cache._tap_swap)
-        total = _lib.lib().sb_pack_conv3_plan(jobs, len(members))
-        if total < 1:
-            raise _lib.NativeError("sb_pack_conv3_plan refused the packing table")
-        host = torch.frombuffer(bytearray(bytes(jobs)), dtype=torch.uint8)
-        plan.update(key=key, table=host.to(members[0][1].device), n=len(members), tiles=int(total))
-    _lib.check(_lib.lib().sb_pack_conv3_batch(plan["table"].data_ptr(), plan["n"], plan["tiles"], _lib.stream_ptr()),
+    _lib.check(_lib.lib().sb_pack_conv3_batch(plan["table"].data_ptr(), len(live), plan["tiles"], _lib.stream_ptr()),
                "sb_pack_conv3_batch")
-    for cache, w, sig, _, bufs in members:
+    for (cache, w), (_, _, _, sig, _, bufs) in zip(live, plan["members"]):
         cache._sync(w)
         cache._fresh.update((nm, sig) for nm in bufs)
-    return len(members)
+    return len(live)
+
+
+def refresh_packs(flat) -> None:
+    """Bring the operand copies that :func:`repack_all` covers up to date if the weights were changed since the last
+    optimizer step by something else (a checkpoint, an initialisation); two comparisons per layer when they were not."""
+    for cache, weight, _, sig, _, bufs in flat.pack_plan.get("members", ()):
+        c, w = cache(), weight()
+        if c is None or w is None:
+            continue
+        c._sync(w)
+        if any((nm, sig) not in c._fresh for nm in bufs):
+            repack_all(flat)
+            return
+
+
+def pack_buffers(flat) -> list:
+    """The operand buffers of :func:`repack_all`'s table (persistent: a captured pass reads them at their addresses)."""
+    return [b for *_, bufs in flat.pack_plan.get("members", ()) for b in bufs.values()]
 
 
 class _PackCache:
@@ -96,7 +132,7 @@ class _PackCache:
         # strides / tap exchange: the same parameter may be read tap-transposed (sharded runs) or directly
         if tap_swap is not None:
             self._tap_swap = int(tap_swap)
-        key = (w.data_ptr(), w._version, w.device, weights_epoch(), tuple(w.stride()), self._tap_swap)
+        key = (w.data_ptr(), w._version, w.device, weights_epoch(w), tuple(w.stride()), self._tap_swap)
         if key != self._key:
             self._key = key
             self._vals = {}
@@ -112,7 +148,9 @@ class _PackCache:
         sig = tuple(src_c)
         name = kind + ("_kd" if kd else "")
         if (name, sig) not in self._fresh:
-            self._asked.add((name, sig))
+            if (name, sig) not in self._asked:
+                self._asked.add((name, sig))
+                _PACK_GENERATION[0] += 1
             self._real[sig] = list(real_c)
             if self._w_ref is None and isinstance(w, torch.nn.Parameter):
                 self._w_ref = weakref.ref(w)
@@ -156,6 +194,16 @@ def _pad_in_channels(w: torch.Tensor, src_channels: Sequence[int], real: Sequenc
     return torch.cat(parts, 1)
 
 
+def _bias_grad(gy: torch.Tensor, n_out: int, bias) -> Optional[torch.Tensor]:
+    """Bias gradient for autograd, or None when it went straight into the flat gradient buffer."""
+    direct = direct_grad_target(bias)
+    gb = ck.bias_grad(gy, n_out, into=direct)
+    if direct is None:
+        return gb
+    notify_grad_written(bias)
+    return None
+
+
 class _ConvSameFn(torch.autograd.Function):
     """k in {1,3} stride-1 'same' conv over voxel-major bf16 sources."""
 
@@ -190,7 +238,7 @@ class _ConvSameFn(torch.autograd.Function):
                             out_dims=out_dims, in_off=in_off, gn_groups=gn, gn_sink=sink)
         mod._gn_partials = sink[0] if sink else None  # picked up by Conv3d.forward, handed to the GroupNorm
         ctx.mod = mod
-        ctx.wparam = weight  # the caller's tensor itself: backward may add into its flat-buffer .grad
+        ctx.wparam, ctx.bparam = weight, bias  # the caller's tensors: backward may add into their flat-buffer .grad
         ctx.in_off, ctx.in_dims = in_off, in_dims
         ctx.src_c, ctx.real_c = src_c, real_c
         ctx.tap_swap = ts
@@ -241,7 +289,7 @@ class _ConvSameFn(torch.autograd.Function):
                     o += sc
                 gw = torch.cat(parts, 1).contiguous()
         if ctx.has_bias and ctx.needs_input_grad[1]:
-            gb = ck.bias_grad(gy, weight.shape[0])
+            gb = _bias_grad(gy, weight.shape[0], ctx.bparam)
         return (gw, gb, None, None, None, *gxs)
 
 
@@ -401,7 +449,7 @@ class _ConvTFn(torch.autograd.Function):
             b32 = mod._cache_b.get(bias, "b", lambda b: b.contiguous())
         y = ck.convT_fwd(x, wf, cout, b32)
         ctx.mod = mod
-        ctx.wparam = weight
+        ctx.wparam, ctx.bparam = weight, bias
         ctx.has_bias = bias is not None
         ctx.save_for_backward(weight, x)
         return y
@@ -424,7 +472,7 @@ class _ConvTFn(torch.autograd.Function):
                 gw = torch.empty(weight.shape, dtype=torch.float32, device=weight.device)  # contiguous whatever the parameter layout
                 ck.conv_wgrad(gy, [x], 2, gw)
         if ctx.has_bias and ctx.needs_input_grad[1]:
-            gb = ck.bias_grad(gy, gy.shape[4])
+            gb = _bias_grad(gy, gy.shape[4], ctx.bparam)
         return gw, gb, None, gx
 
 

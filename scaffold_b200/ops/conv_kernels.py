@@ -126,14 +126,16 @@ def fill_pack_args(a, wc: torch.Tensor, src_c: Sequence[int], real_c: Sequence[i
         setattr(a, name, t.data_ptr() if t is not None else None)
 
 
-def bias_grad(gy: torch.Tensor, n_out: int) -> torch.Tensor:
-    """fp32 sum of a voxel-major bf16 gradient ``[..., C]`` over all voxels, first ``n_out`` channels."""
+def bias_grad(gy: torch.Tensor, n_out: int, into: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """fp32 sum of a voxel-major bf16 gradient ``[..., C]`` over all voxels, first ``n_out`` channels (added to
+    ``into`` when given)."""
     c = gy.shape[-1]
     m = gy.numel() // c
     L = _lib.lib()
-    out = torch.empty(n_out, dtype=torch.float32, device=gy.device)
+    out = into if into is not None else torch.empty(n_out, dtype=torch.float32, device=gy.device)
     work = torch.empty(L.sb_colsum_blocks() * c, dtype=torch.float32, device=gy.device)
-    _lib.check(L.sb_colsum(gy.data_ptr(), m, c, out.data_ptr(), n_out, work.data_ptr(), _lib.stream_ptr()), "sb_colsum")
+    _lib.check(L.sb_colsum(gy.data_ptr(), m, c, out.data_ptr(), n_out, work.data_ptr(), int(into is not None),
+                           _lib.stream_ptr()), "sb_colsum")
     return out
 
 
@@ -289,6 +291,10 @@ _workspaces: dict = {}
 
 
 def _workspace(device, elems: int) -> torch.Tensor:
+    if torch.cuda.is_current_stream_capturing():
+        # a graph keeps its addresses: its scratch comes from its own memory, not from the buffer that later calls
+        # may replace by a larger one
+        return torch.empty(elems, dtype=torch.float32, device=device)
     key = torch.device(device).index or 0
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < elems:

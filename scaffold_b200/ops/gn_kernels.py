@@ -49,6 +49,7 @@ class SbGnArgs(C.Structure):
         ("wait_s", C.c_double),
         ("status", C.c_void_p),
         ("fin", C.c_void_p),
+        ("accumulate", C.c_int),
     ]
 
 
@@ -63,6 +64,12 @@ _lib.register("sb_gn_share", [C.c_void_p, C.c_longlong, C.POINTER(C.c_void_p), C
 # SCAFFOLD_GN_FUSED_FINALIZE=0 collapses the partial statistics in a launch of its own (the A/B switch of the
 # last-block hand-over inside the statistics kernels)
 _FUSED_FINALIZE = os.environ.get("SCAFFOLD_GN_FUSED_FINALIZE", "1") != "0"
+
+
+def _fused_finalize(outputs: int) -> bool:
+    """Whether the last block of a launch collapses its partials. Not inside a captured graph: the launch would keep
+    its block counter for good, and two graphs that replay on two streams could share one."""
+    return _FUSED_FINALIZE and outputs <= 32 and not torch.cuda.is_current_stream_capturing()
 
 
 def _base(x: torch.Tensor, w, b, groups: int, eps: float, relu: bool, shards: int, nsplit: int = 0) -> SbGnArgs:
@@ -100,7 +107,7 @@ def gn_stats(x, w, b, groups, eps, relu, part: Optional[torch.Tensor] = None,
     a.parts[0] = part.data_ptr()
     if fin is None:
         fin = torch.empty(x.shape[0] * groups * 3, dtype=torch.float32, device=x.device)
-    fused = _FUSED_FINALIZE and x.shape[0] * groups <= 32
+    fused = _fused_finalize(x.shape[0] * groups)
     if fused:
         a.fin = fin.data_ptr()  # the last block of the launch collapses the partials: no separate finalize launch
     _lib.check(_lib.lib().sb_gn_stats(C.byref(a), _lib.stream_ptr()), "sb_gn_stats")
@@ -167,7 +174,7 @@ def gn_bwd_partial(dy, x, w, b, mean, rstd, groups, eps, relu, part: Optional[to
         fin = torch.empty(x.shape[0] * x.shape[4] * 2, dtype=torch.float32, device=x.device)
     # The hand-over to the last block pays only while that one block has a handful of outputs to collapse: N*C
     # per-channel sums would make it a serial tail (measured: +1.6 ms per step), so they keep their own launch.
-    fused = _FUSED_FINALIZE and x.shape[0] * x.shape[4] <= 32
+    fused = _fused_finalize(x.shape[0] * x.shape[4])
     if fused:
         a.fin = fin.data_ptr()
     _lib.check(_lib.lib().sb_gn_bwd_partial(C.byref(a), _lib.stream_ptr()), "sb_gn_bwd_partial")
@@ -177,15 +184,21 @@ def gn_bwd_partial(dy, x, w, b, mean, rstd, groups, eps, relu, part: Optional[to
     return fin
 
 
-def gn_bwd_dx(dy, x, w, b, mean, rstd, groups, eps, relu, parts: Sequence[int], shards: int = 1, wait=None):
+def gn_bwd_dx(dy, x, w, b, mean, rstd, groups, eps, relu, parts: Sequence[int], shards: int = 1, wait=None,
+              into=None):
+    """``into``: a (weight gradient, bias gradient) pair that the kernel adds to; returned instead of new tensors."""
     a = _base(x, w, b, groups, eps, relu, shards, nsplit=1)
     _set_wait(a, wait, x.device)
     a.dy = dy.data_ptr()
     a.mean, a.rstd = mean.data_ptr(), rstd.data_ptr()
     dx = torch.empty_like(x)
     c = x.shape[4]
-    dw = torch.empty(c, dtype=torch.float32, device=x.device)
-    db = torch.empty(c, dtype=torch.float32, device=x.device)
+    if into is not None:
+        dw, db = into
+        a.accumulate = 1
+    else:
+        dw = torch.empty(c, dtype=torch.float32, device=x.device)
+        db = torch.empty(c, dtype=torch.float32, device=x.device)
     a.y, a.dw, a.db = dx.data_ptr(), dw.data_ptr(), db.data_ptr()
     a.n_parts = len(parts)
     for i, p in enumerate(parts):
@@ -194,6 +207,6 @@ def gn_bwd_dx(dy, x, w, b, mean, rstd, groups, eps, relu, parts: Sequence[int], 
     return dx, dw, db
 
 
-def gn_backward(dy, x, w, b, mean, rstd, groups: int, eps: float = 1e-5, relu: bool = True):
+def gn_backward(dy, x, w, b, mean, rstd, groups: int, eps: float = 1e-5, relu: bool = True, into=None):
     part = gn_bwd_partial(dy, x, w, b, mean, rstd, groups, eps, relu)
-    return gn_bwd_dx(dy, x, w, b, mean, rstd, groups, eps, relu, [part.data_ptr()])
+    return gn_bwd_dx(dy, x, w, b, mean, rstd, groups, eps, relu, [part.data_ptr()], into=into)

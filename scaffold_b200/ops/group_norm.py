@@ -18,7 +18,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import gn_kernels as gk
-from .layout import from_vm, to_vm, use_cuda_kernels
+from .layout import direct_grad_target, from_vm, notify_grad_written, to_vm, use_cuda_kernels
 
 
 class _GnFn(torch.autograd.Function):
@@ -37,6 +37,7 @@ class _GnFn(torch.autograd.Function):
             y, mean, rstd = spatial.gn_forward(x, w32, b32, groups, eps, relu, fin=fin)
         ctx.save_for_backward(x, w32, b32, mean, rstd)
         ctx.cfg = (groups, eps, relu, spatial)
+        ctx.params = (weight, bias)  # the parameters themselves: backward may add into their flat-buffer .grad
         return y
 
     @staticmethod
@@ -45,7 +46,16 @@ class _GnFn(torch.autograd.Function):
         groups, eps, relu, spatial = ctx.cfg
         gy = gy.contiguous()
         if spatial is None:
-            dx, dw, db = gk.gn_backward(gy, x, w32, b32, mean, rstd, groups, eps, relu)
+            into = None
+            if ctx.needs_input_grad[1] and ctx.needs_input_grad[2]:
+                into = tuple(direct_grad_target(p) for p in ctx.params)
+                if any(t is None for t in into):
+                    into = None
+            dx, dw, db = gk.gn_backward(gy, x, w32, b32, mean, rstd, groups, eps, relu, into=into)
+            if into is not None:
+                dw = db = None
+                for p in ctx.params:
+                    notify_grad_written(p)
         else:
             dx, dw, db = spatial.gn_backward(gy, x, w32, b32, mean, rstd, groups, eps, relu)
         return dx, dw, db, None, None, None, None, None

@@ -63,16 +63,27 @@ def from_vm(y: torch.Tensor) -> torch.Tensor:
 
 
 # Parameters updated through raw pointers (the fused optimizer) do not bump the
-# tensors' version counters; packed operand caches also key on this epoch.
-_weights_epoch = [0]
+# tensors' version counters; packed operand caches also key on weights_epoch().
+_weights_epoch = [0]  # any weights may have changed (a checkpoint was restored)
+_flat_steps = [0]     # steps of all flat optimizers together
+EPOCH_CELL_ATTR = "_sb_epoch_cell"  # on a parameter of a flat optimizer: the one-element step counter of that optimizer
 
 
 def bump_weights_epoch() -> None:
     _weights_epoch[0] += 1
 
 
-def weights_epoch() -> int:
-    return _weights_epoch[0]
+def bump_flat_step(cell) -> None:
+    """A flat optimizer updated its parameters, and only those, through raw pointers."""
+    cell[0] += 1
+    _flat_steps[0] += 1
+
+
+def weights_epoch(w=None):
+    """Changes when ``w`` may have been updated through raw pointers: with the steps of its own optimizer, or, for a
+    tensor that no optimizer has marked (a view of a parameter), with every optimizer's steps."""
+    cell = getattr(w, EPOCH_CELL_ATTR, None)
+    return (_weights_epoch[0], _flat_steps[0] if cell is None else cell[0])
 
 
 # Parameters whose ``.grad`` is a view into a flat gradient buffer (set up by the fused optimizer) are marked
@@ -84,8 +95,8 @@ _grad_written_listeners = []
 
 def direct_grad_target(param):
     """The flat-buffer gradient view of ``param`` when the kernels may accumulate into it directly, else None."""
-    if not getattr(param, FLAT_GRAD_ATTR, False):
-        return None
+    if not getattr(param, FLAT_GRAD_ATTR, False) or param._backward_hooks:
+        return None  # a hook on the parameter wants to see its gradient: autograd's own accumulation
     g = param.grad
     if g is None or g.dtype != torch.float32 or not g.is_contiguous() or g.shape != param.shape:
         return None

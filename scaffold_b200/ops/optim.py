@@ -16,7 +16,7 @@ from typing import Iterable, Optional
 import torch
 
 from . import _lib
-from .layout import FLAT_GRAD_ATTR, bump_weights_epoch
+from .layout import EPOCH_CELL_ATTR, FLAT_GRAD_ATTR, bump_flat_step
 
 _P = C.c_void_p
 _lib.register("sb_opt_blocks", [C.c_longlong], C.c_int)
@@ -42,12 +42,15 @@ class FlatBuffers:
         self.numel = off
         self.data = torch.zeros(off, dtype=torch.float32, device=dev)
         self.grad = torch.zeros(off, dtype=torch.float32, device=dev)
+        self.epoch_cell = [0]  # optimizer steps; shared with the parameters, which key their operand copies on it
+        self.pack_plan = {}    # conv3d.repack_all's table for these parameters
         for p, o in zip(self.params, self.offsets):
             view = self.data[o:o + p.numel()].view_as(p)
             view.copy_(p.data)
             p.data = view
             p.grad = self.grad[o:o + p.numel()].view_as(p)
             setattr(p, FLAT_GRAD_ATTR, True)
+            setattr(p, EPOCH_CELL_ATTR, self.epoch_cell)
 
     def rehome_grad(self, new_grad: torch.Tensor) -> None:
         """Move the gradient buffer into ``new_grad`` (e.g. peer-visible memory) and re-point every ``.grad``."""
@@ -168,7 +171,7 @@ class FusedClipAdam(torch.optim.Adam):
                                   f.numel, float(g["lr"]), float(b1), float(b2), float(g["eps"]), self._steps,
                                   max_norm, self._norm.data_ptr(), float(self.reduce_scale), s), "sb_adam_step")
         self._step_t.fill_(float(self._steps))
-        bump_weights_epoch()
+        bump_flat_step(f.epoch_cell)
         from .conv3d import repack_all
-        repack_all()  # one launch refreshes the bf16 operand copies of every convolution for the next step
+        repack_all(f)  # one launch refreshes the bf16 operand copies of these parameters' convolutions
         return None
