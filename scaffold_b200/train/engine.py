@@ -19,6 +19,7 @@ from ..ops.layout import AMP_DTYPE
 from ..ops.optim import FusedClipAdam
 from ..parallel.ddp import GradReducer
 from ..utils.perf import region
+from .step_graph import StepGraphs
 
 
 class TrainEngine:
@@ -44,6 +45,7 @@ class TrainEngine:
         self.last_ce = self.last_dice = None
         self._loss_event = None
         self._loss_host = None
+        self._graphs = StepGraphs()
 
     # -- data movement --------------------------------------------------------
     def to_device(self, images: torch.Tensor, masks: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -91,9 +93,14 @@ class TrainEngine:
         after the forward pass; ``read_loss()`` then returns it without waiting for backward and the update, so a
         loop that looks at every step's loss does not drain the GPU between steps.
         """
-        images, masks = self.to_device(images, masks)
+        graph = self._graphs.get(self, images, masks, train=True)
+        if graph is None:
+            images, masks = self.to_device(images, masks)
         self.optimizer.zero_grad(set_to_none=self.flat is None)
-        loss, ce, fg, _ = self.forward_loss(images, masks)
+        if graph is None:
+            loss, ce, fg, _ = self.forward_loss(images, masks)
+        else:
+            loss, ce, fg = graph.forward(self, images, masks)
         if loss_host is not None and self.cuda:
             loss_host.copy_(loss.detach().reshape(loss_host.shape), non_blocking=True)
             if self._loss_event is None:
@@ -104,7 +111,10 @@ class TrainEngine:
             loss_host.copy_(loss.detach().reshape(loss_host.shape))
             self._loss_host = loss_host
         with region("backward"):
-            loss.backward()
+            if graph is None:
+                loss.backward()
+            else:
+                graph.backward()
         with region("step_and_update"):
             self.reducer.reduce()
             if not isinstance(self.optimizer, FusedClipAdam):
@@ -127,7 +137,12 @@ class TrainEngine:
     @torch.no_grad()
     def eval_step(self, images: torch.Tensor, masks: torch.Tensor):
         """Returns (loss, hard-dice per (sample, class)) for one validation batch."""
-        images, masks = self.to_device(images, masks)
+        graph = self._graphs.get(self, images, masks, train=False)
+        if graph is not None:
+            return graph.forward(self, images, masks)
+        return self._eval_pass(*self.to_device(images, masks))
+
+    def _eval_pass(self, images: torch.Tensor, masks: torch.Tensor):
         loss, ce, fg, logits = self.forward_loss(images, masks)
         if self.fused_loss:
             logits, masks = logits  # kernel-space pair of the fused path

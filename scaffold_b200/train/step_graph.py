@@ -1,0 +1,195 @@
+"""CUDA graphs of the training and validation passes of a :class:`TrainEngine`.
+
+A step of a small network is bound by its launches: at scale 5 (32 cubed, base width 64) some 200 launches cost about
+25 us of host time each while the kernels need 1.4 ms together, and even at scale 7 the gaps between launches are
+4 % of the step. After a few ordinary passes over batches of one shape the engine therefore captures that pass and
+replays it: one graph for forward and loss, one for backward (so that the loss can be copied to the host between the
+two). The optimizer's update, whose learning rate and step count change from step to step, stays outside.
+
+A graph replays kernels on fixed addresses, so it is used only while nothing that the ordinary pass would have looked
+at has changed: the same parameters at the same addresses, the same modules with the same settings, no hook on any of
+them (see :class:`_Fingerprint`). Otherwise the ordinary pass runs. The batch is copied into the graph's own buffers,
+the results out of them, so inputs may live anywhere and results are the caller's to keep.
+
+Limits: batches whose widest feature map is at most ``MAX_MAP_BYTES`` (2 x 128 cubed x 64 channels), since the graph
+keeps the memory of one pass's activations and larger batches gain less than 1 %; at most ``MAX_SHAPES`` batch shapes
+per engine. The memory is given back with the engine.
+"""
+from __future__ import annotations
+
+import math
+from typing import Optional
+
+import torch
+
+from ..models.unet import UNet
+from ..ops import _lib, conv_kernels as ck, layout, pool_kernels
+from ..ops import conv3d as c3
+from ..ops.optim import FusedClipAdam
+from ..utils import perf
+
+WARM_PASSES = 2        # ordinary passes over a shape before its capture (kernels set up, operand layouts known)
+MAX_SHAPES = 4         # graphs per engine and kind of pass
+MAX_MAP_BYTES = 640 << 20
+
+
+class _Fingerprint:
+    """What a captured pass depends on besides the batch's values; ``holds()`` is a few hundred identity checks."""
+
+    def __init__(self, engine):
+        modules = list(engine.model.modules())
+        self._dicts = [(d, tuple(d.items())) for m in modules for d in (m._parameters, m._buffers, m._modules)]
+        self._hooks = [h for m in modules for h in (m._forward_hooks, m._forward_pre_hooks, m._backward_hooks,
+                                                    m._backward_pre_hooks)]
+        self._params = [(p, p.data_ptr(), p.requires_grad) for p in engine.model.parameters()]
+        self._modules = modules
+        self._settings = self._read(engine)
+
+    def _read(self, engine):
+        out = [m.training for m in self._modules]
+        for m in self._modules:
+            d = m.__dict__
+            if "eps" in d:  # GroupNorm
+                out += (d["eps"], d["num_groups"], d["activation"], d["_spatial"])
+            elif "kernel_size" in d:  # convolutions, pooling
+                out += (d["kernel_size"], d["stride"], d["padding"], d.get("gn_groups_hint"), d.get("_spatial"))
+        cw = engine.class_weights
+        out += (engine.amp, engine.n_classes, id(cw), 0 if cw is None else cw.data_ptr(), engine.model.checkpointing,
+                engine.model._spatial, id(engine.model.forward_padded_logits.__func__), engine.flat.data.data_ptr(),
+                engine.flat.grad.data_ptr(), ck.PAIR_CONV, c3._GN_FROM_EPILOGUE, pool_kernels._USE_INDEX,
+                ck.conv_same, ck.conv_wgrad, ck.convT_fwd, ck.convT_dgrad)
+        return out
+
+    def holds(self, engine) -> bool:
+        for h in self._hooks:
+            if h:
+                return False
+        for d, items in self._dicts:
+            if len(d) != len(items):
+                return False
+            for k, v in items:
+                if d.get(k) is not v:
+                    return False
+        for p, ptr, needs in self._params:
+            if p.data_ptr() != ptr or p.requires_grad is not needs or p._backward_hooks or p._post_accumulate_grad_hooks:
+                return False
+        return self._settings == self._read(engine)
+
+
+class _Pass:
+    """One captured pass: forward + loss (+ backward), with its own input buffers."""
+
+    def __init__(self, engine, images, masks, train: bool):
+        dev = engine.device
+        self.images = torch.empty(images.shape, dtype=images.dtype, device=dev)
+        self.masks = torch.empty(masks.shape, dtype=masks.dtype, device=dev)
+        self.images.copy_(images)
+        self.masks.copy_(masks)
+        self.fingerprint = _Fingerprint(engine)
+        self.class_weights = engine.class_weights  # the kernels read it at its address: keep it alive
+        convs = [c for m in engine.model.modules() for c in (getattr(m, "_cache", None), getattr(m, "_cache_b", None))
+                 if c is not None]
+        # Operand copies that the forward pass makes itself (k = 1 and transposed convolutions, padded biases) must be
+        # made inside the graph, where a replay renews them; the ones of the 3x3x3 layers are persistent buffers that
+        # the optimizer step renews.
+        for c in convs:
+            c._vals = {}
+        engine.flat.rebind_grads()
+        c3.repack_all(engine.flat)
+        self.packs = c3.pack_buffers(engine.flat)
+        pool = torch.cuda.graph_pool_handle()
+        self.forward_graph, self.backward_graph = torch.cuda.CUDAGraph(), None
+        before = _lib.launch_count()
+        try:
+            with torch.cuda.graph(self.forward_graph, pool=pool, capture_error_mode="thread_local"):
+                if train:
+                    loss, ce, fg, _ = engine.forward_loss(self.images, self.masks)
+                    out = (loss.detach(), ce.detach(), fg.detach())
+                else:
+                    with torch.no_grad():
+                        out = engine._eval_pass(self.images, self.masks)
+            self.launches = _lib.launch_count() - before
+            if train:
+                before = _lib.launch_count()
+                self.backward_graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(self.backward_graph, pool=pool, capture_error_mode="thread_local"):
+                    loss.backward()
+                self.back_launches = _lib.launch_count() - before
+        finally:
+            for c in convs:
+                c._vals = {}  # these tensors live in the graph's memory
+        self.out = out
+        self.stream = torch.cuda.current_stream()
+
+    def forward(self, engine, images, masks):
+        stream = torch.cuda.current_stream()
+        if stream != self.stream:  # the buffers are the graph's: a pass on another stream comes after the last one
+            stream.wait_stream(self.stream)
+            self.stream = stream
+        c3.refresh_packs(engine.flat)
+        self.images.copy_(images, non_blocking=True)
+        self.masks.copy_(masks, non_blocking=True)
+        self.forward_graph.replay()
+        _lib.lib().sb_count_launch(self.launches)
+        return tuple(t.clone() for t in self.out)
+
+    def backward(self):
+        self.backward_graph.replay()
+        _lib.lib().sb_count_launch(self.back_launches)
+
+
+class StepGraphs:
+    """The captured passes of one engine."""
+
+    def __init__(self):
+        self._passes = {}   # key -> _Pass, or the number of ordinary passes seen, or None (cannot be captured)
+
+    @staticmethod
+    def _usable(engine, images, masks) -> bool:
+        model = engine.model
+        if not (engine.cuda and engine.fused_loss and engine.flat is not None and type(model) is UNet
+                and isinstance(engine.optimizer, FusedClipAdam) and engine.reducer.world == 1
+                and engine.spatial is None and model._spatial is None):
+            return False
+        widest = images.shape[0] * math.prod(images.shape[2:]) * model.base_width * 2
+        return (widest <= MAX_MAP_BYTES and not model.checkpointing and not layout._aten_only[0]
+                and not torch.is_anomaly_enabled() and not perf._nvtx_enabled()
+                and not torch.nn.modules.module._has_any_global_hook() and torch._C._len_torch_dispatch_stack() == 0
+                and not torch.cuda.is_current_stream_capturing())
+
+    def get(self, engine, images, masks, train: bool) -> Optional[_Pass]:
+        """The captured pass for this batch's shape, or None: run the ordinary pass."""
+        if images.dim() != 5 or not self._usable(engine, images, masks) or torch.is_grad_enabled() is not train:
+            return None
+        key = (train, tuple(images.shape), images.dtype, tuple(masks.shape), masks.dtype)
+        seen = self._passes.get(key, 0)
+        if isinstance(seen, _Pass):
+            if seen.fingerprint.holds(engine):
+                return seen
+            seen = 0  # the model was changed: start over
+            self._passes[key] = seen
+        if seen is None:
+            return None
+        if seen < WARM_PASSES:
+            if key in self._passes or len(self._passes) < 4 * MAX_SHAPES:
+                self._passes[key] = seen + 1
+            return None
+        owned = all(getattr(p, layout.EPOCH_CELL_ATTR, None) is engine.flat.epoch_cell
+                    for p in engine.model.parameters())
+        if not owned:  # a parameter outside the optimizer: nothing would renew its operand copies
+            self._passes[key] = None
+            return None
+        if sum(isinstance(p, _Pass) and k[0] == train for k, p in self._passes.items()) >= MAX_SHAPES:
+            return None
+        probe = _Fingerprint(engine)
+        if not probe.holds(engine):  # hooks are set
+            return None
+        try:
+            self._passes[key] = _Pass(engine, images, masks, train)
+        except RuntimeError as exc:  # no memory for the graph's buffers, or an operation that cannot be captured
+            import logging
+            logging.getLogger("scaffold").warning("the %s pass stays uncaptured: %s", "training" if train else
+                                                  "validation", str(exc).splitlines()[0])
+            self._passes[key] = None
+            torch.cuda.synchronize()
+        return self._passes[key]

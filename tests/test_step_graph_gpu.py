@@ -1,0 +1,104 @@
+"""Captured training / validation passes against the ordinary ones: the same bits, whatever happens in between (GPU)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _engine(graphs: bool, monkeypatch=None, **kw):
+    from scaffold_b200.models.unet import UNet
+    from scaffold_b200.ops.optim import FusedClipAdam
+    from scaffold_b200.train.engine import TrainEngine
+    torch.manual_seed(3)
+    model = UNet(3, 5, layers=2, base_width=32).cuda()
+    eng = TrainEngine(model, FusedClipAdam(model.parameters(), lr=1e-3), 5, torch.device("cuda"), **kw)
+    if not graphs:
+        eng._graphs.get = lambda *a, **k: None
+    return eng
+
+
+def _batch(seed, n=2, edge=(16, 24, 16), device="cuda"):
+    g = torch.Generator().manual_seed(seed)
+    x = torch.rand((n, 3, *edge), generator=g)
+    y = torch.randint(0, 5, (n, *edge), generator=g, dtype=torch.int16)
+    return (x.cuda(), y.cuda()) if device == "cuda" else (x.pin_memory(), y.pin_memory())
+
+
+def _captured(eng):
+    from scaffold_b200.train.step_graph import _Pass
+    return [k for k, v in eng._graphs._passes.items() if isinstance(v, _Pass)]
+
+
+def test_replayed_steps_are_the_ordinary_steps_bit_for_bit():
+    a, b = _engine(True), _engine(False)
+    side = torch.cuda.Stream()
+    kept = []
+    for i in range(14):
+        batch = _batch(i, device="cpu" if i in (5, 6) else "cuda")
+        if i == 7:      # another learning rate
+            for e in (a, b):
+                e.optimizer.param_groups[0]["lr"] = 3e-4
+        if i == 8:      # weights changed behind the optimizer's back
+            for e in (a, b):
+                e.model.load_state_dict({k: v * 0.9 for k, v in e.model.state_dict().items()})
+        if i == 9:      # gradients dropped by the caller
+            for e in (a, b):
+                e.model.zero_grad(set_to_none=True)
+        if i == 10:     # a ragged last batch, then validation between training steps
+            small = _batch(100, n=1)
+            assert torch.equal(a.step(*small), b.step(*small))
+            for _ in range(4):
+                for s, t in zip(a.eval_step(*batch), b.eval_step(*batch)):
+                    assert torch.equal(s, t)
+        if i == 11:
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                la = a.step(*batch)
+            torch.cuda.current_stream().wait_stream(side)
+        else:
+            la = a.step(*batch)
+        lb = b.step(*batch)
+        kept.append((la, lb))
+        assert torch.equal(a.last_ce, b.last_ce) and torch.equal(a.last_dice, b.last_dice)
+        assert torch.equal(a.flat.grad, b.flat.grad) and torch.equal(a.flat.data, b.flat.data), i
+    assert len(_captured(a)) == 2 and not _captured(b)
+    for la, lb in kept:  # a returned loss stays the caller's after later steps
+        assert torch.equal(la, lb)
+
+
+def test_a_changed_model_leaves_the_captured_pass():
+    eng = _engine(True)
+    batch = _batch(1)
+    for _ in range(4):
+        eng.step(*batch)
+    assert _captured(eng)
+    calls = []
+    h = eng.model.down_list[0].register_forward_hook(lambda *a: calls.append(1))
+    eng.step(*batch)
+    assert len(calls) == 1 and not _captured(eng)   # the hook ran: the ordinary pass did
+    eng.step(*batch)
+    eng.step(*batch)
+    assert len(calls) == 3 and not _captured(eng)
+    h.remove()
+    for _ in range(3):
+        eng.step(*batch)
+    assert len(calls) == 3 and _captured(eng)
+    eng.model.up_list[0].conv.double_conv[1].eps = 1e-3
+    eng.step(*batch)
+    assert not _captured(eng)
+
+
+def test_class_weights_are_read_at_replay_and_evaluation_follows_new_weights():
+    cw = torch.tensor([1.0, 5.0, 5.0, 5.0, 5.0], device="cuda")
+    a, b = _engine(True, class_weights=cw), _engine(False, class_weights=cw)
+    batch = _batch(2)
+    for i in range(6):
+        if i == 4:
+            cw.mul_(2.0)
+            for e in (a, b):
+                with torch.no_grad():
+                    for p in e.model.parameters():
+                        p.add_(0.01)
+        for s, t in zip(a.eval_step(*batch), b.eval_step(*batch)):
+            assert torch.equal(s, t), i
+    assert _captured(a)
