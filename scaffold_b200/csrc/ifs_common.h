@@ -22,8 +22,9 @@ namespace sbifs {
 struct Rng {
   uint64_t s;
 };
+constexpr uint64_t RNG_STEP = 0x9E3779B97F4A7C15ull;  // draw i of a seed needs no other draw: its state is seed + i * this
 SB_HD uint64_t next_u64(Rng& r) {
-  uint64_t z = (r.s += 0x9E3779B97F4A7C15ull);
+  uint64_t z = (r.s += RNG_STEP);
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
   z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
   return z ^ (z >> 31);
