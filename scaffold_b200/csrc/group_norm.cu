@@ -305,9 +305,22 @@ __device__ __forceinline__ void merge_group(const GnParams& p, int n, int g, flo
 }
 
 // ----------------------------------------------------------------------------
+// The three streaming kernels are bound by memory and need some 45 KB of loads in flight per SM. They run in ONE wave
+// of GN_WAVE (the sums: GN_WAVE_SUMS) blocks per SM at 64 (85) registers a thread, each thread with as many 16-byte
+// loads in flight as fit. What made room: an octet of channels covers GP groups (1 for the usual eight or more channels
+// per group), so means and the like are GP registers instead of 8; the ReLU's mask is the sign of the forward's own
+// x * a + c, whose `a` is also dx's factor of dy; and xhat is never formed: dx is linear in x - mean, and
+// sum(dy xhat) = rstd * sum(dy (x - mean)). With 97 / 92 registers two blocks fitted per SM, and four blocks' worth of
+// them came in two waves. 64 channels at 2 x 128^3, before / after: sums 225 / 176 us (6.1 TB/s), dx 295 / 248 us
+// (6.5 TB/s), forward 186 / 181 us (5.9 TB/s).
+// ----------------------------------------------------------------------------
+constexpr int GN_WAVE = 4;
+constexpr int GN_WAVE_SUMS = 3;  // the backward sums: 16 more registers of accumulators
+
+// ----------------------------------------------------------------------------
 // forward: normalise + affine + ReLU
 // ----------------------------------------------------------------------------
-__global__ void __launch_bounds__(GN_THREADS) gn_apply_kernel(const GnParams p) {
+__global__ void __launch_bounds__(GN_THREADS, GN_WAVE) gn_apply_kernel(const GnParams p) {
   __shared__ float s_mean[256], s_rstd[256];
   const int n = blockIdx.y;
   if (!gn_wait_peers(p, 61)) return;
@@ -364,7 +377,8 @@ __global__ void __launch_bounds__(GN_THREADS) gn_apply_kernel(const GnParams p) 
 // ----------------------------------------------------------------------------
 // backward: per-channel partial sums
 // ----------------------------------------------------------------------------
-__global__ void __launch_bounds__(GN_THREADS) gn_bwd_partial_kernel(const GnParams p) {
+template <int GP>
+__global__ void __launch_bounds__(GN_THREADS, GN_WAVE_SUMS) gn_bwd_partial_kernel(const GnParams p) {
   __shared__ float s_a[GN_THREADS * 8], s_b[GN_THREADS * 8];
   const int split = blockIdx.x, n = blockIdx.y;
   const int tpv = p.C / 8;
@@ -375,15 +389,14 @@ __global__ void __launch_bounds__(GN_THREADS) gn_bwd_partial_kernel(const GnPara
   const long long chunk = (p.S + p.nsplit - 1) / p.nsplit;
   const long long v0 = (long long)split * chunk;
   const long long v1 = v0 + chunk < p.S ? v0 + chunk : p.S;
-  float mu[8], rs[8], wv[8], bv[8], A[8], B[8];
+  float a[8], c[8], A[8], B[8], mu[GP];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int ch = oct * 8 + i;
     const int g = ch / cg;
-    mu[i] = p.mean[n * p.G + g];
-    rs[i] = p.rstd[n * p.G + g];
-    wv[i] = p.w[ch];
-    bv[i] = p.b[ch];
+    a[i] = p.rstd[n * p.G + g] * p.w[ch];
+    c[i] = p.b[ch] - p.mean[n * p.G + g] * a[i];
+    if (i % (8 / GP) == 0) mu[i / (8 / GP)] = p.mean[n * p.G + g];
     A[i] = 0.f;
     B[i] = 0.f;
   }
@@ -395,27 +408,30 @@ __global__ void __launch_bounds__(GN_THREADS) gn_bwd_partial_kernel(const GnPara
       unpack8(rd, fd);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const float xh = (fx[i] - mu[i]) * rs[i];
         float d = fd[i];
-        if (p.relu && fmaf(xh, wv[i], bv[i]) <= 0.f) d = 0.f;
+        if (p.relu && fmaf(fx[i], a[i], c[i]) <= 0.f) d = 0.f;
         A[i] += d;
-        B[i] += d * xh;
+        B[i] = fmaf(d, fx[i] - mu[i / (8 / GP)], B[i]);
       }
     };
     // two voxels (four 16-byte loads) in flight per thread; the summation order per thread is unchanged
+    const __nv_bfloat16* px = p.x + base + (v0 + vl) * p.C;
+    const __nv_bfloat16* pd = p.dy + base + (v0 + vl) * p.C;
+    const long long row = (long long)vpb * p.C;
     long long v = v0 + vl;
-    for (; v + vpb < v1; v += 2 * vpb) {
-      const uint4 rx0 = __ldg(reinterpret_cast<const uint4*>(p.x + base + v * p.C));
-      const uint4 rd0 = __ldg(reinterpret_cast<const uint4*>(p.dy + base + v * p.C));
-      const uint4 rx1 = __ldg(reinterpret_cast<const uint4*>(p.x + base + (v + vpb) * p.C));
-      const uint4 rd1 = __ldg(reinterpret_cast<const uint4*>(p.dy + base + (v + vpb) * p.C));
+    for (; v + vpb < v1; v += 2 * vpb, px += 2 * row, pd += 2 * row) {
+      const uint4 rx0 = __ldg(reinterpret_cast<const uint4*>(px));
+      const uint4 rd0 = __ldg(reinterpret_cast<const uint4*>(pd));
+      const uint4 rx1 = __ldg(reinterpret_cast<const uint4*>(px + row));
+      const uint4 rd1 = __ldg(reinterpret_cast<const uint4*>(pd + row));
       body(rx0, rd0);
       body(rx1, rd1);
     }
-    for (; v < v1; v += vpb)
-      body(__ldg(reinterpret_cast<const uint4*>(p.x + base + v * p.C)),
-           __ldg(reinterpret_cast<const uint4*>(p.dy + base + v * p.C)));
+    for (; v < v1; v += vpb, px += row, pd += row)
+      body(__ldg(reinterpret_cast<const uint4*>(px)), __ldg(reinterpret_cast<const uint4*>(pd)));
   }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) B[i] *= p.rstd[n * p.G + (oct * 8 + i) / cg];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     s_a[threadIdx.x * 8 + i] = A[i];
@@ -445,7 +461,8 @@ __global__ void __launch_bounds__(GN_THREADS) gn_bwd_partial_kernel(const GnPara
 // ----------------------------------------------------------------------------
 // backward: dx (+ dweight / dbias)
 // ----------------------------------------------------------------------------
-__global__ void __launch_bounds__(GN_THREADS) gn_bwd_dx_kernel(const GnParams p) {
+template <int GP>
+__global__ void __launch_bounds__(GN_THREADS, GN_WAVE) gn_bwd_dx_kernel(const GnParams p) {
   extern __shared__ float sm[];
   float* s_A = sm;              // [C] this rank's sum(dy')
   float* s_B = sm + p.C;        // [C] this rank's sum(dy' xhat)
@@ -503,46 +520,49 @@ __global__ void __launch_bounds__(GN_THREADS) gn_bwd_dx_kernel(const GnParams p)
   const int oct = threadIdx.x % tpv;
   const int vl = threadIdx.x / tpv;
   if (vl >= vpb) return;
-  float mu[8], rs[8], wv[8], bv[8], c1[8], c2[8];
+  // dx = rstd (d w - c1 - xhat c2) = d a + (x - mean) q + r
+  float a[8], c[8], mu[GP], q[GP], r[GP];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int ch = oct * 8 + i;
     const int g = ch / cg;
-    mu[i] = p.mean[n * p.G + g];
-    rs[i] = p.rstd[n * p.G + g];
-    wv[i] = p.w[ch];
-    bv[i] = p.b[ch];
-    c1[i] = s_c1[g];
-    c2[i] = s_c2[g];
+    const float m = p.mean[n * p.G + g], rs = p.rstd[n * p.G + g];
+    a[i] = rs * p.w[ch];
+    c[i] = p.b[ch] - m * a[i];
+    if (i % (8 / GP) == 0) {
+      mu[i / (8 / GP)] = m;
+      q[i / (8 / GP)] = -rs * rs * s_c2[g];
+      r[i / (8 / GP)] = -rs * s_c1[g];
+    }
   }
   const long long base = (long long)n * p.S * p.C + oct * 8;
-  auto body = [&](const uint4 rx, const uint4 rd, long long v) {
+  auto body = [&](const uint4 rx, const uint4 rd, long long at) {
     float fx[8], fd[8];
     unpack8(rx, fx);
     unpack8(rd, fd);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const float xh = (fx[i] - mu[i]) * rs[i];
       float d = fd[i];
-      if (p.relu && fmaf(xh, wv[i], bv[i]) <= 0.f) d = 0.f;
-      fx[i] = rs[i] * (d * wv[i] - c1[i] - xh * c2[i]);
+      if (p.relu && fmaf(fx[i], a[i], c[i]) <= 0.f) d = 0.f;
+      fx[i] = fmaf(d, a[i], fmaf(fx[i] - mu[i / (8 / GP)], q[i / (8 / GP)], r[i / (8 / GP)]));
     }
-    *reinterpret_cast<uint4*>(p.y + base + v * p.C) = pack8(fx);
+    *reinterpret_cast<uint4*>(p.y + at) = pack8(fx);
   };
   // two voxels (four 16-byte loads) in flight per thread
   const long long stride = (long long)gridDim.x * vpb;
+  const long long row = stride * p.C;
   long long v = (long long)blockIdx.x * vpb + vl;
-  for (; v + stride < p.S; v += 2 * stride) {
-    const uint4 rx0 = __ldg(reinterpret_cast<const uint4*>(p.x + base + v * p.C));
-    const uint4 rd0 = __ldg(reinterpret_cast<const uint4*>(p.dy + base + v * p.C));
-    const uint4 rx1 = __ldg(reinterpret_cast<const uint4*>(p.x + base + (v + stride) * p.C));
-    const uint4 rd1 = __ldg(reinterpret_cast<const uint4*>(p.dy + base + (v + stride) * p.C));
-    body(rx0, rd0, v);
-    body(rx1, rd1, v + stride);
+  long long at = base + v * p.C;
+  for (; v + stride < p.S; v += 2 * stride, at += 2 * row) {
+    const uint4 rx0 = __ldg(reinterpret_cast<const uint4*>(p.x + at));
+    const uint4 rd0 = __ldg(reinterpret_cast<const uint4*>(p.dy + at));
+    const uint4 rx1 = __ldg(reinterpret_cast<const uint4*>(p.x + at + row));
+    const uint4 rd1 = __ldg(reinterpret_cast<const uint4*>(p.dy + at + row));
+    body(rx0, rd0, at);
+    body(rx1, rd1, at + row);
   }
-  for (; v < p.S; v += stride)
-    body(__ldg(reinterpret_cast<const uint4*>(p.x + base + v * p.C)),
-         __ldg(reinterpret_cast<const uint4*>(p.dy + base + v * p.C)), v);
+  for (; v < p.S; v += stride, at += row)
+    body(__ldg(reinterpret_cast<const uint4*>(p.x + at)), __ldg(reinterpret_cast<const uint4*>(p.dy + at)), at);
 }
 
 // ----------------------------------------------------------------------------
@@ -659,10 +679,13 @@ static unsigned int* gn_ticket() {
   return g_gn_ticket_ptr[dev] + (g_gn_ticket_seq.fetch_add(1u) % 256u);
 }
 
+// groups that eight consecutive channels cover: 1, 2 or 4 (gn_channels_ok)
+static int groups_per_octet(const GnParams& p) { return p.C / p.G >= 8 ? 1 : 8 / (p.C / p.G); }
+
 static int apply_blocks(const GnParams& p) {
   const int vpb = GN_THREADS / (p.C / 8);
   long long need = (p.S + vpb - 1) / vpb;
-  long long cap = (148LL * 8 + p.N - 1) / p.N;
+  long long cap = 148LL * GN_WAVE / p.N;  // one wave; more samples than its slots: one block each
   long long b = need < cap ? need : cap;
   return (int)(b < 1 ? 1 : b);
 }
@@ -675,22 +698,22 @@ using namespace sb;
 extern "C" int sb_gn_supported(int C, int G) { return gn_channels_ok(C, G) ? 1 : 0; }
 
 // Splits of a sample's voxels, at least `rows` rows of voxels (one per thread) in each.
-static int gn_nsplit(int N, long long S, int C, int rows) {
+static int gn_nsplit(int N, long long S, int C, int rows, int wave) {
   if (N < 1 || S < 1 || C < 8 || C / 8 > GN_THREADS) return 1;  // unsupported shapes are refused by the launchers
   const long long step = (long long)rows * (GN_THREADS / (C / 8));
   const long long maxs = (S + step - 1) / step;
-  long long want = (148LL * 4 + N - 1) / N;
+  long long want = 148LL * wave / N;  // all samples' splits in one wave
   long long s = want < maxs ? want : maxs;
   if (s > 1024) s = 1024;
   return (int)(s < 1 ? 1 : s);
 }
 
-extern "C" int sb_gn_nsplit(int N, long long S, int C) { return gn_nsplit(N, S, C, 1); }
+extern "C" int sb_gn_nsplit(int N, long long S, int C) { return gn_nsplit(N, S, C, 1, GN_WAVE); }
 
 // Splits of the backward sums (never more than sb_gn_nsplit). Their partials have 2 C floats per split, so with one
 // row of voxels per split a small wide tensor (512 voxels of 1024 channels) would write and read back twice its own
 // bytes; four rows keep them below a quarter of the two tensors that the pass reads.
-extern "C" int sb_gn_bwd_nsplit(int N, long long S, int C) { return gn_nsplit(N, S, C, 4); }
+extern "C" int sb_gn_bwd_nsplit(int N, long long S, int C) { return gn_nsplit(N, S, C, 4, GN_WAVE_SUMS); }
 
 extern "C" int sb_gn_stats(const SbGnArgs* a, cudaStream_t stream) {
   GnParams p;
@@ -716,7 +739,12 @@ extern "C" int sb_gn_bwd_partial(const SbGnArgs* a, cudaStream_t stream) {
   int rc = gn_fill(a, p);
   if (rc) return rc;
   if (p.fin != nullptr && (p.ticket = gn_ticket()) == nullptr) return SB_ERR_DRIVER;
-  gn_bwd_partial_kernel<<<dim3(p.nsplit, p.N), GN_THREADS, 0, stream>>>(p);
+  const dim3 grid(p.nsplit, p.N);
+  switch (groups_per_octet(p)) {
+    case 1: gn_bwd_partial_kernel<1><<<grid, GN_THREADS, 0, stream>>>(p); break;
+    case 2: gn_bwd_partial_kernel<2><<<grid, GN_THREADS, 0, stream>>>(p); break;
+    default: gn_bwd_partial_kernel<4><<<grid, GN_THREADS, 0, stream>>>(p);
+  }
   sb_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }
@@ -726,7 +754,12 @@ extern "C" int sb_gn_bwd_dx(const SbGnArgs* a, cudaStream_t stream) {
   int rc = gn_fill(a, p);
   if (rc) return rc;
   const size_t smem = (size_t)(4 * p.C + 2 * p.G) * sizeof(float);
-  gn_bwd_dx_kernel<<<dim3(apply_blocks(p), p.N), GN_THREADS, smem, stream>>>(p);
+  const dim3 grid(apply_blocks(p), p.N);
+  switch (groups_per_octet(p)) {
+    case 1: gn_bwd_dx_kernel<1><<<grid, GN_THREADS, smem, stream>>>(p); break;
+    case 2: gn_bwd_dx_kernel<2><<<grid, GN_THREADS, smem, stream>>>(p); break;
+    default: gn_bwd_dx_kernel<4><<<grid, GN_THREADS, smem, stream>>>(p);
+  }
   sb_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }
