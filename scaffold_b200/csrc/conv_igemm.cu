@@ -3,13 +3,29 @@
 //   Y[voxel, co] = sum_{tap, ci} X[voxel + off(tap), ci] * Wp[tap][co][ci]
 //
 // Activations are NDHWC bf16. One CTA tile is 128 output voxels (a small brick
-// h x w x d x n, h fastest) by BN output channels. Per K step the producer warp
-// issues ONE 5-D TMA box load of the (shifted) input brick and one 3-D box load
-// of the packed weights; TMA out-of-bounds zero fill is the convolution's zero
-// padding, so no im2col buffer and no padded copy of the activation exists.
+// h x w x d x n; h fastest with the w-shift reuse below, else w fastest) by BN
+// output channels. Per K step the producer warp issues ONE 5-D TMA box load of
+// the (shifted) input brick and one 3-D box load of the packed weights; TMA
+// out-of-bounds zero fill is the convolution's zero padding, so no im2col buffer
+// and no padded copy of the activation exists.
 // A single elected thread issues tcgen05.mma into a TMEM accumulator
 // (double-buffered, so the epilogue of tile i overlaps the main loop of tile
 // i+1); four epilogue warps read TMEM with tcgen05.ld and store bf16.
+//
+// Stores: a lane holds one voxel's channels, so stores from registers touch 32 lines per instruction, and the 1x1x1
+// head, its backward-data and the transposed convolution, which do next to no arithmetic, were bound by them. Each
+// epilogue warp therefore lays its 32 rows x up to 64 channels out in shared memory (two buffers, swizzled: no bank
+// conflicts) and one lane hands the tile to the TMA store, which also clips it at the volume's edges. A 1x1x1 call
+// walks the voxels as one row, so a tile's output is contiguous; a transposed convolution writes through four strided
+// views of the fine grid, one per (kd, kh), where the two kw taps of a voxel are one run of 2*Cout channels.
+// Calls that no TMA box covers (two destinations with a bias or split off the 16-channel grid, unaligned views) keep
+// the stores from registers. At 2 x 128^3, before / after: transposed 128 -> 64 354 / 162 us (671 MB), head 64 -> 16
+// 121 / 117 us, its backward-data 320 / 257 us (its 32-byte rows now bound by the TMA loads).
+//
+// Small volumes: a tile's reduction over 27 taps is one SM's serial work (L2 to one SM is about 60 bytes a clock: 81 us
+// for 512 -> 512 channels at 6 x 5 x 7), so when the tiles leave SMs idle the taps x channel blocks are split over
+// them; the slices leave fp32 partial sums that a second kernel adds in slice order (all such layers of a step at
+// 2 x 44x60x76: 472 / 225 us).
 //
 // W-shift reuse: with rows ordered h-fastest and 8 rows per swizzle atom, a
 // shift of the input by one voxel along w is a shift of the shared-memory start
@@ -54,8 +70,66 @@ struct IgemmParams {
   const float* bias;
   int scatter;  // 1: columns are (tap8, co) of a k2s2 transposed conv
   int sc_cout;
+  uint32_t inv_cout, inv_2cout;  // ceil(2^32 / n): __umulhi(col, inv) = col / n for the columns here (col * n < 2^32)
+  // row order of the brick and of every box: w fastest (plain loads) or h fastest (w-shift reuse)
+  int wfirst;
+  // TMA stores: one map per destination (scatter: per (kd,kh) view); ocols channels x a 32-row sub-brick per store
+  CUtensorMap mapO[4];
+  int ocols;          // 64 / 32 / 16; 0: stores from registers
+  int stg_off;        // staging buffers (4 warps x 2) and then the bias in dynamic shared memory
+  int bias_off, bias_n;
+  // split reduction
+  int splits, k_per_split;
+  float* ws;
   uint32_t* status;
 };
+
+// Position of a work item, (slice, column tile, w, h, d, n) with the slice fastest. A CTA's next item is gridDim.x
+// further: adding that step digit by digit keeps some 2000 clocks of divisions per tile off the producer lane and the
+// epilogue, more than a 1x1x1 tile's loads and stores take.
+struct Walk { int sl, co, w, h, d, n; };
+__device__ __forceinline__ Walk walk_at(const IgemmParams& p, int item) {
+  Walk t;
+  t.sl = item % p.splits; item /= p.splits;
+  t.co = item % p.tiles_co; item /= p.tiles_co;
+  t.w = item % p.tiles_w; item /= p.tiles_w;
+  t.h = item % p.tiles_h; item /= p.tiles_h;
+  t.d = item % p.tiles_d;
+  t.n = item / p.tiles_d;
+  return t;
+}
+__device__ __forceinline__ void walk_step(const IgemmParams& p, Walk& t, const Walk& by) {
+  t.sl += by.sl; t.co += by.co; t.w += by.w; t.h += by.h; t.d += by.d; t.n += by.n;
+  if (t.sl >= p.splits) { t.sl -= p.splits; ++t.co; }
+  if (t.co >= p.tiles_co) { t.co -= p.tiles_co; ++t.w; }
+  if (t.w >= p.tiles_w) { t.w -= p.tiles_w; ++t.h; }
+  if (t.h >= p.tiles_h) { t.h -= p.tiles_h; ++t.d; }
+  if (t.d >= p.tiles_d) { t.d -= p.tiles_d; ++t.n; }
+}
+
+__device__ __forceinline__ void tma_store_5d(const CUtensorMap* m, const void* smem_src, int c0, int c1, int c2, int c3,
+                                             int c4) {
+  asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(m)),
+               "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+// 8 accumulator columns (+ bias) -> 16 bytes of bf16
+__device__ __forceinline__ uint4 pack_octet(const uint32_t* v, const float* bias) {
+  float f[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(v[j]);
+  if (bias) {
+    const float4 a = reinterpret_cast<const float4*>(bias)[0], b = reinterpret_cast<const float4*>(bias)[1];
+    f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
+    f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
+  }
+  uint4 o;
+  o.x = pack_bf16x2(f[0], f[1]); o.y = pack_bf16x2(f[2], f[3]);
+  o.z = pack_bf16x2(f[4], f[5]); o.w = pack_bf16x2(f[6], f[7]);
+  return o;
+}
 
 __global__ void __launch_bounds__(192, 2) igemm_kernel(const __grid_constant__ IgemmParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -88,44 +162,45 @@ __global__ void __launch_bounds__(192, 2) igemm_kernel(const __grid_constant__ I
     tmem_alloc(&tmem_base_s, 256);
     tmem_relinquish();
   }
+  float* bias_s = reinterpret_cast<float*>(smem + p.bias_off);
+  for (int i = threadIdx.x; i < p.bias_n; i += blockDim.x) bias_s[i] = p.bias[i];
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_s;
 
   const int kiters = p.n_outer * p.cblks;
+  const int work = p.num_tiles * p.splits;  // (tile, slice of the reduction), slices fastest
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
       for (int i = 0; i < 8; ++i) tma_prefetch_desc(&p.mapA[i]);
       tma_prefetch_desc(&p.mapB);
-      uint32_t it = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
-        int t = tile;
-        const int co_t = t % p.tiles_co; t /= p.tiles_co;
-        const int w_t = t % p.tiles_w; t /= p.tiles_w;
-        const int h_t = t % p.tiles_h; t /= p.tiles_h;
-        const int d_t = t % p.tiles_d; t /= p.tiles_d;
-        const int n_t = t;
-        const int h0 = h_t * p.TH, w0 = w_t * p.TW, d0 = d_t * p.TD, n0 = n_t * p.TN;
-        const int co0 = co_t * p.BN;
-        for (int o = 0; o < p.n_outer && ok; ++o) {
-          for (int cb = 0; cb < p.cblks; ++cb, ++it) {
-            const int s = it % p.stages;
-            const uint32_t ph = (it / p.stages) & 1u;
-            if (!mbar_wait(&empty_bar[s], ph ^ 1u, abort_flag, p.status, 1)) { ok = false; break; }
-            uint8_t* sa = smem + (size_t)s * p.stage_bytes;
-            uint8_t* sbm = sa + p.a_bytes;
-            mbar_expect_tx(&full_bar[s], (uint32_t)p.tx_bytes);
-            const int second = cb >= p.cblks0 ? 1 : 0;
-            const int mi = p.tap_map[o] + second;
-            const int c = (second ? cb - p.cblks0 : cb) * p.BK;
-            tma_load_5d(sa, &p.mapA[mi], &full_bar[s], c, h0 + p.tap_dh[o], w0 + p.tap_dw[o],
-                        d0 + p.tap_dd[o], n0);
-            tma_load_3d(sbm, &p.mapB, &full_bar[s], cb * p.BK, co0, o * p.KWS * p.KHS);
-          }
+      uint32_t s = 0, ph = 0;
+      const Walk by = walk_at(p, gridDim.x);
+      Walk t = walk_at(p, blockIdx.x);
+      for (int item = blockIdx.x; item < work && ok; item += gridDim.x, walk_step(p, t, by)) {
+        const int h0 = t.h * p.TH, w0 = t.w * p.TW, d0 = t.d * p.TD, n0 = t.n * p.TN;
+        const int co0 = t.co * p.BN;
+        const int k0 = t.sl * p.k_per_split;
+        const int k1 = k0 + p.k_per_split < kiters ? k0 + p.k_per_split : kiters;
+        int o = 0, cb = 0;
+        if (k0 > 0) { o = k0 / p.cblks; cb = k0 - o * p.cblks; }
+        for (int k = k0; k < k1; ++k) {
+          if (!mbar_wait(&empty_bar[s], ph ^ 1u, abort_flag, p.status, 1)) { ok = false; break; }
+          uint8_t* sa = smem + (size_t)s * p.stage_bytes;
+          uint8_t* sbm = sa + p.a_bytes;
+          mbar_expect_tx(&full_bar[s], (uint32_t)p.tx_bytes);
+          const int second = cb >= p.cblks0 ? 1 : 0;
+          const int mi = p.tap_map[o] + second;
+          const int c = (second ? cb - p.cblks0 : cb) * p.BK;
+          const int hc = h0 + p.tap_dh[o], wc = w0 + p.tap_dw[o];
+          tma_load_5d(sa, &p.mapA[mi], &full_bar[s], c, p.wfirst ? wc : hc, p.wfirst ? hc : wc, d0 + p.tap_dd[o], n0);
+          tma_load_3d(sbm, &p.mapB, &full_bar[s], cb * p.BK, co0, o * p.KWS * p.KHS);
+          if (++cb == p.cblks) { cb = 0; ++o; }
+          if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
         }
       }
     }
@@ -149,13 +224,15 @@ __global__ void __launch_bounds__(192, 2) igemm_kernel(const __grid_constant__ I
       const uint32_t s0 = smem_u32(smem);
       uint32_t stage = 0, sph = 0, tcount = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x, ++tcount) {
+      for (int item = blockIdx.x; item < work && ok; item += gridDim.x, ++tcount) {
+        const int k0 = p.splits > 1 ? (item % p.splits) * p.k_per_split : 0;
+        const int k1 = k0 + p.k_per_split < kiters ? k0 + p.k_per_split : kiters;
         const uint32_t buf = tcount & 1u;
         const uint32_t bph = (tcount >> 1) & 1u;
         if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[buf], bph ^ 1u, abort_flag, p.status, 2))) { ok = false; break; }
         tc_fence_after();
         const uint32_t acc = tmem_base + buf * 128u;
-        for (int ki = 0; ki < kiters; ++ki) {
+        for (int ki = 0; ki < k1 - k0; ++ki) {
           if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[stage], sph, abort_flag, p.status, 3))) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = s0 + stage * (uint32_t)p.stage_bytes;
@@ -183,28 +260,101 @@ __global__ void __launch_bounds__(192, 2) igemm_kernel(const __grid_constant__ I
     // -------------------------------- epilogue --------------------------------
     const int q = warp & 3;
     const int row = q * 32 + lane;
-    const int rh = row % p.TH;
-    const int rw = (row / p.TH) % p.TW;
+    const int rh = p.wfirst ? (row / p.TW) % p.TH : row % p.TH;
+    const int rw = p.wfirst ? row % p.TW : (row / p.TH) % p.TW;
     const int rd = (row / (p.TH * p.TW)) % p.TD;
     const int rn = row / (p.TH * p.TW * p.TD);
     uint32_t tcount = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x, ++tcount) {
+    // TMA stores: this warp's two staging buffers; its rows start at the brick position of lane 0
+    const int stg_bytes = 64 * p.ocols;
+    uint8_t* stg = smem + p.stg_off + q * 2 * stg_bytes;
+    const uint32_t row_off = (uint32_t)(lane * p.ocols * 2);
+    const uint32_t swz = p.ocols == 64 ? (uint32_t)(lane & 7) << 4
+                         : p.ocols == 32 ? (uint32_t)((lane >> 1) & 3) << 4 : (uint32_t)((lane >> 2) & 1) << 4;
+    uint32_t nstore = 0;
+    const Walk by = walk_at(p, gridDim.x);
+    Walk t = walk_at(p, blockIdx.x);
+    for (int item = blockIdx.x; item < work && ok; item += gridDim.x, ++tcount, walk_step(p, t, by)) {
       const uint32_t buf = tcount & 1u;
       const uint32_t bph = (tcount >> 1) & 1u;
       if (!mbar_wait(&tfull_bar[buf], bph, abort_flag, p.status, 4)) { ok = false; break; }
       tc_fence_after();
-      int t = tile;
-      const int co_t = t % p.tiles_co; t /= p.tiles_co;
-      const int w_t = t % p.tiles_w; t /= p.tiles_w;
-      const int h_t = t % p.tiles_h; t /= p.tiles_h;
-      const int d_t = t % p.tiles_d; t /= p.tiles_d;
-      const int n_t = t;
-      const int h = h_t * p.TH + rh, w = w_t * p.TW + rw, d = d_t * p.TD + rd, n = n_t * p.TN + rn;
+      const int h = t.h * p.TH + rh, w = t.w * p.TW + rw, d = t.d * p.TD + rd, n = t.n * p.TN + rn;
       const bool valid = (rn < p.TN) && h < p.H && w < p.W && d < p.D && n < p.N;
       const long long vox = (((long long)n * p.D + d) * p.H + h) * p.W + w;
-      const int co0 = co_t * p.BN;
+      const int co0 = t.co * p.BN;
       const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + buf * 128u;
+      if (p.splits > 1) {
+        // fp32 partial sums [slice][voxel][column]; a second kernel adds the slices in order
+        const long long rows_all = (long long)p.N * p.D * p.H * p.W;
+        const int ld = p.tiles_co * p.BN;
+        float* dst = p.ws + ((long long)t.sl * rows_all + vox) * ld + co0;
+        for (int c = 0; c < p.BN; c += 16) {
+          uint32_t v[16];
+          tmem_ld_32x16(tbase + c, v);
+          tmem_ld_wait();
+          if (valid) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              reinterpret_cast<uint4*>(dst + c)[j] = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tempty_bar[buf]);
+        continue;
+      }
+      if (p.ocols > 0) {
+        for (int c = 0; c < p.BN; c += p.ocols, ++nstore) {
+          uint8_t* sbuf = stg + (nstore & 1u) * stg_bytes;
+          // the store before the last one has read this buffer
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          __syncwarp();
+          const int col = co0 + c;
+          // bias: of the column, or of the column's channel within its tap
+          int bcol = p.scatter ? col - (int)__umulhi((uint32_t)col, p.inv_cout) * p.sc_cout : col;
+          if (p.ocols >= 32) {
+            for (int hh = 0; hh < p.ocols; hh += 32) {
+              uint32_t v[32];
+              tmem_ld_32x32(tbase + c + hh, v);
+              tmem_ld_wait();
+#pragma unroll
+              for (int g = 0; g < 4; ++g) {
+                const uint4 o = pack_octet(v + 8 * g, p.bias_n ? bias_s + bcol : nullptr);
+                bcol += 8;
+                if (p.scatter && bcol >= p.sc_cout) bcol = 0;
+                *reinterpret_cast<uint4*>(sbuf + row_off + ((uint32_t)(hh * 2 + g * 16) ^ swz)) = o;
+              }
+            }
+          } else {
+            uint32_t v[16];
+            tmem_ld_32x16(tbase + c, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+              const uint4 o = pack_octet(v + 8 * g, p.bias_n ? bias_s + bcol : nullptr);
+              bcol += 8;
+              if (p.scatter && bcol >= p.sc_cout) bcol = 0;
+              *reinterpret_cast<uint4*>(sbuf + row_off + ((uint32_t)(g * 16) ^ swz)) = o;
+            }
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0 && valid) {  // lane 0's voxel is the sub-brick's first: nothing of a box that starts outside
+            int mi = 0, oc = col;
+            if (p.scatter) { mi = (int)__umulhi((uint32_t)col, p.inv_2cout); oc = col - mi * 2 * p.sc_cout; }
+            else if (col >= p.width0) { mi = 1; oc = col - p.width0; }
+            if (p.scatter || oc < (mi ? p.width1 : p.width0))
+              tma_store_5d(&p.mapO[mi], sbuf, oc, p.wfirst ? w : h, p.wfirst ? h : w, d, n);
+          }
+          __syncwarp();
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tempty_bar[buf]);
+        continue;
+      }
       const int nchunk = (p.BN + 31) / 32;
       for (int ch = 0; ch < nchunk; ++ch) {
         uint32_t v[32];
@@ -273,6 +423,7 @@ __global__ void __launch_bounds__(192, 2) igemm_kernel(const __grid_constant__ I
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[buf]);
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // none pending without TMA stores
   }
 
   // ------------------------------- teardown ---------------------------------
@@ -369,21 +520,63 @@ static void choose_brick(IgemmParams& p, bool shift) {
   p.KHS = 1;
   if (shift) {
     p.TH = 8; p.TW = 16; p.TD = 1; p.TN = 1; p.KWS = 3;
+    p.wfirst = 0;
   } else {
+    // w fastest; of all bricks of 128 voxels with power-of-two edges the one that covers the volume with the fewest
+    // tiles, and of those the one with the longest runs along w
     p.KWS = 1;
-    p.TH = p.H >= 8 ? 8 : pow2_floor(p.H);
-    int rem = 128 / p.TH;
-    p.TW = p.W >= rem ? rem : pow2_floor(p.W);
-    if (p.TW > 16) p.TW = 16;
-    rem = 128 / (p.TH * p.TW);
-    p.TD = p.D >= rem ? rem : pow2_floor(p.D);
-    rem = 128 / (p.TH * p.TW * p.TD);
-    p.TN = p.N >= rem ? rem : pow2_floor(p.N);
+    p.wfirst = 1;
+    long long best = -1;
+    for (int tw = 128; tw >= 1; tw /= 2)
+      for (int th = 128 / tw; th >= 1; th /= 2)
+        for (int td = 128 / (tw * th); td >= 1; td /= 2) {
+          const int tn = 128 / (tw * th * td);
+          const long long tiles = (long long)cdiv(p.W, tw) * cdiv(p.H, th) * cdiv(p.D, td) * cdiv(p.N, tn);
+          if (best < 0 || tiles < best) {
+            best = tiles;
+            p.TW = tw; p.TH = th; p.TD = td; p.TN = tn;
+          }
+        }
   }
   p.tiles_h = cdiv(p.H, p.TH);
   p.tiles_w = cdiv(p.W, p.TW);
   p.tiles_d = cdiv(p.D, p.TD);
   p.tiles_n = cdiv(p.N, p.TN);
+}
+
+// Tensor map of an output (or of one strided view of it) for stores of p.ocols channels x the 32-row sub-brick of a
+// warp. dims / strides in the order C, W, H, D, N.
+static int out_map(const IgemmParams& p, CUtensorMap* m, const void* base, const long long* dims,
+                   const long long* strides) {
+  int left = 32;
+  const int t[4] = {p.wfirst ? p.TW : p.TH, p.wfirst ? p.TH : p.TW, p.TD, p.TN};
+  int box[5] = {p.ocols, 1, 1, 1, 1};
+  for (int i = 0; i < 4; ++i) {
+    box[1 + i] = t[i] < left ? t[i] : left;
+    left /= box[1 + i];
+  }
+  long long dm[5], st[5];
+  for (int i = 0; i < 5; ++i) {
+    const int j = p.wfirst ? i : i == 1 ? 2 : i == 2 ? 1 : i;
+    dm[i] = dims[j];
+    st[i] = strides[j];
+  }
+  return make_map_bf16(m, base, 5, dm, st, box, p.ocols * 2);
+}
+
+// (C, H, W, ...) -> (C, W, H, ...)
+static void w_first(long long* dims, long long* strides, int* box) {
+  const long long d = dims[1], s = strides[1];
+  const int b = box[1];
+  dims[1] = dims[2]; strides[1] = strides[2]; box[1] = box[2];
+  dims[2] = d; strides[2] = s; box[2] = b;
+}
+
+// Channels per TMA store: the widest of 64 / 32 / 16 that never crosses a tile or a destination's end (`run` channels).
+static int store_columns(int bn, int run) {
+  for (int c = 64; c >= 16; c /= 2)
+    if (bn % c == 0 && run % c == 0) return c;
+  return 0;
 }
 
 static int finish_and_launch(IgemmParams& p, int cout_rows, cudaStream_t stream) {
@@ -394,22 +587,34 @@ static int finish_and_launch(IgemmParams& p, int cout_rows, cudaStream_t stream)
   p.a_bytes = ((rows_alloc * rowb + 1023) / 1024) * 1024;
   p.b_bytes = p.KWS * p.KHS * p.BN * rowb;
   p.stage_bytes = ((p.a_bytes + p.b_bytes + 1023) / 1024) * 1024;
-  // Two CTAs per SM when there are tiles for them and three stages fit in half the shared memory: the second
-  // CTA's MMAs and epilogue fill the first one's waits (each CTA allocates 256 of the 512 TMEM columns).
   p.tiles_co = cdiv(cout_rows, p.BN);
   p.num_tiles = p.tiles_co * p.tiles_w * p.tiles_h * p.tiles_d * p.tiles_n;
+  const int kiters = p.n_outer * p.cblks;
+  if (p.splits < 1) p.splits = 1;
+  p.k_per_split = cdiv(kiters, p.splits);
+  if (p.splits > 1) p.ocols = 0;
+  p.bias_n = p.ocols > 0 && p.bias ? (p.scatter ? p.sc_cout : p.width0) : 0;
+  // dynamic shared memory behind the stages: staging buffers (8 of 32 rows), bias
+  const int extra = 8 * 64 * p.ocols + (p.bias_n ? ((cout_rows * 4 + 127) / 128) * 128 : 0);
+  // Two CTAs per SM when there are tiles for them and three stages fit in half the shared memory (two where the
+  // staging buffers take their share and the whole reduction is at most two steps): the second CTA's MMAs and epilogue
+  // fill the first one's waits (each CTA allocates 256 of the 512 TMEM columns).
   const int half = g_smem_limit / 2 - 2048;
-  const bool dual = p.num_tiles > g_sm_count && (half - 1024) / p.stage_bytes >= 3;
-  int st = ((dual ? half : g_smem_limit) - 1024) / p.stage_bytes;
+  const int need = p.ocols > 0 && kiters <= 2 ? 2 : 3;
+  const bool dual = p.num_tiles * p.splits > g_sm_count && (half - 1024 - extra) / p.stage_bytes >= need;
+  int st = ((dual ? half : g_smem_limit) - 1024 - extra) / p.stage_bytes;
   if (st > MAX_STAGES) st = MAX_STAGES;
   if (st < 2) return SB_ERR_SHAPE;
   p.stages = st;
+  p.stg_off = st * p.stage_bytes;
+  p.bias_off = p.stg_off + 8 * 64 * p.ocols;
   // expected transaction bytes are what the two boxes really deliver
   p.tx_bytes = rows_a * rowb + p.b_bytes;
   const IgemmParams& q = p;
   const int slots = dual ? 2 * g_sm_count : g_sm_count;
-  int grid = q.num_tiles < slots ? q.num_tiles : slots;
-  const size_t smem = (size_t)q.stages * q.stage_bytes + 1024;
+  const int work = q.num_tiles * q.splits;
+  int grid = work < slots ? work : slots;
+  const size_t smem = (size_t)q.stages * q.stage_bytes + extra + 1024;
   igemm_kernel<<<grid, 192, smem, stream>>>(q);
   sb_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
@@ -429,13 +634,47 @@ int conv_plane3_launch(const SbConvArgs* a, cudaStream_t stream);
 int conv_plane3_gn_splits(const SbConvArgs* a);
 int conv_small_launch(const SbConvArgs* a, cudaStream_t stream);
 long long conv_small_workspace(const SbConvArgs* a);
+int conv_reduce_slices(const SbConvArgs* a, const float* ws, int splits, cudaStream_t stream);
 }
 
 // fp32 scratch elements sb_conv_fwd wants for this call (0: none)
 static bool automatic(const SbConvArgs* a) { return a->force_plain == 0 || a->force_plain == 4; }
 
+static int block_channels(const SbConvArgs* a) {
+  const int tot = a->src_c[0] + a->src_c[1];
+  int bk = 64;
+  while (bk > 16 && (a->src_c[0] % bk != 0 || tot % bk != 0)) bk /= 2;
+  return a->src_c[0] % bk != 0 || tot % bk != 0 ? 0 : bk;
+}
+
+// Slices of the reduction for a 3x3x3 call on a volume that is too small for the plane kernels (the only calls that
+// reach the generic kernel by themselves). Worth it when at least half of the SMs would idle and a slice keeps eight
+// steps.
+static int generic_splits(const SbConvArgs* a) {
+  if (!automatic(a) || a->ksize != 3 || (a->W >= 16 && a->H >= 8) || a->wpack == nullptr || a->cout_pad % 16) return 1;
+  const int bk = block_channels(a);
+  const int bn = a->cout_pad >= 128 ? 128 : a->cout_pad;
+  if (bk == 0 || a->cout_pad % bn != 0 || device_setup()) return 1;
+  IgemmParams p;
+  p.N = a->N; p.D = a->D; p.H = a->H; p.W = a->W;
+  choose_brick(p, false);
+  const long long tiles = (long long)p.tiles_h * p.tiles_w * p.tiles_d * p.tiles_n * (a->cout_pad / bn);
+  const int kiters = 27 * ((a->src_c[0] + a->src_c[1]) / bk);
+  if (tiles * 2 > g_sm_count || kiters < 32) return 1;
+  int splits = (int)(g_sm_count / tiles);
+  if (splits > kiters / 8) splits = kiters / 8;
+  if (splits > 32) splits = 32;
+  return cdiv(kiters, cdiv(kiters, splits));  // no empty slice
+}
+
+static long long generic_workspace(const SbConvArgs* a, int splits) {
+  return splits < 2 ? 0 : (long long)splits * a->N * a->D * a->H * a->W * a->cout_pad;
+}
+
 extern "C" long long sb_conv_fwd_workspace(const SbConvArgs* a) {
-  return automatic(a) ? conv_small_workspace(a) : 0;
+  if (!automatic(a)) return 0;
+  const long long small = conv_small_workspace(a);
+  return small > 0 ? small : generic_workspace(a, generic_splits(a));
 }
 
 static bool pair_first(const SbConvArgs* a) { return a->force_plain == 0 && a->wpack_kd == nullptr; }
@@ -477,9 +716,8 @@ extern "C" int sb_conv_fwd(const SbConvArgs* a, cudaStream_t stream) {
   memset(&p, 0, sizeof(p));
   const int cin_tot = a->src_c[0] + a->src_c[1];
   const int nsrc = a->src_c[1] > 0 ? 2 : 1;
-  int bk = 64;
-  while (bk > 16 && (a->src_c[0] % bk != 0 || cin_tot % bk != 0)) bk /= 2;
-  if (a->src_c[0] % bk != 0 || cin_tot % bk != 0) return SB_ERR_SHAPE;
+  const int bk = block_channels(a);
+  if (bk == 0) return SB_ERR_SHAPE;
   p.BK = bk;
   p.BN = a->cout_pad >= 128 ? 128 : a->cout_pad;
   if (p.BN % 16 != 0 || a->cout_pad % p.BN != 0) return SB_ERR_SHAPE;
@@ -487,6 +725,16 @@ extern "C" int sb_conv_fwd(const SbConvArgs* a, cudaStream_t stream) {
   p.N = a->N; p.D = a->D; p.H = a->H; p.W = a->W;
   const bool can_shift = a->ksize == 3 && a->W >= 16 && a->H >= 8;
   const bool shift = can_shift && a->force_plain != 1;
+  long long iD = a->in_d ? a->in_d : a->D, iH = a->in_h ? a->in_h : a->H, iW = a->in_w ? a->in_w : a->W;
+  const long long voxels = (long long)a->N * a->D * a->H * a->W;
+  if (a->ksize == 1 && !a->off_d && !a->off_h && !a->off_w && iD == a->D && iH == a->H && iW == a->W &&
+      voxels < 0x7fffff00ll) {
+    // no neighbours: the voxels are one row
+    p.N = p.D = p.H = 1;
+    p.W = (int)voxels;
+    iD = iH = 1;
+    iW = voxels;
+  }
   choose_brick(p, shift);
   if (shift && a->force_plain == 3) p.KHS = 3;
   const int taps = a->ksize * a->ksize * a->ksize;
@@ -506,10 +754,10 @@ extern "C" int sb_conv_fwd(const SbConvArgs* a, cudaStream_t stream) {
   const int rowb = bk * 2;
   for (int s = 0; s < nsrc; ++s) {
     const long long C = a->src_ld[s];
-    const long long iD = a->in_d ? a->in_d : a->D, iH = a->in_h ? a->in_h : a->H, iW = a->in_w ? a->in_w : a->W;
-    long long dims[5] = {a->src_c[s], iH, iW, iD, a->N};
+    long long dims[5] = {a->src_c[s], iH, iW, iD, p.N};
     long long str[5] = {1, iW * C, C, iH * iW * C, iD * iH * iW * C};
     int box[5] = {bk, p.TH + p.KHS - 1, p.TW + p.KWS - 1, p.TD, p.TN};
+    if (p.wfirst) w_first(dims, str, box);
     rc = make_map_bf16(&p.mapA[s], a->src[s], 5, dims, str, box, rowb);
     if (rc) return rc;
   }
@@ -532,6 +780,23 @@ extern "C" int sb_conv_fwd(const SbConvArgs* a, cudaStream_t stream) {
   p.scatter = 0;
   p.sc_cout = 1;
   p.status = a->status;
+  const int splits = generic_splits(a);
+  if (splits > 1 && a->workspace != nullptr && a->workspace_elems >= generic_workspace(a, splits)) {
+    p.splits = splits;
+    p.ws = a->workspace;
+    rc = finish_and_launch(p, a->cout_pad, stream);
+    return rc ? rc : conv_reduce_slices(a, p.ws, splits, stream);
+  }
+  // the bias belongs to the first destination; a destination narrower than its columns is clipped by its map
+  p.ocols = p.out1 ? (p.bias ? 0 : store_columns(p.BN, p.width0)) : store_columns(p.BN, p.BN);
+  if ((reinterpret_cast<uintptr_t>(p.out0) | reinterpret_cast<uintptr_t>(p.out1)) & 15) p.ocols = 0;
+  for (int i = 0; p.ocols > 0 && i < (p.out1 ? 2 : 1); ++i) {
+    const long long C = i ? p.ld1 : p.ld0;
+    const long long dims[5] = {i ? p.width1 : p.width0, p.W, p.H, p.D, p.N};
+    const long long str[5] = {1, C, p.W * C, (long long)p.H * p.W * C, (long long)p.D * p.H * p.W * C};
+    rc = out_map(p, &p.mapO[i], i ? p.out1 : p.out0, dims, str);
+    if (rc) return rc;
+  }
   return finish_and_launch(p, a->cout_pad, stream);
 }
 
@@ -560,6 +825,7 @@ extern "C" int sb_convT_fwd(const SbConvTArgs* a, cudaStream_t stream) {
     long long dims[5] = {a->cin, a->H, a->W, a->D, a->N};
     long long str[5] = {1, (long long)a->W * C, C, (long long)a->H * a->W * C, (long long)a->D * a->H * a->W * C};
     int box[5] = {bk, p.TH, p.TW, p.TD, p.TN};
+    w_first(dims, str, box);
     rc = make_map_bf16(&p.mapA[0], a->src, 5, dims, str, box, rowb);
     if (rc) return rc;
     for (int s = 1; s < 8; ++s) p.mapA[s] = p.mapA[0];
@@ -577,7 +843,18 @@ extern "C" int sb_convT_fwd(const SbConvTArgs* a, cudaStream_t stream) {
   p.bias = a->bias;
   p.scatter = 1;
   p.sc_cout = a->cout;
+  p.inv_cout = (uint32_t)(0xffffffffu / (uint32_t)a->cout + 1u);
+  p.inv_2cout = (uint32_t)(0xffffffffu / (2u * (uint32_t)a->cout) + 1u);
   p.status = a->status;
+  p.ocols = a->dst_ld == a->cout && (reinterpret_cast<uintptr_t>(a->dst) & 15) == 0
+                ? store_columns(p.BN, 2 * a->cout) : 0;
+  for (int o = 0; p.ocols > 0 && o < 4; ++o) {
+    const long long C = a->cout, W2 = 2LL * a->W, H2 = 2LL * a->H, D2 = 2LL * a->D;
+    const long long dims[5] = {2 * C, a->W, a->H, a->D, a->N};
+    const long long str[5] = {1, 2 * C, 2 * W2 * C, 2 * H2 * W2 * C, D2 * H2 * W2 * C};
+    rc = out_map(p, &p.mapO[o], p.out0 + ((o >> 1) * H2 + (o & 1)) * W2 * C, dims, str);
+    if (rc) return rc;
+  }
   return finish_and_launch(p, ncols, stream);
 }
 
@@ -615,6 +892,7 @@ extern "C" int sb_convT_dgrad(const SbConvTArgs* a, cudaStream_t stream) {
     long long dims[5] = {kc, a->H, a->W, a->D, a->N};
     long long str[5] = {1, 2 * W2 * C, 2 * C, 2 * H2 * W2 * C, D2 * H2 * W2 * C};
     int box[5] = {bk, p.TH, p.TW, p.TD, p.TN};
+    w_first(dims, str, box);
     rc = make_map_bf16(&p.mapA[o], base, 5, dims, str, box, rowb);
     if (rc) return rc;
     p.tap_map[o] = (signed char)o;
@@ -633,5 +911,13 @@ extern "C" int sb_convT_dgrad(const SbConvTArgs* a, cudaStream_t stream) {
   p.scatter = 0;
   p.sc_cout = 1;
   p.status = a->status;
+  p.ocols = (reinterpret_cast<uintptr_t>(a->dst) & 15) == 0 && a->dst_ld % 8 == 0 ? store_columns(p.BN, p.BN) : 0;
+  if (p.ocols > 0) {
+    const long long L = a->dst_ld;
+    const long long dims[5] = {a->cin, a->W, a->H, a->D, a->N};
+    const long long str[5] = {1, L, a->W * L, (long long)a->H * a->W * L, (long long)a->D * a->H * a->W * L};
+    rc = out_map(p, &p.mapO[0], a->dst, dims, str);
+    if (rc) return rc;
+  }
   return finish_and_launch(p, rows, stream);
 }

@@ -238,6 +238,8 @@ long long conv_small_workspace(const SbConvArgs* a) {
   return (long long)small_splits(a, g_sm_sms) * a->N * a->D * 64 * a->cout_pad;
 }
 
+int conv_reduce_slices(const SbConvArgs* a, const float* ws, int splits, cudaStream_t stream);
+
 // Returns -1 when the call is not eligible or no workspace was given.
 int conv_small_launch(const SbConvArgs* a, cudaStream_t stream) {
   if (!small_eligible(a)) return -1;
@@ -281,11 +283,17 @@ int conv_small_launch(const SbConvArgs* a, cudaStream_t stream) {
   const size_t smem = (size_t)SM_STAGES * p.stage_bytes + 1024;
   conv_small_kernel<<<grid, 192, smem, stream>>>(p);
   if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
+  sb_count_launch(1);
+  return conv_reduce_slices(a, p.ws, p.splits, stream);
+}
+
+// Adds the [slice][voxel][cout_pad] partial sums of a convolution in slice order into its destinations (+ bias).
+int conv_reduce_slices(const SbConvArgs* a, const float* ws, int splits, cudaStream_t stream) {
   SmallReduceParams r;
   memset(&r, 0, sizeof(r));
-  r.ws = p.ws;
-  r.rows = (long long)a->N * a->D * 64;
-  r.splits = p.splits;
+  r.ws = ws;
+  r.rows = (long long)a->N * a->D * a->H * a->W;
+  r.splits = splits;
   r.cout_pad = a->cout_pad;
   r.out0 = (__nv_bfloat16*)a->dst[0];
   r.out1 = (__nv_bfloat16*)a->dst[1];
@@ -299,7 +307,7 @@ int conv_small_launch(const SbConvArgs* a, cudaStream_t stream) {
   long long blocks = (total + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
   conv_small_reduce_kernel<<<(int)blocks, 256, 0, stream>>>(r);
-  sb_count_launch(2);
+  sb_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }
 

@@ -246,8 +246,8 @@ def conv_same(srcs: Sequence[torch.Tensor], wpack: torch.Tensor, ksize: int,
         else:
             a.gn_groups = 0
     need = _lib.lib().sb_conv_fwd_workspace(C.byref(a))
-    if need > 0:  # kernels that split the reduction keep fp32 partial sums here
-        ws = _workspace(srcs[0].device, need)
+    if need > 0:  # kernels that split the reduction keep fp32 partial sums here (the call's own: streams may overlap)
+        ws = torch.empty(need, dtype=torch.float32, device=srcs[0].device)
         a.workspace, a.workspace_elems = ws.data_ptr(), ws.numel()
     _lib.check(_lib.lib().sb_conv_fwd(C.byref(a), _lib.stream_ptr()), "sb_conv_fwd")
     return outs
