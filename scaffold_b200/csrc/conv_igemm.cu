@@ -107,14 +107,6 @@ __device__ __forceinline__ void walk_step(const IgemmParams& p, Walk& t, const W
   if (t.d >= p.tiles_d) { t.d -= p.tiles_d; ++t.n; }
 }
 
-__device__ __forceinline__ void tma_store_5d(const CUtensorMap* m, const void* smem_src, int c0, int c1, int c2, int c3,
-                                             int c4) {
-  asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];" ::"l"(
-                   reinterpret_cast<uint64_t>(m)),
-               "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
-               : "memory");
-  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
 // 8 accumulator columns (+ bias) -> 16 bytes of bf16
 __device__ __forceinline__ uint4 pack_octet(const uint32_t* v, const float* bias) {
   float f[8];
@@ -309,7 +301,7 @@ __global__ void __launch_bounds__(192, 2) igemm_kernel(const __grid_constant__ I
         for (int c = 0; c < p.BN; c += p.ocols, ++nstore) {
           uint8_t* sbuf = stg + (nstore & 1u) * stg_bytes;
           // the store before the last one has read this buffer
-          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          if (lane == 0) bulk_wait_read_but_one();
           __syncwarp();
           const int col = co0 + c;
           // bias: of the column, or of the column's channel within its tap
@@ -339,7 +331,7 @@ __global__ void __launch_bounds__(192, 2) igemm_kernel(const __grid_constant__ I
               *reinterpret_cast<uint4*>(sbuf + row_off + ((uint32_t)(g * 16) ^ swz)) = o;
             }
           }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          fence_proxy_async();
           __syncwarp();
           if (lane == 0 && valid) {  // lane 0's voxel is the sub-brick's first: nothing of a box that starts outside
             int mi = 0, oc = col;
@@ -348,6 +340,7 @@ __global__ void __launch_bounds__(192, 2) igemm_kernel(const __grid_constant__ I
             if (p.scatter || oc < (mi ? p.width1 : p.width0))
               tma_store_5d(&p.mapO[mi], sbuf, oc, p.wfirst ? w : h, p.wfirst ? h : w, d, n);
           }
+          if (lane == 0) bulk_commit();
           __syncwarp();
         }
         tc_fence_before();
@@ -423,7 +416,7 @@ __global__ void __launch_bounds__(192, 2) igemm_kernel(const __grid_constant__ I
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[buf]);
     }
-    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // none pending without TMA stores
+    if (lane == 0) bulk_wait_all();  // none pending without TMA stores
   }
 
   // ------------------------------- teardown ---------------------------------

@@ -12,6 +12,12 @@
 // are double-buffered; to make two sets fit, channel blocks are 32 wide (64-byte rows, 64B swizzle).
 // Weight taps arrive as [kh][kw][2-kd] boxes of three taps.
 //
+// A stem of at most three channels (STEM) would spend 27 of 32 channels on padding, nine times over: its 64-channel
+// output at 2 x 128^3 took 446 us where writing it takes 85. The staging kernel therefore puts the nine in-plane
+// neighbours x 3 channels of a voxel into the 32 (stage.cu), and what is left here is one (kh, kw) pair: no halo in h
+// and w, three weight taps, 1/9 of the MMAs. The epilogue is what remains: eight warps per SM, TMA stores, 237 us with
+// the statistics and 169 without (32 output channels: 336 before, 183 and 134).
+//
 // Everything else (row-shifted descriptors, TMA zero padding, warp roles, bounded waits, epilogue)
 // is as in conv_plane.cu.
 #include "common.cuh"
@@ -30,6 +36,8 @@ constexpr int P3_MAX_B = 8;
 struct Plane3Params {
   CUtensorMap mapA[2];
   CUtensorMap mapB;
+  CUtensorMap mapO;        // STEM: the output, stored `ocols` channels x 8 h x 4 w (a warp's rows) at a time
+  int ocols_log2, stg_off; // STEM: 4 warps x 2 staging buffers of 32 rows x BN channels
   CUtensorMap mapHalo[4];  // [source * 2 + face]: landing slabs of the depth neighbours' boundary planes
   int BN, TD;
   int bgroup;  // (kh,kw) pairs per weight box: 1, or 3 (a whole kh row, fewer waits) when shared memory allows
@@ -74,9 +82,12 @@ __device__ __forceinline__ P3Job p3_decode(const Plane3Params& p, int job) {
 
 // STATS: the epilogue also writes GroupNorm partials (forward passes only; the variant without them keeps the
 // register count low enough for small co-resident kernels, e.g. the overlapped gradient reduction, during backward)
-template <int TD, bool STATS>
+template <int TD, bool STATS, bool STEM>
 __global__ void __launch_bounds__(224, 2) conv_plane3_kernel(const __grid_constant__ Plane3Params p) {
   constexpr int planes = TD + 2;
+  constexpr int PAIRS = STEM ? 1 : 9;             // (kh, kw) pairs
+  constexpr int LEAD = STEM ? 0 : 1;              // halo of the activation box in h and w
+  constexpr int RH = STEM ? 8 : P3_RH;            // rows per w column of the box
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_b = smem + (size_t)p.nsets * planes * p.a_slot_bytes;
@@ -147,10 +158,10 @@ __global__ void __launch_bounds__(224, 2) conv_plane3_kernel(const __grid_consta
                 halo_ready[face] = true;
               }
               tma_load_5d(smem + (size_t)s * p.a_slot_bytes, &p.mapHalo[second * 2 + face], &a_full[set], c,
-                          jc.h0 - 1 + p.off_h, jc.w0 - 1 + p.off_w, 0, jc.n);
+                          jc.h0 - LEAD + p.off_h, jc.w0 - LEAD + p.off_w, 0, jc.n);
             } else {
-              tma_load_5d(smem + (size_t)s * p.a_slot_bytes, &p.mapA[second], &a_full[set], c, jc.h0 - 1 + p.off_h,
-                          jc.w0 - 1 + p.off_w, dz, jc.n);
+              tma_load_5d(smem + (size_t)s * p.a_slot_bytes, &p.mapA[second], &a_full[set], c, jc.h0 - LEAD + p.off_h,
+                          jc.w0 - LEAD + p.off_w, dz, jc.n);
             }
           }
         }
@@ -165,7 +176,7 @@ __global__ void __launch_bounds__(224, 2) conv_plane3_kernel(const __grid_consta
       for (int job = blockIdx.x; job < p.num_jobs && ok; job += gridDim.x) {
         const P3Job jc = p3_decode(p, job);
         for (int cb = 0; cb < p.cblks && ok; ++cb) {
-          for (int khw = 0; khw < 9; khw += p.bgroup, ++it) {
+          for (int khw = 0; khw < PAIRS; khw += p.bgroup, ++it) {
             const int s = it % p.b_slots;
             const uint32_t ph = (it / p.b_slots) & 1u;
             if (!mbar_wait(&b_empty[s], ph ^ 1u, abort_flag, p.status, 72)) { ok = false; break; }
@@ -184,7 +195,7 @@ __global__ void __launch_bounds__(224, 2) conv_plane3_kernel(const __grid_consta
     // accumulators) are awaited in the middle of step g, behind the N = 192 MMAs already queued.
     const bool leader = elect_one();
     const uint32_t swz = swizzle_code_for(P3_ROWB);
-    const uint32_t a_hi = desc_hi((uint32_t)P3_RH * P3_ROWB, swz);
+    const uint32_t a_hi = desc_hi((uint32_t)RH * P3_ROWB, swz);
     const uint32_t b_hi = desc_hi(8u * P3_ROWB, swz);
     uint32_t idesc[4];
 #pragma unroll
@@ -217,13 +228,13 @@ __global__ void __launch_bounds__(224, 2) conv_plane3_kernel(const __grid_consta
           if (!P3_WAIT(st_a, &a_full[set], (sets2 ? (uses >> 1) : uses) & 1u, 74)) { ok = false; break; }
         }
         const uint32_t a_set = desc_lo(sa0 + set * planes * (uint32_t)p.a_slot_bytes, 16u);
-        for (int khw = 0; khw < 9; ++khw) {
+        for (int khw = 0; khw < PAIRS; ++khw) {
           const int kh = khw / 3, kw = khw - kh * 3;
           tc_fence_after();
           const int sub = p.bgroup == 3 ? kw : 0;             // position of this (kh,kw) pair inside its weight box
           const bool box_done = p.bgroup == 3 ? kw == 2 : true;  // last pair of the box: the next step reads a new slot
           const uint32_t b_lo0 = desc_lo(sb0 + b_slot * (uint32_t)p.b_slot_bytes, 16u) + (uint32_t)sub * 3u * b_tap;
-          const uint32_t a_tap = a_set + (((uint32_t)(kw * P3_RH + kh) * P3_ROWB) >> 4);
+          const uint32_t a_tap = a_set + (((uint32_t)(kw * RH + kh) * P3_ROWB) >> 4);
           const bool first = (cb | khw) == 0;
           uint32_t nb_slot = b_slot + 1, nb_par = b_par;
           if (nb_slot == (uint32_t)p.b_slots) { nb_slot = 0; nb_par ^= 1u; }
@@ -259,10 +270,10 @@ __global__ void __launch_bounds__(224, 2) conv_plane3_kernel(const __grid_consta
             }
             if (half == 0) {
               // look ahead: what the next step reads
-              const bool more = !(last_job && last_cb && khw == 8);
+              const bool more = !(last_job && last_cb && khw == PAIRS - 1);
               if (more) {
                 if (box_done && !P3_WAIT(st_b, &b_full[nb_slot], nb_par, 73)) { ok = false; break; }
-                if (khw == 8) {
+                if (khw == PAIRS - 1) {
                   const uint32_t nu = uses + 1;
                   if (sets2 && !P3_WAIT(st_a, &a_full[nu & 1u], (nu >> 1) & 1u, 74)) { ok = false; break; }
                   if (last_cb && bufs2) {
@@ -276,7 +287,7 @@ __global__ void __launch_bounds__(224, 2) conv_plane3_kernel(const __grid_consta
           if (!ok) break;
           if (leader) {
             if (box_done) tc_commit(&b_empty[b_slot]);
-            if (khw == 8) {
+            if (khw == PAIRS - 1) {
               tc_commit(&set_empty[set]);
               if (last_cb) tc_commit(&tfull[buf]);
             }
@@ -322,6 +333,67 @@ __global__ void __launch_bounds__(224, 2) conv_plane3_kernel(const __grid_consta
 #pragma unroll
         for (int i = 0; i < 16; ++i) { gsum[i] = 0.f; gsq[i] = 0.f; }
       }
+      if constexpr (STEM) {
+        // Little arithmetic, so the stores are the work: a plane's 32 rows go through shared memory (swizzled, two
+        // buffers) and the TMA store, and 32 columns are read from TMEM behind one wait.
+        const uint32_t piece = 64u << p.ocols_log2;  // bytes of 32 rows x ocols channels
+        const uint32_t row = (uint32_t)lane << (p.ocols_log2 + 1);
+        const uint32_t swz = p.ocols_log2 == 6 ? (uint32_t)(lane & 7) << 4
+                             : p.ocols_log2 == 5 ? (uint32_t)((lane >> 1) & 3) << 4 : (uint32_t)((lane >> 2) & 1) << 4;
+#pragma unroll 1
+        for (int t = 0; t < TD; ++t) {
+          const int d = jc.d0 + t;
+          const bool valid = h < p.H && w < p.W && d < p.D;
+          uint8_t* sbuf = smem + p.stg_off + (size_t)(q * 2 + (t & 1)) * 64 * p.BN;
+          if (lane == 0) bulk_wait_read_but_one();
+          __syncwarp();
+          const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + (buf * TD + t) * p.BN;
+          uint32_t v[2][16];
+          if (stats && valid) gcnt += 1.f;
+#pragma unroll
+          for (int ci = 0; ci < 4; ++ci) {
+            if (ci * 16 >= p.BN) break;
+            if (ci % 2 == 0) {
+              tmem_ld_32x16(tbase + ci * 16, v[0]);
+              if (ci * 16 + 16 < p.BN) tmem_ld_32x16(tbase + ci * 16 + 16, v[1]);
+              tmem_ld_wait();
+            }
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+              const int col = ci * 16 + g * 8;
+              float f[8];
+#pragma unroll
+              for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[ci % 2][g * 8 + e]);
+              if (p.bias && jc.co0 + col < p.width0) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) f[e] += p.bias[jc.co0 + col + e];
+              }
+              uint4 o;
+              o.x = pack_bf16x2(f[0], f[1]); o.y = pack_bf16x2(f[2], f[3]);
+              o.z = pack_bf16x2(f[4], f[5]); o.w = pack_bf16x2(f[6], f[7]);
+              if (stats && valid) {
+                const uint32_t w4[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const float lo = __uint_as_float(w4[e] << 16), hi = __uint_as_float(w4[e] & 0xffff0000u);
+                  gsum[ci * 4 + g * 2 + (e >> 1)] += lo + hi;
+                  gsq[ci * 4 + g * 2 + (e >> 1)] += lo * lo + hi * hi;
+                }
+              }
+              const uint32_t in_piece = (uint32_t)(col & ((1 << p.ocols_log2) - 1)) * 2u;
+              *reinterpret_cast<uint4*>(sbuf + (col >> p.ocols_log2) * piece + row + (in_piece ^ swz)) = o;
+            }
+          }
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+            if (valid)  // lane 0's voxel is the box's first; the map clips the rest
+              for (int c = 0; c < p.BN && jc.co0 + c < p.width0; c += 1 << p.ocols_log2)
+                tma_store_5d(&p.mapO, sbuf + (c >> p.ocols_log2) * piece, jc.co0 + c, h, w, d, jc.n);
+            bulk_commit();
+          }
+        }
+      } else
       for (int t = 0; t < TD; ++t) {
         const int d = jc.d0 + t;
         const bool valid = h < p.H && w < p.W && d < p.D;
@@ -394,23 +466,26 @@ __global__ void __launch_bounds__(224, 2) conv_plane3_kernel(const __grid_consta
         }
       }
       if (stats) {
-        // warp sums; every epilogue warp owns 32 rows of the tile and writes its own partial (no cross-warp barrier)
+        // warp sums; every epilogue warp owns 32 rows of the tile and writes its own partial (no cross-warp barrier).
+        // 32 values over 32 lanes: at each step a lane hands over one half of its values and adds the other lane's
+        // sums of the half it keeps, 31 shuffles instead of 160; lane L ends with the total of value L.
+        float val[32];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
+        for (int i = 0; i < 16; ++i) { val[2 * i] = gsum[i]; val[2 * i + 1] = gsq[i]; }
 #pragma unroll
-          for (int o2 = 16; o2 > 0; o2 >>= 1) {
-            gsum[i] += __shfl_xor_sync(0xffffffffu, gsum[i], o2);
-            gsq[i] += __shfl_xor_sync(0xffffffffu, gsq[i], o2);
+        for (int o2 = 16; o2 > 0; o2 >>= 1) {
+          const bool upper = (lane & o2) != 0;
+#pragma unroll
+          for (int i = 0; i < o2; ++i) {
+            const float keep = upper ? val[i + o2] : val[i], give = upper ? val[i] : val[i + o2];
+            val[i] = keep + __shfl_xor_sync(0xffffffffu, give, o2);
           }
         }
 #pragma unroll
         for (int o2 = 16; o2 > 0; o2 >>= 1) gcnt += __shfl_xor_sync(0xffffffffu, gcnt, o2);
         __syncwarp();
-        if (lane == 0) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) { gn_s[q][2 * i] = gsum[i]; gn_s[q][2 * i + 1] = gsq[i]; }
-          gn_s[q][32] = gcnt;
-        }
+        gn_s[q][lane] = val[0];
+        if (lane == 0) gn_s[q][32] = gcnt;
         __syncwarp();
         const int groups_here = p.BN / p.gn_cg;      // groups this channel tile covers (at most 16)
         if (lane < groups_here) {
@@ -434,6 +509,7 @@ __global__ void __launch_bounds__(224, 2) conv_plane3_kernel(const __grid_consta
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[buf]);
     }
+    if (STEM && lane == 0) bulk_wait_all();
     if (p.stall && threadIdx.x == 96) {
       atomicAdd(&p.stall[4], (unsigned long long)(clock64() - ep_begin));
       atomicAdd(&p.stall[5], (unsigned long long)st_f);
@@ -463,11 +539,15 @@ static int p3_setup() {
   int lim = 0, sms = 0;
   cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const void* fns[6] = {(const void*)conv_plane3_kernel<1, false>, (const void*)conv_plane3_kernel<2, false>,
-                        (const void*)conv_plane3_kernel<4, false>, (const void*)conv_plane3_kernel<1, true>,
-                        (const void*)conv_plane3_kernel<2, true>, (const void*)conv_plane3_kernel<4, true>};
-  for (int i = 0; i < 6; ++i)
-    if (cudaFuncSetAttribute(fns[i], cudaFuncAttributeMaxDynamicSharedMemorySize, lim - 2048) != cudaSuccess)
+  const void* fns[12] = {
+      (const void*)conv_plane3_kernel<1, false, false>, (const void*)conv_plane3_kernel<2, false, false>,
+      (const void*)conv_plane3_kernel<4, false, false>, (const void*)conv_plane3_kernel<1, true, false>,
+      (const void*)conv_plane3_kernel<2, true, false>,  (const void*)conv_plane3_kernel<4, true, false>,
+      (const void*)conv_plane3_kernel<1, false, true>,  (const void*)conv_plane3_kernel<2, false, true>,
+      (const void*)conv_plane3_kernel<4, false, true>,  (const void*)conv_plane3_kernel<1, true, true>,
+      (const void*)conv_plane3_kernel<2, true, true>,   (const void*)conv_plane3_kernel<4, true, true>};
+  for (const void* fn : fns)
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, lim - 2048) != cudaSuccess)
       return SB_ERR_DRIVER;
   g_p3_smem = lim - 2048;
   g_p3_sms = sms;
@@ -485,6 +565,10 @@ static int p3_plan(const SbConvArgs* a, Plane3Params& p, bool& dual) {
   if (a->cout_pad % 16 != 0 || (a->cout_pad > 64 && a->cout_pad % 64 != 0)) return -1;
   const int cin_tot = a->src_c[0] + a->src_c[1];
   if (a->src_c[0] % P3_BK != 0 || cin_tot % P3_BK != 0) return -1;
+  if (a->stem && (cin_tot != P3_BK || a->off_d || a->off_h || a->off_w || (a->in_d && a->in_d != a->D) ||
+                  (a->in_h && a->in_h != a->H) || (a->in_w && a->in_w != a->W) || a->halo_land[0][0] ||
+                  a->halo_land[0][1] || a->slab_out[0]))
+    return -1;
   int rc = p3_setup();
   if (rc) return rc;
   memset(&p, 0, sizeof(p));
@@ -493,7 +577,7 @@ static int p3_plan(const SbConvArgs* a, Plane3Params& p, bool& dual) {
   p.tiles_h = cdiv_p3(a->H, 8);
   p.tiles_w = cdiv_p3(a->W, 16);
   p.tiles_co = a->cout_pad / p.BN;
-  p.a_tx = P3_RH * P3_RW * P3_ROWB;
+  p.a_tx = (a->stem ? 8 * 16 : P3_RH * P3_RW) * P3_ROWB;
   p.a_slot_bytes = ((p.a_tx + 511) / 512) * 512;  // the 64-byte swizzle pattern repeats every 512 bytes
   // Deep reductions (>= 4 channel blocks) run two CTAs per SM, each with one plane set and one
   // accumulator buffer: while one CTA's issuing thread sits in a wait, a commit or the turn-around
@@ -511,7 +595,8 @@ static int p3_plan(const SbConvArgs* a, Plane3Params& p, bool& dual) {
     const bool d2 = mode == 0;  // two CTAs per SM first: it wins ties
     const int m_slots = (d2 ? 2 : 1) * g_p3_sms;
     const int m_tmem = d2 ? 256 : 512, m_bufs = d2 ? 1 : 2;
-    const double pref = d2 ? (cblks_all >= 4 ? 1.0 : 0.9) : (cblks_all >= 4 ? 0.93 : 1.0);
+    // (the stem's MMAs are a fraction of its stores: eight epilogue warps per SM instead of four)
+    const double pref = a->stem ? (d2 ? 1.0 : 0.8) : d2 ? (cblks_all >= 4 ? 1.0 : 0.9) : (cblks_all >= 4 ? 0.93 : 1.0);
     for (int cand = 4; cand >= 1; cand /= 2) {
       if (cand > a->D || m_bufs * cand * p.BN > m_tmem) continue;
       const long long jobs = (long long)a->N * cdiv_p3(a->D, cand) * p.tiles_h * p.tiles_w * p.tiles_co;
@@ -566,10 +651,10 @@ int conv_plane3_launch(const SbConvArgs* a, cudaStream_t stream) {
   const int a_bytes = p.nsets * (td + 2) * p.a_slot_bytes;
   // weight boxes of a whole kh row (nine taps) when two of them fit: a third of the waits and commits
   int b_slots = 0;
-  for (p.bgroup = 3; p.bgroup >= 1; p.bgroup -= 2) {
+  for (p.bgroup = a->stem ? 1 : 3; p.bgroup >= 1; p.bgroup -= 2) {
     p.b_tx = 3 * p.bgroup * p.BN * P3_ROWB;
     p.b_slot_bytes = ((p.b_tx + 1023) / 1024) * 1024;
-    b_slots = (budget - 1024 - a_bytes) / p.b_slot_bytes;
+    b_slots = (budget - 1024 - a_bytes - (a->stem ? 512 * p.BN : 0)) / p.b_slot_bytes;
     if (b_slots >= 2) break;
   }
   if (b_slots > P3_MAX_B) b_slots = P3_MAX_B;
@@ -582,13 +667,13 @@ int conv_plane3_launch(const SbConvArgs* a, cudaStream_t stream) {
     const long long iD = a->in_d ? a->in_d : a->D, iH = a->in_h ? a->in_h : a->H, iW = a->in_w ? a->in_w : a->W;
     long long dims[5] = {a->src_c[s], iH, iW, iD, a->N};
     long long str[5] = {1, iW * C, C, iH * iW * C, iD * iH * iW * C};
-    int box[5] = {P3_BK, P3_RH, P3_RW, 1, 1};
+    int box[5] = {P3_BK, a->stem ? 8 : P3_RH, a->stem ? 16 : P3_RW, 1, 1};
     rc = make_map_bf16(&p.mapA[s], a->src[s], 5, dims, str, box, P3_ROWB);
     if (rc) return rc;
   }
   if (nsrc == 1) p.mapA[1] = p.mapA[0];
   {
-    long long dims[3] = {cin_tot, a->cout_pad, 27};
+    long long dims[3] = {cin_tot, a->cout_pad, a->stem ? 3 : 27};
     long long str[3] = {1, cin_tot, (long long)a->cout_pad * cin_tot};
     int box[3] = {P3_BK, p.BN, 3 * p.bgroup};
     rc = make_map_bf16(&p.mapB, a->wpack_kd, 3, dims, str, box, P3_ROWB);
@@ -601,6 +686,19 @@ int conv_plane3_launch(const SbConvArgs* a, cudaStream_t stream) {
   p.ld0 = a->dst_ld[0];
   p.ld1 = a->dst_ld[1];
   if (p.width0 % 8 || p.width1 % 8 || p.ld0 % 8 || p.ld1 % 8) return SB_ERR_SHAPE;
+  size_t stg_bytes = 0;
+  if (a->stem) {
+    if (p.out1 != nullptr || (reinterpret_cast<uintptr_t>(p.out0) & 15)) return SB_ERR_SHAPE;
+    p.ocols_log2 = p.BN % 64 == 0 ? 6 : p.BN % 32 == 0 ? 5 : 4;
+    p.stg_off = a_bytes + p.b_slots * p.b_slot_bytes;  // slots of planes and weights are multiples of 1024 bytes
+    stg_bytes = (size_t)512 * p.BN;
+    const long long C = p.ld0;
+    long long dims[5] = {p.width0, a->H, a->W, a->D, a->N};
+    long long str[5] = {1, a->W * C, C, (long long)a->H * a->W * C, (long long)a->D * a->H * a->W * C};
+    int box[5] = {1 << p.ocols_log2, 8, 4, 1, 1};
+    rc = make_map_bf16(&p.mapO, a->dst[0], 5, dims, str, box, 2 << p.ocols_log2);
+    if (rc) return rc;
+  }
   p.wide = (p.width0 % 16 == 0 && p.width1 % 16 == 0 && p.ld0 % 16 == 0 && p.ld1 % 16 == 0 &&
             (reinterpret_cast<uintptr_t>(p.out0) & 31) == 0 && (reinterpret_cast<uintptr_t>(p.out1) & 31) == 0) ? 1 : 0;
   p.bias = a->bias;
@@ -637,14 +735,19 @@ int conv_plane3_launch(const SbConvArgs* a, cudaStream_t stream) {
                       (reinterpret_cast<uintptr_t>(p.slab_out[1]) & 31) != 0))
     p.wide = 0;
   const int grid = p.num_jobs < slots ? p.num_jobs : slots;
-  const size_t smem = (size_t)a_bytes + (size_t)p.b_slots * p.b_slot_bytes + 1024;
-  if (p.gn_part != nullptr) {
-    if (td == 4) conv_plane3_kernel<4, true><<<grid, 224, smem, stream>>>(p);
-    else if (td == 2) conv_plane3_kernel<2, true><<<grid, 224, smem, stream>>>(p);
-    else conv_plane3_kernel<1, true><<<grid, 224, smem, stream>>>(p);
-  } else if (td == 4) conv_plane3_kernel<4, false><<<grid, 224, smem, stream>>>(p);
-  else if (td == 2) conv_plane3_kernel<2, false><<<grid, 224, smem, stream>>>(p);
-  else conv_plane3_kernel<1, false><<<grid, 224, smem, stream>>>(p);
+  const size_t smem = (size_t)a_bytes + (size_t)p.b_slots * p.b_slot_bytes + 1024 + stg_bytes;
+  typedef void (*Kernel)(const Plane3Params);
+  const bool st = p.gn_part != nullptr;
+  Kernel fn;
+  if (a->stem)
+    fn = td == 4 ? (st ? conv_plane3_kernel<4, true, true> : conv_plane3_kernel<4, false, true>)
+       : td == 2 ? (st ? conv_plane3_kernel<2, true, true> : conv_plane3_kernel<2, false, true>)
+                 : (st ? conv_plane3_kernel<1, true, true> : conv_plane3_kernel<1, false, true>);
+  else
+    fn = td == 4 ? (st ? conv_plane3_kernel<4, true, false> : conv_plane3_kernel<4, false, false>)
+       : td == 2 ? (st ? conv_plane3_kernel<2, true, false> : conv_plane3_kernel<2, false, false>)
+                 : (st ? conv_plane3_kernel<1, true, false> : conv_plane3_kernel<1, false, false>);
+  fn<<<grid, 224, smem, stream>>>(p);
   sb_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }

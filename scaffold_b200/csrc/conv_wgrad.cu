@@ -10,6 +10,12 @@
 // of the start address by one atom, so one halo'd box of Q serves the three kw
 // taps, which accumulate into three TMEM accumulators.
 //
+// Stem of at most three channels: x holds the nine in-plane neighbours x channels of a voxel in 32 channels
+// (stage.cu), so the gradient is three kd taps: the N side is the 32 channels of planes d-1, d, d+1, three boxes back to
+// back, ONE 64 x 96 x 16 MMA per 16 voxels, one read of gy. Blocks walk along d so that the three planes are read from
+// L2. 3 -> 64 channels at 2 x 128^3: 407 us as 27 taps of padded channels, now 185 (805 MB; the TMA takes a 64-byte row
+// every three clocks or so, 512 rows a block).
+//
 // Split-K is deterministic: the voxel blocks are cut into `splits` contiguous
 // ranges, every CTA writes its fp32 partial to a workspace slice, and
 // wgrad_reduce_kernel adds the slices in index order while permuting into the
@@ -41,6 +47,7 @@ struct WgradParams {
   int m_tiles, n_tiles, m_tiles0, n_tiles0;  // tiles in total / in the first source of that side
   int splits, blocks_per_split;
   int stages, stage_bytes, m_bytes, boxm_bytes, boxn_bytes, tx_bytes;
+  int stem;  // the N boxes are the planes d-1, d, d+1 of one 32-channel block
   int m_off_d, m_off_h, m_off_w;  // added to the M-side box origin (halo'd x on the M side)
   signed char o_map[16], o_dd[16], o_dh[16], o_dw[16];
   int Mtot, Ntot, T;  // workspace extents: ws[split][T][Mtot][Ntot]
@@ -104,9 +111,11 @@ __global__ void __launch_bounds__(192, 1) wgrad_kernel(const __grid_constant__ W
         const uint32_t ph = (i / p.stages) & 1u;
         if (!mbar_wait(&empty_bar[s], ph ^ 1u, abort_flag, p.status, 11)) break;
         int b = blk_begin + i;
+        int d = 0;
+        if (p.stem) { d = b % p.D; b /= p.D; }
         const int wt = b % p.tiles_w; b /= p.tiles_w;
         const int ht = b % p.tiles_h; b /= p.tiles_h;
-        const int d = b % p.D; b /= p.D;
+        if (!p.stem) { d = b % p.D; b /= p.D; }
         const int n = b;
         const int h0 = ht * 8, w0 = wt * p.TW;
         uint8_t* sm = smem + (size_t)s * p.stage_bytes;
@@ -116,8 +125,8 @@ __global__ void __launch_bounds__(192, 1) wgrad_kernel(const __grid_constant__ W
           tma_load_5d(sm + (size_t)j * p.boxm_bytes, mm, &full_bar[s], mc0 + j * p.CBm, h0 + p.m_off_h,
                       w0 + p.m_off_w, d + p.m_off_d, n);
         for (int j = 0; j < p.n_boxes; ++j)
-          tma_load_5d(sn + (size_t)j * p.boxn_bytes, mn, &full_bar[s], nc0 + j * p.CBn, h0 + p.o_dh[o],
-                      w0 + p.o_dw[o], d + p.o_dd[o], n);
+          tma_load_5d(sn + (size_t)j * p.boxn_bytes, mn, &full_bar[s], p.stem ? 0 : nc0 + j * p.CBn, h0 + p.o_dh[o],
+                      w0 + p.o_dw[o], p.stem ? d + j - 1 : d + p.o_dd[o], n);
       }
     }
   } else if (warp == 1) {
@@ -213,6 +222,7 @@ __global__ void __launch_bounds__(192, 1) wgrad_kernel(const __grid_constant__ W
 //   mode 0: conv,  M side = gy (m = co, n = ci)   dw[co][ci][tap]
 //   mode 1: conv,  M side = x  (m = ci, n = co)   dw[co][ci][tap]
 //   mode 2: convT, M side = x  (m = ci, n = kw*cout+co), T = 4 -> dw[ci][co][kd][kh][kw]
+//   mode 3: stem,  M side = gy (m = co, n = kd*32 + (kh*3+kw)*cin + ci), T = 1 -> dw[co][ci][tap]
 struct ReduceParams {
   const float* ws;
   float* dw;
@@ -229,10 +239,16 @@ __device__ __forceinline__ int wg_swap_tap(int tap, int mode) {
   return mode == 1 ? (kh * 9 + kd * 3 + kw) : (kw * 9 + kh * 3 + kd);
 }
 
-__global__ void wgrad_reduce_kernel(const ReduceParams p) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= p.total) return;
-  int tap, m, n;
+// SL threads share an output, each adds every SL-th slice and the first adds their sums in order: a small weight has few
+// outputs and some 150 slices, which one thread would walk at one L2 latency after the other.
+template <int SL>
+__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const ReduceParams p) {
+  constexpr int OUT = 256 / SL;
+  __shared__ float part[SL][OUT];
+  const int sl = threadIdx.x / OUT;
+  const long long idx = (long long)blockIdx.x * OUT + threadIdx.x % OUT;
+  const bool live = idx < p.total;
+  int tap = 0, m = 0, n = 0;
   if (p.mode == 2) {
     // dw[ci][co][kd][kh][kw]
     const int t8 = (int)(idx % 8);
@@ -242,6 +258,10 @@ __global__ void wgrad_reduce_kernel(const ReduceParams p) {
     tap = kd * 2 + kh;
     m = ci;
     n = kw * p.cout + co;
+  } else if (p.mode == 3) {
+    const int t = (int)(idx % 27), ci = (int)((idx / 27) % p.cin);
+    m = (int)(idx / (27LL * p.cin));
+    n = t / 9 * 32 + (t % 9) * p.cin + ci;
   } else {
     tap = (int)(idx % p.taps);
     if (p.taps == 27) tap = wg_swap_tap(tap, p.tap_swap);  // idx walks the parameter's order; ws holds the kernels'
@@ -252,7 +272,17 @@ __global__ void wgrad_reduce_kernel(const ReduceParams p) {
   const size_t slice = (size_t)p.T * p.Mtot * p.Ntot;
   const float* src = p.ws + ((size_t)tap * p.Mtot + m) * p.Ntot + n;
   float acc = 0.f;
-  for (int s = 0; s < p.splits; ++s) acc += src[(size_t)s * slice];
+  if (live) {
+#pragma unroll 4
+    for (int s = sl; s < p.splits; s += SL) acc += src[(size_t)s * slice];
+  }
+  if (SL > 1) {
+    part[sl][threadIdx.x % OUT] = acc;
+    __syncthreads();
+    if (sl > 0) return;
+    for (int k = 1; k < SL; ++k) acc += part[k][threadIdx.x];
+  }
+  if (!live) return;
   if (p.accumulate) acc += p.dw[idx];
   p.dw[idx] = acc;
 }
@@ -392,10 +422,15 @@ static int build_plan(const SbWgradArgs* a, Plan& pl, bool maps) {
   const bool convT = a->ksize == 2;
   if (!(a->ksize == 1 || a->ksize == 2 || a->ksize == 3)) return SB_ERR_SHAPE;
   if (xc % 16 || gc % 16) return SB_ERR_SHAPE;
+  const bool stem = a->stem != 0;
+  if (stem && (a->ksize != 3 || xc != 32 || a->x_c[1] || a->dw_cin > 3 || a->tap_swap || a->xoff_d || a->xoff_h ||
+               a->xoff_w || a->xhalo[0][0] || a->xhalo[0][1]))
+    return SB_ERR_SHAPE;
   p.N = a->N; p.D = a->D; p.H = a->H; p.W = a->W;
   // which tensor sits on the M side (needs >= 64 channels to fill the MMA rows)
   bool m_is_x;
   if (convT) m_is_x = true;
+  else if (stem) m_is_x = false;
   else if (gc >= 128) m_is_x = false;
   else if (xc >= 128) m_is_x = true;
   else m_is_x = gc < 64 && xc >= 64;
@@ -416,23 +451,25 @@ static int build_plan(const SbWgradArgs* a, Plan& pl, bool maps) {
   if (p.NT < 64 && nc_full != p.NT) return SB_ERR_SHAPE;
   p.CBn = box_c(p.NT);
   p.n_boxes = p.NT / p.CBn;
+  if (stem) { p.stem = 1; p.NT = 96; p.CBn = 32; p.n_boxes = 3; }
   p.m_tiles = mc / p.MT;
   p.m_tiles0 = m_first / p.MT;
-  p.n_tiles = nc_full / p.NT;
-  p.n_tiles0 = n_first / p.NT;
+  p.n_tiles = stem ? 1 : nc_full / p.NT;
+  p.n_tiles0 = stem ? 1 : n_first / p.NT;
   // voxel blocks: 8 h x TW w
   p.TW = a->W >= 16 ? 16 : (a->W >= 8 ? 8 : (a->W >= 4 ? 4 : 2));
   p.KV = 8 * p.TW;
   p.tiles_h = cdiv(a->H, 8);
   p.tiles_w = cdiv(a->W, p.TW);
   p.nblocks = a->N * a->D * p.tiles_h * p.tiles_w;
-  p.KWS = a->ksize == 3 ? 3 : 1;
-  p.n_outer = a->ksize == 3 ? 9 : (convT ? 4 : 1);
-  p.T = a->ksize == 3 ? 27 : (convT ? 4 : 1);
+  const bool taps27 = a->ksize == 3 && !stem;
+  p.KWS = taps27 ? 3 : 1;
+  p.n_outer = taps27 ? 9 : (convT ? 4 : 1);
+  p.T = taps27 ? 27 : (convT ? 4 : 1);
   p.flip = (!convT && m_is_x) ? 1 : 0;  // shifted tensor is gy: accumulator j <-> kw = 2-j
   const int sign = p.flip ? -1 : 1;
   for (int o = 0; o < p.n_outer; ++o) {
-    if (a->ksize == 3) {
+    if (taps27) {
       const int kd = o / 3, kh = o % 3;
       p.o_map[o] = 0;
       p.o_dd[o] = (signed char)(sign * (kd - 1));
@@ -443,7 +480,7 @@ static int build_plan(const SbWgradArgs* a, Plan& pl, bool maps) {
     }
   }
   p.Mtot = mc;
-  p.Ntot = nc_full;
+  p.Ntot = stem ? 96 : nc_full;
   const int base_ctas = p.n_outer * p.m_tiles * p.n_tiles;
   int sms = g_wg_sms > 0 ? g_wg_sms : 148;
   int splits = a->splits > 0 ? a->splits : (sms + base_ctas - 1) / base_ctas;
@@ -462,7 +499,7 @@ static int build_plan(const SbWgradArgs* a, Plan& pl, bool maps) {
   // reduce
   ReduceParams& r = pl.r;
   r.splits = p.splits; r.T = p.T; r.Mtot = p.Mtot; r.Ntot = p.Ntot;
-  r.mode = convT ? 2 : (m_is_x ? 1 : 0);
+  r.mode = convT ? 2 : stem ? 3 : (m_is_x ? 1 : 0);
   r.accumulate = a->accumulate;
   if (!maps) return 0;
 
@@ -547,7 +584,7 @@ int wgrad_plane_launch(const SbWgradArgs* a, cudaStream_t stream, int* splits_ou
 
 // a->splits < 0 forces the generic kernel (tests); >= 0 prefers the plane kernel when eligible
 extern "C" long long sb_conv_wgrad_workspace(const SbWgradArgs* a) {
-  if (a->splits >= 0) {
+  if (a->splits >= 0 && !a->stem) {
     const long long w = wgrad_plane_workspace(a);
     if (w >= 0) return w;
   }
@@ -578,15 +615,17 @@ static int run_reduce(const SbWgradArgs* a, ReduceParams& r, cudaStream_t stream
     while (ct > 32 && (long long)(r.cin / ct) * r.cout < 296) ct /= 2;
     if (r.splits >= 4) wgrad_reduce_t_kernel<true><<<dim3(r.cin / ct, r.cout), threads, 0, stream>>>(r, ct);
     else wgrad_reduce_t_kernel<false><<<dim3(r.cin / ct, r.cout), threads, 0, stream>>>(r, ct);
-  } else
-    wgrad_reduce_kernel<<<(unsigned)blocks, threads, 0, stream>>>(r);
+  } else if (r.splits >= 16)
+    wgrad_reduce_kernel<8><<<(unsigned)((r.total + 31) / 32), threads, 0, stream>>>(r);
+  else
+    wgrad_reduce_kernel<1><<<(unsigned)blocks, threads, 0, stream>>>(r);
   sb_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }
 
 extern "C" int sb_conv_wgrad(const SbWgradArgs* a, cudaStream_t stream) {
   int rc;
-  if (a->splits >= 0) {
+  if (a->splits >= 0 && !a->stem) {
     int splits = 0;
     rc = wgrad_plane_launch(a, stream, &splits);
     if (rc > 0) return rc;

@@ -64,6 +64,9 @@ typedef struct {
   // so the normalisation that follows skips its own pass over the tensor.
   float* gn_part;
   int gn_groups;
+  // Stem of at most three channels (ksize 3, one source from sb_stage_stem): the source's 32 channels are the nine
+  // in-plane neighbours x channels of a voxel, wpack_kd is sb_pack_stem's [3][cout_pad][32]. kd-fused kernel only.
+  int stem;
 } SbConvArgs;
 
 // One pass over fp32 3x3x3 weights [cout][cin][27] -> bf16 operand layouts (null = not wanted):
@@ -128,6 +131,7 @@ typedef struct {
   // same exchange as SbPackArgs.tap_swap (3x3x3 only): the gradient is computed in the kernels' tap order and
   // stored into dw in the parameter's own order
   int tap_swap;
+  int stem;  // x is sb_stage_stem's tensor (32 channels, see SbConvArgs.stem); dw_cin is the real channel count
 } SbWgradArgs;
 
 // GroupNorm (+ReLU), channels-last bf16. `parts` lists the partial-statistics

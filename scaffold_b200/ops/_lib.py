@@ -57,6 +57,7 @@ class SbConvArgs(C.Structure):
         ("workspace_elems", C.c_longlong),
         ("gn_part", C.c_void_p),
         ("gn_groups", C.c_int),
+        ("stem", C.c_int),
     ]
 
 
@@ -108,6 +109,7 @@ class SbWgradArgs(C.Structure):
         ("xoff_d", C.c_int), ("xoff_h", C.c_int), ("xoff_w", C.c_int),
         ("xhalo", (C.c_void_p * 2) * 2),
         ("tap_swap", C.c_int),
+        ("stem", C.c_int),
     ]
 
 
@@ -150,6 +152,8 @@ _SIGNATURES = {
     "sb_pack_conv3": ([C.POINTER(SbPackArgs), _P], C.c_int),
     "sb_pack_conv3_plan": ([C.POINTER(SbPackJob), C.c_int], C.c_longlong),
     "sb_pack_conv3_batch": ([_P, C.c_int, C.c_longlong, _P], C.c_int),
+    "sb_stage_stem": ([_P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P, _P], C.c_int),
+    "sb_pack_stem": ([_P, C.c_int, C.c_int, C.c_int, _P, _P], C.c_int),
     "sb_stage_input": ([_P, C.c_int, C.c_int, C.c_int, C.c_longlong, _P, C.c_int, _P], C.c_int),
     "sb_colsum_blocks": ([], C.c_int),
     "sb_colsum": ([_P, C.c_longlong, C.c_int, _P, C.c_int, _P, C.c_int, _P], C.c_int),

@@ -293,6 +293,44 @@ class _ConvSameFn(torch.autograd.Function):
         return (gw, gb, None, None, None, *gxs)
 
 
+class _StemFn(torch.autograd.Function):
+    """3x3x3 conv over the network input (at most three channels, no gradient of its own), staged as in-plane
+    neighbourhoods; nothing but the staged copy is kept for backward."""
+
+    @staticmethod
+    def forward(ctx, weight, bias, mod, x):
+        xs = ck.stage_stem(x)
+        wf = mod._cache.get(weight, "stem", ck.pack_stem)
+        cout_pad = wf.shape[1]
+        bpad = None
+        if bias is not None:
+            bpad = mod._cache_b.get(bias, "b", lambda b: F.pad(b, (0, cout_pad - b.shape[0])).contiguous())
+        sink = []
+        gn = mod.gn_groups_hint if (_GN_FROM_EPILOGUE and cout_pad == weight.shape[0]) else 0
+        (y,) = ck.conv_same([xs], wf, 3, [cout_pad], bias=bpad, gn_groups=gn, gn_sink=sink, stem=True)
+        mod._gn_partials = sink[0] if sink else None
+        ctx.wparam, ctx.bparam = weight, bias
+        ctx.save_for_backward(weight, xs)
+        return y
+
+    @staticmethod
+    def backward(ctx, gy):
+        weight, xs = ctx.saved_tensors
+        gy = gy.contiguous()
+        gw = gb = None
+        if ctx.needs_input_grad[0]:
+            direct = direct_grad_target(ctx.wparam)
+            if direct is not None:
+                ck.conv_wgrad(gy, [xs], 3, direct, accumulate=True, stem=True)
+                notify_grad_written(ctx.wparam)
+            else:
+                gw = torch.empty(weight.shape, dtype=torch.float32, device=weight.device)
+                ck.conv_wgrad(gy, [xs], 3, gw, stem=True)
+        if ctx.bparam is not None and ctx.needs_input_grad[1]:
+            gb = _bias_grad(gy, weight.shape[0], ctx.bparam)
+        return gw, gb, None, None
+
+
 class _ConvHaloFn(torch.autograd.Function):
     """3x3x3 conv on a depth-sharded volume with the halo fused into the kernels (no padded copy)."""
 
@@ -424,12 +462,18 @@ class Conv3d(nn.Conv3d):
             halo = self.kernel_size[0] // 2
             xs = [sp.halo_pad(t, halo) for t in xs]
             off = tuple(halo if d in sp.dims else 0 for d in (2, 3, 4))
+        x = xs[0]
+        if (len(xs) == 1 and self.kernel_size[0] == 3 and sp is None and x.dim() == 5 and not x.requires_grad
+                and x.is_contiguous() and x.dtype in (torch.float32, torch.bfloat16)
+                and x.shape[1] == self.in_channels
+                and ck.stem_eligible(self.in_channels, ck.pad_channels(self.out_channels), x.shape[2:])):
+            return _StemFn.apply(self.weight, self.bias, self, x)
         vms = [to_vm(t, pad16=True) for t in xs]
         fwd_vms = None
         if (len(xs) == 1 and self.kernel_size[0] == 3 and self.in_channels < 16 and not xs[0].requires_grad
                 and vms[0].shape[2] >= 8 and vms[0].shape[3] >= 16):
-            # few input channels (the stem): the forward pass reads a copy padded to 32 channels so that it runs
-            # the kd-fused kernel; the weight gradient keeps the 16-channel copy
+            # few input channels (a stem of four and more, or sharded): the forward pass reads a copy padded to 32
+            # channels so that it runs the kd-fused kernel; the weight gradient keeps the 16-channel copy
             fwd_vms = (to_vm(xs[0], pad16=True, pad_to=32),)
         return _ConvSameFn.apply(self.weight, self.bias, self, off, fwd_vms, *vms)
 

@@ -126,6 +126,35 @@ def fill_pack_args(a, wc: torch.Tensor, src_c: Sequence[int], real_c: Sequence[i
         setattr(a, name, t.data_ptr() if t is not None else None)
 
 
+STEM_CHANNELS = 32  # nine in-plane neighbours x up to three channels, padded
+
+
+def stem_eligible(cin: int, rows: int, dims: Sequence[int]) -> bool:
+    """True when a 3x3x3 layer over a ``cin``-channel network input runs on its staged in-plane neighbourhoods."""
+    _, h, w = dims
+    return 1 <= cin <= 3 and h >= 8 and w >= 16 and rows % 16 == 0 and (rows <= 64 or rows % 64 == 0)
+
+
+def stage_stem(x: torch.Tensor) -> torch.Tensor:
+    """Contiguous fp32 / bf16 ``[N, C <= 3, D, H, W]`` -> bf16 ``[N, D, H, W, 32]``: channel (kh * 3 + kw) * C + c is
+    the voxel's (kh, kw) neighbour in its plane."""
+    n, c, d, h, w = x.shape
+    y = torch.empty((n, d, h, w, STEM_CHANNELS), dtype=torch.bfloat16, device=x.device)
+    _lib.check(_lib.lib().sb_stage_stem(x.data_ptr(), int(x.dtype == torch.bfloat16), n, c, d, h, w, y.data_ptr(),
+                                        _lib.stream_ptr()), "sb_stage_stem")
+    return y
+
+
+def pack_stem(w: torch.Tensor) -> torch.Tensor:
+    """fp32 ``[Cout, C <= 3, 3, 3, 3]`` -> bf16 ``[3, cout_pad, 32]``, planes in the order 2 - kd."""
+    w = w.contiguous()
+    co, ci = w.shape[:2]
+    out = torch.empty((3, pad_channels(co), STEM_CHANNELS), dtype=torch.bfloat16, device=w.device)
+    _lib.check(_lib.lib().sb_pack_stem(w.data_ptr(), co, pad_channels(co), ci, out.data_ptr(), _lib.stream_ptr()),
+               "sb_pack_stem")
+    return out
+
+
 def bias_grad(gy: torch.Tensor, n_out: int, into: Optional[torch.Tensor] = None) -> torch.Tensor:
     """fp32 sum of a voxel-major bf16 gradient ``[..., C]`` over all voxels, first ``n_out`` channels (added to
     ``into`` when given)."""
@@ -168,7 +197,7 @@ def conv_same(srcs: Sequence[torch.Tensor], wpack: torch.Tensor, ksize: int,
               force_plain: bool = False, out: Optional[Sequence[torch.Tensor]] = None,
               out_dims: Optional[Sequence[int]] = None, in_off: Sequence[int] = (0, 0, 0), halo=None,
               slabs: Optional[Sequence[torch.Tensor]] = None, kd_fused: bool = True, gn_groups: int = 0,
-              gn_sink: Optional[list] = None):
+              gn_sink: Optional[list] = None, stem: bool = False):
     """Stride-1 'same' convolution of the channel concatenation of ``srcs``.
 
     Returns a list of outputs, one per entry of ``dst_channels`` (the output
@@ -179,6 +208,7 @@ def conv_same(srcs: Sequence[torch.Tensor], wpack: torch.Tensor, ksize: int,
     ``gn_groups`` > 0 asks the kernel to also produce the GroupNorm statistics of its output (groups over
     the padded output channels); when the call can (kd-fused kernel, one destination) the triple
     ``(partials, splits, groups)`` is appended to ``gn_sink``, the input of :func:`gn_kernels.gn_finalize`.
+    ``stem``: the source comes from :func:`stage_stem`, ``wpack`` from :func:`pack_stem`.
     """
     for s in srcs:
         _chk_act(s)
@@ -198,7 +228,10 @@ def conv_same(srcs: Sequence[torch.Tensor], wpack: torch.Tensor, ksize: int,
     a.in_d, a.in_h, a.in_w = srcs[0].shape[1:4]
     a.off_d, a.off_h, a.off_w = (int(v) for v in in_off)
     a.ksize = ksize
-    if isinstance(wpack, Packed):
+    a.stem = int(stem)
+    if stem:
+        std, kd = None, wpack
+    elif isinstance(wpack, Packed):
         std, kd = wpack.std, (wpack.kd if kd_fused else None)
     else:
         std, kd = wpack, (getattr(wpack, "kd_order", None) if kd_fused else None)
@@ -305,10 +338,11 @@ def _workspace(device, elems: int) -> torch.Tensor:
 
 def conv_wgrad(gy: torch.Tensor, xs: Sequence[torch.Tensor], ksize: int, dw: torch.Tensor,
                accumulate: bool = False, splits: int = 0, x_off: Sequence[int] = (0, 0, 0),
-               x_halo=None, tap_swap: int = 0) -> torch.Tensor:
+               x_halo=None, tap_swap: int = 0, stem: bool = False) -> torch.Tensor:
     """Weight gradient into ``dw`` (fp32, parameter layout).
 
     ksize 1/3: ``dw`` is [Cout, Cin, k,k,k]; ``gy`` and ``xs`` share the voxel grid.
+    ``stem``: ``xs`` is one tensor from :func:`stage_stem`.
     ksize 2:   k2s2 transposed conv, ``dw`` is [Cin, Cout, 2,2,2]; ``gy`` is on the fine grid.
     """
     _chk_act(gy)
@@ -333,6 +367,7 @@ def conv_wgrad(gy: torch.Tensor, xs: Sequence[torch.Tensor], ksize: int, dw: tor
             for f in range(2):
                 a.xhalo[si][f] = pair[f].data_ptr() if pair[f] is not None else None
     a.ksize = ksize
+    a.stem = int(stem)
     a.splits = splits
     a.tap_swap = int(tap_swap) if ksize == 3 else 0
     a.accumulate = 1 if accumulate else 0

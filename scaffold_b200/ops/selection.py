@@ -57,13 +57,20 @@ def kernel_selection(model: nn.Module, batch: int, local_dims: Sequence[int], sp
             p = ConvProblem(n, c, mod.out_channels, (d, h, w), kernel=mod.kernel_size[0], split_cin=split)
             halo = _halo_mode(mod, spatial, split or (p.kernel_variant().cin,), (d, h, w))
         fwd, dgrad = p.route("fwd", ck.PAIR_CONV), p.route("dgrad", ck.PAIR_CONV)
+        wgrad = p.route("wgrad")
         if not p.transposed and c < 16:
-            # the stem: its forward pass reads a copy padded to 32 channels, and the network input needs no gradient
-            fwd = ConvProblem(n, 32, mod.out_channels, (d, h, w), kernel=p.kernel).route("fwd") + " (32-ch padded input)"
+            # the stem reads a staged copy of 32 channels (in-plane neighbours, or padding), and the network input needs
+            # no gradient
+            staged = p.kernel == 3 and spatial is None and ck.stem_eligible(c, ck.pad_channels(mod.out_channels),
+                                                                            (d, h, w))
+            fwd = ConvProblem(n, 32, mod.out_channels, (d, h, w), kernel=p.kernel).route("fwd")
+            fwd += " (32-ch input of in-plane neighbours)" if staged else " (32-ch padded input)"
             dgrad = "-"
+            if staged:
+                wgrad = "wgrad(generic, in-plane neighbours)"
         rows.append({"layer": names[mod], "op": f"conv{'T' if p.transposed else ''} k{p.kernel} {p.cin}->{p.cout}",
                      "input": f"{n}x{d}x{h}x{w}", "fwd": fwd, "dgrad": dgrad,
-                     "wgrad": p.route("wgrad"), "halo": halo})
+                     "wgrad": wgrad, "halo": halo})
 
     def gn_hook(mod, args):
         n, c, d, h, w = args[0].shape
