@@ -627,6 +627,7 @@ int conv_plane3_launch(const SbConvArgs* a, cudaStream_t stream);
 int conv_plane3_gn_splits(const SbConvArgs* a);
 int conv_small_launch(const SbConvArgs* a, cudaStream_t stream);
 long long conv_small_workspace(const SbConvArgs* a);
+int conv_point_launch(const SbConvArgs* a, cudaStream_t stream);
 int conv_reduce_slices(const SbConvArgs* a, const float* ws, int splits, cudaStream_t stream);
 }
 
@@ -681,12 +682,14 @@ extern "C" int sb_conv_gn_splits(const SbConvArgs* a) {
   return conv_plane3_gn_splits(a);
 }
 
-// force_plain: 0 = automatic (8 x 8 plane kernel; the two-SM pair kernel for wide outputs given tap-ordered
+// force_plain: 0 = automatic (k = 1 from 16 or 32 channels; 8 x 8 plane kernel; the two-SM pair kernel for wide outputs given tap-ordered
 // weights only; kd-fused or plane-walk kernel when the shape is eligible; else this file's generic kernel),
 // 1 = generic kernel one tap per load, 2 = generic kernel with the w-shift reuse, 3 = generic kernel with the
 // (h, w)-shift reuse, 4 = automatic without the pair kernel.
 extern "C" int sb_conv_fwd(const SbConvArgs* a, cudaStream_t stream) {
   if (automatic(a)) {
+    const int pt = conv_point_launch(a, stream);
+    if (pt >= 0) return pt;
     const int sm = conv_small_launch(a, stream);
     if (sm >= 0) return sm;
     // with a partial-statistics buffer only when the pair kernel is the one that sized it (sb_conv_gn_splits)

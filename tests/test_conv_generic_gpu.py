@@ -79,3 +79,17 @@ def test_small_volumes_split_and_whole_reductions(dims, cins, couts):
     _lib.check_status()
     ref = F.conv3d(torch.cat(xs, 1).double(), wt.double(), padding=1)
     assert torch.equal(torch.cat([_nc(y) for y in ys], 1), _bf(ref))
+
+
+@pytest.mark.parametrize("voxels", [1, 7, 8, 9, 16, 17, 129, 5000, 150001])
+@pytest.mark.parametrize("cin,cout", [(16, 64), (32, 64), (16, 32), (16, 16), (32, 48), (32, 128)])
+def test_few_channels_pointwise(voxels, cin, cout):
+    """Fragments of 16 voxels, a ragged last one; without a bias (the head's backward-data)."""
+    from scaffold_b200.ops import _lib, conv_kernels as ck
+    x, wt = _tri((1, cin, 1, 1, voxels), 11), _tri((cout, cin, 1, 1, 1), 12)
+    out = torch.full((1, 1, 1, voxels + 1, cout), 7.0, dtype=torch.bfloat16, device="cuda")  # one voxel more than is written
+    ck.conv_same([_vm(x)], ck.pack_weight_fwd(wt), 1, [cout], out=[out[:, :, :, :voxels]])
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert torch.equal(_nc(out[:, :, :, :voxels]), _bf(F.conv3d(x.double(), wt.double())))
+    assert bool((out[:, :, :, voxels] == 7).all())
