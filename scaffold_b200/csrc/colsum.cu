@@ -23,7 +23,11 @@ __global__ void __launch_bounds__(CS_THREADS) colsum_partial_kernel(const __nv_b
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.f;
   if (rl < rpb) {
-    const long long stride = (long long)gridDim.x * rpb;
+    // a block owns consecutive rows, four of them (16 bytes each) in flight per thread: 64 channels at 2 x 128^3 98 us
+    // with the final sum, 128 with rows dealt round-robin to the blocks
+    const long long chunk = (M + gridDim.x - 1) / gridDim.x;
+    const long long r0 = blockIdx.x * chunk;
+    const long long r1 = r0 + chunk < M ? r0 + chunk : M;
     auto add = [&](const uint4 raw) {
       const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
@@ -33,14 +37,17 @@ __global__ void __launch_bounds__(CS_THREADS) colsum_partial_kernel(const __nv_b
         acc[2 * i + 1] += f.y;
       }
     };
-    long long r = (long long)blockIdx.x * rpb + rl;
-    for (; r + stride < M; r += 2 * stride) {
-      const uint4 a = __ldg(reinterpret_cast<const uint4*>(x + r * C + oct * 8));
-      const uint4 b = __ldg(reinterpret_cast<const uint4*>(x + (r + stride) * C + oct * 8));
-      add(a);
-      add(b);
+    const __nv_bfloat16* px = x + (r0 + rl) * C + oct * 8;
+    const long long row = (long long)rpb * C;
+    long long r = r0 + rl;
+    for (; r + 3 * rpb < r1; r += 4 * rpb, px += 4 * row) {
+      uint4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = __ldg(reinterpret_cast<const uint4*>(px + u * row));
+#pragma unroll
+      for (int u = 0; u < 4; ++u) add(v[u]);
     }
-    for (; r < M; r += stride) add(__ldg(reinterpret_cast<const uint4*>(x + r * C + oct * 8)));
+    for (; r < r1; r += rpb, px += row) add(__ldg(reinterpret_cast<const uint4*>(px)));
   }
 #pragma unroll
   for (int i = 0; i < 8; ++i) sm[threadIdx.x * 8 + i] = acc[i];

@@ -20,6 +20,7 @@
 namespace sb {
 
 constexpr int PK_T = 32;  // tile of output and input channels
+constexpr int PK_FLIGHT = 5;
 
 __device__ __forceinline__ int kd_pos(int p) {  // (kd,kh,kw) index -> (kh,kw,2-kd) index
   const int kd = p / 9, r = p - kd * 9;
@@ -49,13 +50,14 @@ __device__ __forceinline__ void pack_tile(const SbPackArgs& a, const int bx, con
   const int nco = min(PK_T, a.cout - co0), nci = min(PK_T, a.cin - ci0);
   const int run = nci * 27;
   if (nci == PK_T && (a.cin % 4 == 0) && ((reinterpret_cast<uintptr_t>(a.w) & 15) == 0)) {
-    // full tile: each row is 864 contiguous floats starting on a 16-byte boundary; 16-byte loads, two in flight
+    // full tile: each row is 864 contiguous floats starting on a 16-byte boundary; 16-byte loads, PK_FLIGHT in flight
+    // (three blocks fit on an SM: two in flight were 24 KB of the 45 that the memory wants; 90 M parameters 188 / 150 us)
     constexpr int V = PK_T * 27 / 4;  // float4 per row
-    for (int i = threadIdx.x; i < PK_T * V; i += 2 * blockDim.x) {
-      float4 v[2];
-      int rr[2], jj[2];
+    for (int i = threadIdx.x; i < PK_T * V; i += PK_FLIGHT * blockDim.x) {
+      float4 v[PK_FLIGHT];
+      int rr[PK_FLIGHT], jj[PK_FLIGHT];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
+      for (int u = 0; u < PK_FLIGHT; ++u) {
         const int iu = i + u * blockDim.x;
         rr[u] = iu / V;
         jj[u] = (iu - rr[u] * V) * 4;
@@ -64,7 +66,7 @@ __device__ __forceinline__ void pack_tile(const SbPackArgs& a, const int bx, con
           v[u] = __ldg(reinterpret_cast<const float4*>(a.w + ((long long)(co0 + rr[u]) * a.cin + ci0) * 27 + jj[u]));
       }
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
+      for (int u = 0; u < PK_FLIGHT; ++u) {
         if (i + u * blockDim.x >= PK_T * V) continue;
         const float e[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
 #pragma unroll
@@ -162,12 +164,13 @@ __global__ void __launch_bounds__(256) pack_conv3_kernel(SbPackArgs a) {
 // All layers of a model in one launch: block b belongs to the job with tile0 <= b < tile0 + tiles.
 __global__ void __launch_bounds__(256) pack_conv3_batch_kernel(const SbPackJob* __restrict__ jobs, int njobs) {
   extern __shared__ __nv_bfloat16 tile[];
+  // the last job that starts at or before this block, all starts read at once (one by one they were some 20 dependent
+  // L2 reads in front of every block)
   __shared__ int job_s;
-  if (threadIdx.x == 0) {
-    int j = 0;
-    while (j + 1 < njobs && (int)blockIdx.x >= jobs[j + 1].tile0) ++j;
-    job_s = j;
-  }
+  if (threadIdx.x == 0) job_s = 0;
+  __syncthreads();
+  for (int j = threadIdx.x; j < njobs; j += blockDim.x)
+    if (jobs[j].tile0 <= (int)blockIdx.x) atomicMax(&job_s, j);
   __syncthreads();
   const SbPackJob& jb = jobs[job_s];
   const int t = blockIdx.x - jb.tile0;
