@@ -186,7 +186,9 @@ def check(rc: int, what: str) -> None:
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream's handle (``torch.cuda.current_stream().cuda_stream`` without the stream object: that takes
+    10 us, a fifth of the host time of a launch)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def ptr(t) -> int:
