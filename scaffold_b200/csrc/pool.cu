@@ -165,8 +165,13 @@ __global__ void __launch_bounds__(256) maxpool2_fwd_idx_kernel(const __nv_bfloat
   }
 }
 
+// `add` (optional): the other gradient of x, where x also feeds a skip connection. gx is then their sum in one pass
+// over the volume (fp32, rounded once: the bits of adding the two tensors), instead of writing gx and reading both back:
+// 64 channels at 2 x 128^3 107 + 178 us as two passes (103 + 237 inside a step), 190 as one (1.2 GB).
+template <bool ADD>
 __global__ void __launch_bounds__(256) maxpool2_bwd_idx_kernel(const __nv_bfloat16* __restrict__ gy,
                                                                const unsigned long long* __restrict__ idx,
+                                                               const __nv_bfloat16* __restrict__ add,
                                                                __nv_bfloat16* __restrict__ gx, int N, int D, int H,
                                                                int W, int C) {
   const int OD = D / 2, OH = H / 2, OW = W / 2, C8 = C / 8;
@@ -182,6 +187,14 @@ __global__ void __launch_bounds__(256) maxpool2_bwd_idx_kernel(const __nv_bfloat
     const uint4 rg = __ldg(reinterpret_cast<const uint4*>(gy + i * 8));
     const unsigned long long which = __ldg(idx + i);
     const unsigned short* gs = reinterpret_cast<const unsigned short*>(&rg);
+    uint4 other[8];
+    if constexpr (ADD) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const long long v = (((long long)n * D + (2 * od + (k >> 2))) * H + (2 * oh + ((k >> 1) & 1))) * W + (2 * ow + (k & 1));
+        other[k] = __ldg(reinterpret_cast<const uint4*>(add + v * C + c8 * 8));
+      }
+    }
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int kd = k >> 2, kh = (k >> 1) & 1, kw = k & 1;
@@ -190,14 +203,26 @@ __global__ void __launch_bounds__(256) maxpool2_bwd_idx_kernel(const __nv_bfloat
       unsigned short* os = reinterpret_cast<unsigned short*>(&o);
 #pragma unroll
       for (int j = 0; j < 8; ++j) os[j] = ((which >> (8 * j)) & 0xffull) == (unsigned long long)k ? gs[j] : (unsigned short)0;
+      if constexpr (ADD) {
+        float a[8], b[8];
+        unpack8p(o, a);
+        unpack8p(other[k], b);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[j] += b[j];
+        o.x = pack_bf16x2(a[0], a[1]);
+        o.y = pack_bf16x2(a[2], a[3]);
+        o.z = pack_bf16x2(a[4], a[5]);
+        o.w = pack_bf16x2(a[6], a[7]);
+      }
       *reinterpret_cast<uint4*>(gx + v * C + c8 * 8) = o;
     }
   }
 }
 
-// zero the planes a floor-mode pool never reads (odd extents). One thread per 8 channels of a voxel: as one thread per
+// zero the planes a floor-mode pool never reads (odd extents), or copy `add` there. One thread per 8 channels of a voxel: as one thread per
 // voxel with 2-byte stores, 2 x 11 x 15 x 19 voxels of 256 channels took 67 us.
-__global__ void __launch_bounds__(256) maxpool2_bwd_tail_kernel(__nv_bfloat16* gx, int N, int D, int H, int W, int C) {
+__global__ void __launch_bounds__(256) maxpool2_bwd_tail_kernel(__nv_bfloat16* gx,
+                                                                const __nv_bfloat16* __restrict__ add, int N, int D, int H, int W, int C) {
   const int C8 = C / 8;
   const long long total = (long long)N * D * H * W * C8;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -206,7 +231,8 @@ __global__ void __launch_bounds__(256) maxpool2_bwd_tail_kernel(__nv_bfloat16* g
     const long long row = v / W;
     const int w = (int)(v - row * W), h = (int)(row % H), d = (int)((row / H) % D);
     if (w >= (W / 2) * 2 || h >= (H / 2) * 2 || d >= (D / 2) * 2)
-      *reinterpret_cast<uint4*>(gx + i * 8) = make_uint4(0u, 0u, 0u, 0u);
+      *reinterpret_cast<uint4*>(gx + i * 8) =
+          add ? __ldg(reinterpret_cast<const uint4*>(add + i * 8)) : make_uint4(0u, 0u, 0u, 0u);
   }
 }
 
@@ -236,7 +262,7 @@ extern "C" int sb_maxpool2_bwd(const void* gy, const void* x, const void* y, voi
                                                             (const __nv_bfloat16*)y, (__nv_bfloat16*)gx, N, D, H, W, C);
   sb_count_launch(1);
   if ((D | H | W) & 1) {
-    maxpool2_bwd_tail_kernel<<<pool_grid((long long)N * D * H * W * (C / 8)), 256, 0, stream>>>((__nv_bfloat16*)gx, N, D, H, W, C);
+    maxpool2_bwd_tail_kernel<<<pool_grid((long long)N * D * H * W * (C / 8)), 256, 0, stream>>>((__nv_bfloat16*)gx, nullptr, N, D, H, W, C);
     sb_count_launch(1);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
@@ -253,17 +279,21 @@ extern "C" int sb_maxpool2_fwd_idx(const void* x, void* y, void* idx, int N, int
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }
 
-// Backward from the index words: reads gy and idx only.
-extern "C" int sb_maxpool2_bwd_idx(const void* gy, const void* idx, void* gx, int N, int D, int H, int W, int C,
-                                   cudaStream_t stream) {
+// Backward from the index words: reads gy and idx, and `add` (the gradient that x gets from elsewhere) unless null.
+extern "C" int sb_maxpool2_bwd_idx(const void* gy, const void* idx, const void* add, void* gx, int N, int D, int H,
+                                   int W, int C, cudaStream_t stream) {
   if (C % 8 != 0 || D < 2 || H < 2 || W < 2 || idx == nullptr) return SB_ERR_SHAPE;
   const long long total = (long long)N * (D / 2) * (H / 2) * (W / 2) * (C / 8);
-  maxpool2_bwd_idx_kernel<<<pool_grid(total), 256, 0, stream>>>((const __nv_bfloat16*)gy,
-                                                                (const unsigned long long*)idx, (__nv_bfloat16*)gx, N,
-                                                                D, H, W, C);
+  const __nv_bfloat16* ad = (const __nv_bfloat16*)add;
+  if (ad)
+    maxpool2_bwd_idx_kernel<true><<<pool_grid(total), 256, 0, stream>>>(
+        (const __nv_bfloat16*)gy, (const unsigned long long*)idx, ad, (__nv_bfloat16*)gx, N, D, H, W, C);
+  else
+    maxpool2_bwd_idx_kernel<false><<<pool_grid(total), 256, 0, stream>>>(
+        (const __nv_bfloat16*)gy, (const unsigned long long*)idx, ad, (__nv_bfloat16*)gx, N, D, H, W, C);
   sb_count_launch(1);
   if ((D | H | W) & 1) {
-    maxpool2_bwd_tail_kernel<<<pool_grid((long long)N * D * H * W * (C / 8)), 256, 0, stream>>>((__nv_bfloat16*)gx, N, D, H, W, C);
+    maxpool2_bwd_tail_kernel<<<pool_grid((long long)N * D * H * W * (C / 8)), 256, 0, stream>>>((__nv_bfloat16*)gx, ad, N, D, H, W, C);
     sb_count_launch(1);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;

@@ -26,7 +26,8 @@ import torch.utils.checkpoint
 from ..ops.conv3d import Conv3d, ConvTranspose3d
 from ..ops.group_norm import GroupNorm
 from ..ops.layout import use_cuda_kernels
-from ..ops.pool import MaxPool3d
+from ..ops import pool_kernels
+from ..ops.pool import MaxPool3d, pool_with_skip
 from ..utils.perf import annotate
 
 
@@ -63,6 +64,12 @@ class DoubleConv(nn.Module):
         return self.double_conv(x)
 
 
+def _observed(m: nn.Module) -> bool:
+    """True when someone would notice that ``m`` is not called: a hook, or a forward of its own."""
+    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                or "forward" in m.__dict__)
+
+
 class Down(nn.Module):
     def __init__(self, in_channels: int, out_channels: int, group_norm_groups: int):
         super().__init__()
@@ -71,6 +78,24 @@ class Down(nn.Module):
     @annotate("Down.forward")
     def forward(self, x):
         return self.maxpool_conv(x)
+
+    def forward_with_skip(self, x):
+        """``(self(x), x)``; on the training path of the kernels the pooling's backward pass also adds the gradient that
+        the returned ``x`` collects, as one pass over the volume. A hook, a subclass or a replaced ``forward`` on any of
+        the modules this passes by keeps the ordinary call."""
+        seq = self.maxpool_conv
+        pool = seq[0] if type(seq) is nn.Sequential and len(seq) == 2 else None
+        if not (type(self) is Down and type(pool) is MaxPool3d and pool.kernel_size in (2, (2, 2, 2))
+                and torch.is_grad_enabled() and x.requires_grad and use_cuda_kernels(x) and pool_kernels._USE_INDEX
+                and not any(_observed(m) for m in (self, seq, pool))
+                and not torch.nn.modules.module._has_any_global_hook()):
+            return self(x), x
+        pooled, skip = pool_with_skip(x)
+        return self._after_pool(pooled), skip
+
+    @annotate("Down.forward")
+    def _after_pool(self, pooled):
+        return self.maxpool_conv[1](pooled)
 
 
 class Up(nn.Module):
@@ -164,7 +189,12 @@ class UNet(nn.Module):
             x = x.contiguous()  # the input staging kernel reads a dense NCDHW tensor
         skips = [self._run(self.down_list[0], x)]
         for i in range(1, self.layers + 1):
-            skips.append(self._run(self.down_list[i], skips[-1]))
+            block = self.down_list[i]
+            if self.checkpointing or not isinstance(block, Down):
+                skips.append(self._run(block, skips[-1]))
+            else:
+                out, skips[-1] = block.forward_with_skip(skips[-1])
+                skips.append(out)
         skips.reverse()
         out = skips[0]
         for i in range(len(self.up_list) - 1):

@@ -14,3 +14,10 @@ class MaxPool3d(nn.MaxPool3d):
             from . import pool_kernels as pk
             return from_vm(pk.MaxPool2Fn.apply(to_vm(x)))  # a missing native library raises; no silent ATen path
         return F.max_pool3d(x, self.kernel_size, self.stride, self.padding, self.dilation, self.ceil_mode)
+
+
+def pool_with_skip(x: torch.Tensor):
+    """``(MaxPool3d(2)(x), x)`` for an ``x`` that is used twice (see :class:`pool_kernels.MaxPool2SkipFn`)."""
+    from . import pool_kernels as pk
+    pooled, skip = pk.MaxPool2SkipFn.apply(to_vm(x))
+    return from_vm(pooled), from_vm(skip)

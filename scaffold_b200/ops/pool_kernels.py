@@ -12,7 +12,7 @@ _P = C.c_void_p
 _lib.register("sb_maxpool2_fwd", [_P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P], C.c_int)
 _lib.register("sb_maxpool2_bwd", [_P, _P, _P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P], C.c_int)
 _lib.register("sb_maxpool2_fwd_idx", [_P, _P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P], C.c_int)
-_lib.register("sb_maxpool2_bwd_idx", [_P, _P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P], C.c_int)
+_lib.register("sb_maxpool2_bwd_idx", [_P, _P, _P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P], C.c_int)
 
 
 def available() -> bool:
@@ -45,11 +45,12 @@ def maxpool2_fwd_idx(x: torch.Tensor):
     return y, idx
 
 
-def maxpool2_bwd_idx(gy: torch.Tensor, idx: torch.Tensor, in_shape) -> torch.Tensor:
-    """Backward from the index words: reads ``gy`` and ``idx`` (3/16 of a volume), writes the input gradient."""
+def maxpool2_bwd_idx(gy: torch.Tensor, idx: torch.Tensor, in_shape, add: torch.Tensor = None) -> torch.Tensor:
+    """Backward from the index words: reads ``gy`` and ``idx`` (3/16 of a volume), writes the input gradient, plus
+    ``add`` (another gradient of the input) when given."""
     n, d, h, w, c = in_shape
     gx = torch.empty(tuple(in_shape), dtype=gy.dtype, device=gy.device)
-    _lib.check(_lib.lib().sb_maxpool2_bwd_idx(gy.data_ptr(), idx.data_ptr(), gx.data_ptr(), n, d, h, w, c,
+    _lib.check(_lib.lib().sb_maxpool2_bwd_idx(gy.data_ptr(), idx.data_ptr(), _lib.ptr(add), gx.data_ptr(), n, d, h, w, c,
                                               _lib.stream_ptr()), "sb_maxpool2_bwd_idx")
     return gx
 
@@ -79,3 +80,23 @@ class MaxPool2Fn(torch.autograd.Function):
             return maxpool2_bwd_idx(gy.contiguous(), saved[0], ctx.in_shape)
         x, y = saved
         return maxpool2_bwd(gy.contiguous(), x, y)
+
+
+class MaxPool2SkipFn(torch.autograd.Function):
+    """(pooled x, x) of a tensor that is pooled and also feeds a skip connection: backward adds the two gradients in the
+    pass that spreads the pooled one."""
+
+    @staticmethod
+    def forward(ctx, x):
+        ctx.in_shape = tuple(x.shape)
+        ctx.set_materialize_grads(False)
+        y, idx = maxpool2_fwd_idx(x)
+        ctx.save_for_backward(idx)
+        return y, x
+
+    @staticmethod
+    def backward(ctx, gy, gskip):
+        if gy is None:
+            return gskip
+        (idx,) = ctx.saved_tensors
+        return maxpool2_bwd_idx(gy.contiguous(), idx, ctx.in_shape, None if gskip is None else gskip.contiguous())
