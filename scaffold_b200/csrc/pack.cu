@@ -177,7 +177,71 @@ __global__ void __launch_bounds__(256) pack_conv3_batch_kernel(const SbPackJob* 
   pack_tile(jb.a, t % jb.tiles_x, t / jb.tiles_x, tile);
 }
 
+// Operands of the k2s2 transposed convolution, w [cin][cout][8] fp32 -> fwd [tap * cout + co][cin] and / or dgrad
+// [kd * 2 + kh][cin_pad][kw * cout + co], and of a 1x1x1 convolution (below): one launch per layer where torch took four
+// (permute, cast, zero fill, copy) of 2 us each, 50 us of the 2.9 ms step at scale 6. A block turns a tile of 32 x 32
+// channels x 8 taps over in shared memory; all accesses are runs of at least 64 bytes.
+constexpr int PT_LD = PK_T * 8 + 2;
+__global__ void __launch_bounds__(256) pack_convT_kernel(const float* __restrict__ w, int cin, int cout, int cin_pad,
+                                                         __nv_bfloat16* __restrict__ fwd,
+                                                         __nv_bfloat16* __restrict__ dgrad) {
+  __shared__ __nv_bfloat16 t[PK_T * PT_LD];  // [ci][co * 8 + tap]
+  const int ci0 = blockIdx.x * PK_T, co0 = blockIdx.y * PK_T;
+  const int nci = min(PK_T, cin_pad - ci0), nco = min(PK_T, cout - co0);
+  for (int i = threadIdx.x; i < PK_T * PK_T * 8; i += 256) {
+    const int ci = i / (PK_T * 8), j = i % (PK_T * 8);
+    const bool in = ci0 + ci < cin && j < nco * 8;
+    t[ci * PT_LD + j] = __float2bfloat16(in ? w[((long long)(ci0 + ci) * cout + co0) * 8 + j] : 0.f);
+  }
+  __syncthreads();
+  if (fwd) {
+    for (int i = threadIdx.x; i < PK_T * PK_T * 8; i += 256) {
+      const int ci = i % PK_T, co = (i / PK_T) % PK_T, tap = i / (PK_T * PK_T);
+      if (ci0 + ci < cin && co < nco)
+        fwd[((long long)tap * cout + co0 + co) * cin + ci0 + ci] = t[ci * PT_LD + co * 8 + tap];
+    }
+  }
+  if (dgrad) {
+    for (int i = threadIdx.x; i < PK_T * PK_T * 8; i += 256) {
+      const int co = i % PK_T, ci = (i / PK_T) % PK_T, tap = i / (PK_T * PK_T);
+      if (ci < nci && co < nco)
+        dgrad[((long long)(tap >> 1) * cin_pad + ci0 + ci) * (2 * cout) + (tap & 1) * cout + co0 + co] =
+            t[ci * PT_LD + co * 8 + tap];
+    }
+  }
+}
+
+// w [rows][k] fp32 (or its transpose, when `transposed` w is [k][rows]) -> bf16 [rows_pad][k_pad], zeros behind both
+__global__ void __launch_bounds__(256) pack_point_kernel(const float* __restrict__ w, int rows, int k, int rows_pad,
+                                                         int k_pad, int transposed, __nv_bfloat16* __restrict__ y) {
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= (long long)rows_pad * k_pad) return;
+  const int c = (int)(i % k_pad), r = (int)(i / k_pad);
+  float v = 0.f;
+  if (r < rows && c < k) v = transposed ? w[(long long)c * rows + r] : w[(long long)r * k + c];
+  y[i] = __float2bfloat16(v);
+}
+
 }  // namespace sb
+
+extern "C" int sb_pack_convT(const float* w, int cin, int cout, int cin_pad, void* fwd, void* dgrad,
+                             cudaStream_t stream) {
+  if (cin < 1 || cout < 1 || cin_pad < cin) return SB_ERR_SHAPE;
+  const dim3 grid((cin_pad + sb::PK_T - 1) / sb::PK_T, (cout + sb::PK_T - 1) / sb::PK_T);
+  sb::pack_convT_kernel<<<grid, 256, 0, stream>>>(w, cin, cout, cin_pad, (__nv_bfloat16*)fwd, (__nv_bfloat16*)dgrad);
+  sb_count_launch(1);
+  return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
+}
+
+extern "C" int sb_pack_point(const float* w, int rows, int k, int rows_pad, int k_pad, int transposed, void* y,
+                             cudaStream_t stream) {
+  if (rows < 1 || k < 1 || rows_pad < rows || k_pad < k) return SB_ERR_SHAPE;
+  const long long total = (long long)rows_pad * k_pad;
+  sb::pack_point_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(w, rows, k, rows_pad, k_pad, transposed,
+                                                                            (__nv_bfloat16*)y);
+  sb_count_launch(1);
+  return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
+}
 
 static int pack_configure(int smem) {
   static bool configured = false;

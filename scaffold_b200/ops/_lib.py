@@ -152,6 +152,8 @@ _SIGNATURES = {
     "sb_pack_conv3": ([C.POINTER(SbPackArgs), _P], C.c_int),
     "sb_pack_conv3_plan": ([C.POINTER(SbPackJob), C.c_int], C.c_longlong),
     "sb_pack_conv3_batch": ([_P, C.c_int, C.c_longlong, _P], C.c_int),
+    "sb_pack_convT": ([_P, C.c_int, C.c_int, C.c_int, _P, _P, _P], C.c_int),
+    "sb_pack_point": ([_P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P, _P], C.c_int),
     "sb_stage_stem": ([_P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P, _P], C.c_int),
     "sb_pack_stem": ([_P, C.c_int, C.c_int, C.c_int, _P, _P], C.c_int),
     "sb_stage_input": ([_P, C.c_int, C.c_int, C.c_int, C.c_longlong, _P, C.c_int, _P], C.c_int),

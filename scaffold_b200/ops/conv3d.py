@@ -194,6 +194,13 @@ def _pad_in_channels(w: torch.Tensor, src_channels: Sequence[int], real: Sequenc
     return torch.cat(parts, 1)
 
 
+def _pack_point(w: torch.Tensor, src_c: Sequence[int], real_c: Sequence[int], dgrad: bool) -> torch.Tensor:
+    """bf16 operand of a 1x1x1 weight; a padded source inside a concatenation takes the general packing."""
+    if len(src_c) == 1 or list(src_c) == list(real_c):
+        return ck.pack_point(w, sum(src_c), dgrad)
+    return (ck.pack_weight_dgrad if dgrad else ck.pack_weight_fwd)(_pad_in_channels(w, src_c, real_c))
+
+
 def _bias_grad(gy: torch.Tensor, n_out: int, bias) -> Optional[torch.Tensor]:
     """Bias gradient for autograd, or None when it went straight into the flat gradient buffer."""
     direct = direct_grad_target(bias)
@@ -226,8 +233,7 @@ class _ConvSameFn(torch.autograd.Function):
             kd = ck.kd_eligible(ck.pad_channels(weight.shape[0]), sum(src_c), out_dims, src_c[0])
             wf = mod._cache.conv3(weight, src_c, real_c, "fwd", kd, ts)
         else:
-            wf = mod._cache.get(weight, f"fwd{src_c}",
-                                lambda w: ck.pack_weight_fwd(_pad_in_channels(w, src_c, real_c)))
+            wf = mod._cache.get(weight, f"fwd{src_c}", lambda w: _pack_point(w, src_c, real_c, False))
         cout_pad = wf.shape[1]
         bpad = None
         if bias is not None:
@@ -261,8 +267,7 @@ class _ConvSameFn(torch.autograd.Function):
                 kd = ck.kd_eligible(sum(src_c), gy.shape[4], ctx.in_dims)
                 wd = mod._cache.conv3(weight, src_c, real_c, "dgrad", kd, ctx.tap_swap)
             else:
-                wd = mod._cache.get(weight, f"dgrad{src_c}",
-                                    lambda w: ck.pack_weight_dgrad(_pad_in_channels(w, src_c, real_c)))
+                wd = mod._cache.get(weight, f"dgrad{src_c}", lambda w: _pack_point(w, src_c, real_c, True))
             # a halo'd input gets a halo'd gradient: output grid = input extents, gy read at -offset
             outs = ck.conv_same([gy], wd, ks, src_c, out_dims=ctx.in_dims, in_off=[-o for o in ctx.in_off])
             for i, o in enumerate(outs):
@@ -487,7 +492,9 @@ class _ConvTFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, weight, bias, mod, x):
         cout = weight.shape[1]
-        wf = mod._cache.get(weight, "fwd", ck.pack_weight_convT_fwd)
+        # with a backward pass to come, both operands from one reading of the weight
+        both = mod._cache.get(weight, "both", lambda w: ck.pack_convT(w, True, True)) if ctx.needs_input_grad[3] else None
+        wf = both[0] if both else mod._cache.get(weight, "fwd", lambda w: ck.pack_convT(w, True, False)[0])
         b32 = None
         if bias is not None:
             b32 = mod._cache_b.get(bias, "b", lambda b: b.contiguous())
@@ -505,7 +512,7 @@ class _ConvTFn(torch.autograd.Function):
         gy = gy.contiguous()
         gx = gw = gb = None
         if ctx.needs_input_grad[3]:
-            wd = mod._cache.get(weight, "dgrad", ck.pack_weight_convT_dgrad)
+            wd = mod._cache.get(weight, "both", lambda w: ck.pack_convT(w, True, True))[1]
             gx = ck.convT_dgrad(gy, wd, x.shape[4])
         if ctx.needs_input_grad[0]:
             direct = direct_grad_target(ctx.wparam)

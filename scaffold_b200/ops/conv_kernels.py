@@ -183,6 +183,31 @@ def pack_weight_convT_dgrad(w: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def pack_convT(w: torch.Tensor, want_fwd: bool, want_dgrad: bool):
+    """``(pack_weight_convT_fwd(w), pack_weight_convT_dgrad(w))`` of a CUDA fp32 weight in one kernel; None where not
+    wanted."""
+    w = w.contiguous()
+    ci, co = w.shape[:2]
+    bf16 = {"dtype": torch.bfloat16, "device": w.device}
+    fwd = torch.empty((8 * co, ci), **bf16) if want_fwd else None
+    dgrad = torch.empty((4, pad_channels(ci), 2 * co), **bf16) if want_dgrad else None
+    _lib.check(_lib.lib().sb_pack_convT(w.data_ptr(), ci, co, pad_channels(ci), _lib.ptr(fwd), _lib.ptr(dgrad),
+                                        _lib.stream_ptr()), "sb_pack_convT")
+    return fwd, dgrad
+
+
+def pack_point(w: torch.Tensor, k_pad: int, dgrad: bool) -> torch.Tensor:
+    """Operand of a 1x1x1 CUDA fp32 weight over one source of ``k_pad`` (padded) channels, in one kernel: forward
+    ``[1, cout_pad, k_pad]``, backward-data ``[1, k_pad, cout_pad]``."""
+    w = w.contiguous()
+    co, ci = w.shape[:2]
+    rows, k, rows_pad, kp = (ci, co, k_pad, pad_channels(co)) if dgrad else (co, ci, pad_channels(co), k_pad)
+    out = torch.empty((1, rows_pad, kp), dtype=torch.bfloat16, device=w.device)
+    _lib.check(_lib.lib().sb_pack_point(w.data_ptr(), rows, k, rows_pad, kp, int(dgrad), out.data_ptr(),
+                                        _lib.stream_ptr()), "sb_pack_point")
+    return out
+
+
 # ---------------------------------------------------------------------------
 # launchers
 # ---------------------------------------------------------------------------

@@ -93,3 +93,16 @@ def test_few_channels_pointwise(voxels, cin, cout):
     _lib.check_status()
     assert torch.equal(_nc(out[:, :, :, :voxels]), _bf(F.conv3d(x.double(), wt.double())))
     assert bool((out[:, :, :, voxels] == 7).all())
+
+
+@pytest.mark.parametrize("cin,cout", [(16, 8), (32, 16), (48, 40), (64, 32), (96, 72), (128, 64)])
+def test_packed_operands_equal_the_general_packing(cin, cout):
+    from scaffold_b200.ops import conv_kernels as ck
+    wt = torch.randn((cin, cout, 2, 2, 2), device="cuda")
+    want = (ck.pack_weight_convT_fwd(wt), ck.pack_weight_convT_dgrad(wt))
+    for both in ((True, True), (True, False), (False, True)):
+        for got, ref, asked in zip(ck.pack_convT(wt, *both), want, both):
+            assert torch.equal(got, ref) if asked else got is None
+    w1 = torch.randn((cout, cin, 1, 1, 1), device="cuda")
+    assert torch.equal(ck.pack_point(w1, ck.pad_channels(cin), False), ck.pack_weight_fwd(w1))
+    assert torch.equal(ck.pack_point(w1, ck.pad_channels(cin), True), ck.pack_weight_dgrad(w1))
