@@ -324,32 +324,14 @@ __global__ void __launch_bounds__(GN_THREADS, GN_WAVE) gn_apply_kernel(const GnP
   __shared__ float s_mean[256], s_rstd[256];
   const int n = blockIdx.y;
   if (!gn_wait_peers(p, 61)) return;
-  auto keep = [&](int g, float m, float r) {
+  for (int g = threadIdx.x; g < p.G; g += GN_THREADS) {
+    float m, r;
+    merge_group(p, n, g, m, r);
     s_mean[g] = m;
     s_rstd[g] = r;
     if (blockIdx.x == 0) {
       p.mean[n * p.G + g] = m;
       p.rstd[n * p.G + g] = r;
-    }
-  };
-  if (p.n_parts == 1 && p.nsplit > 1) {
-    // few partials: every block collapses them itself, a warp per group, to the bits of the finalize kernel. A small
-    // tensor's layer is launch after launch, and that launch (4.7 us of a 7 us pass) costs more than these reads.
-    const int lane = threadIdx.x & 31;
-    for (int g = threadIdx.x >> 5; g < p.G; g += GN_THREADS / 32) {
-      const StatSums a = stat_warp_sum(stat_walk(p.parts[0] + ((long long)n * p.nsplit * p.G + g) * 3, p.G, lane, 32,
-                                                 p.nsplit));
-      if (lane == 0) {
-        float e[3];
-        stat_store(e, a);
-        keep(g, e[1], rsqrtf(e[2] / e[0] + p.eps));
-      }
-    }
-  } else {
-    for (int g = threadIdx.x; g < p.G; g += GN_THREADS) {
-      float m, r;
-      merge_group(p, n, g, m, r);
-      keep(g, m, r);
     }
   }
   __syncthreads();

@@ -133,17 +133,12 @@ def _set_wait(a: SbGnArgs, wait, device) -> None:
         a.status = _lib.status_tensor(device).data_ptr()
 
 
-# Partials (of all groups) of a sample that gn_apply collapses by itself: every block reads them, 24 KB at most
-DIRECT_PARTIALS = 2048
-
-
-def gn_apply(x, w, b, groups, eps, relu, parts: Sequence[int], shards: int = 1, wait=None, nsplit: int = 1):
-    """Pass 2: merge ``parts`` (device pointers, own first) and normalise. ``nsplit`` > 1: the single part holds that
-    many uncollapsed partials per sample.
+def gn_apply(x, w, b, groups, eps, relu, parts: Sequence[int], shards: int = 1, wait=None):
+    """Pass 2: merge ``parts`` (device pointers, own first) and normalise.
 
     ``wait`` = (pointer to ``len(parts)`` flag words, epoch): the kernel first waits until every
     flag reached the epoch (peers push their statistics and then raise the flag)."""
-    a = _base(x, w, b, groups, eps, relu, shards, nsplit=nsplit)
+    a = _base(x, w, b, groups, eps, relu, shards, nsplit=1)
     _set_wait(a, wait, x.device)
     n = x.shape[0]
     y = torch.empty_like(x)

@@ -25,18 +25,13 @@ class _GnFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, groups, eps, relu, spatial, partials):
         w32, b32 = weight.detach().float().contiguous(), bias.detach().float().contiguous()
-        fin = direct = None
+        fin = None
         if partials is not None:
             # the producing convolution left (count, mean, M2) partials of this very tensor: no statistics pass
             part, splits, pg = partials
             if pg == groups and part.numel() == x.shape[0] * splits * groups * 3:
-                if spatial is None and 1 < splits and splits * groups <= gk.DIRECT_PARTIALS:
-                    direct = part
-                else:
-                    fin = gk.gn_finalize(part, x.shape[0], groups, splits)
-        if direct is not None:
-            y, mean, rstd = gk.gn_apply(x, w32, b32, groups, eps, relu, [direct.data_ptr()], nsplit=splits)
-        elif spatial is None:
+                fin = gk.gn_finalize(part, x.shape[0], groups, splits)
+        if spatial is None:
             y, mean, rstd = gk.gn_forward(x, w32, b32, groups, eps, relu, fin=fin)
         else:
             y, mean, rstd = spatial.gn_forward(x, w32, b32, groups, eps, relu, fin=fin)

@@ -149,22 +149,3 @@ def test_finalize_pools_partials_like_fp64(nsplit):
     ref = torch.stack([tot, mean, (m2 + n * (m - mean[:, None]) ** 2).sum(1)], -1)
     # sums in double, results rounded once to fp32: 2^-24, doubled for the subtraction in M2
     torch.testing.assert_close(got, ref, rtol=2 ** -22, atol=1e-3)
-
-
-@pytest.mark.parametrize("n,c,groups,nsplit", [(1, 64, 8, 2), (2, 32, 8, 33), (3, 128, 8, 256), (1, 16, 8, 7),
-                                               (2, 48, 3, 100), (1, 256, 32, 64)])
-def test_apply_collapses_few_partials_like_the_finalize_kernel(n, c, groups, nsplit):
-    import torch
-
-    from scaffold_b200.ops import gn_kernels as gk
-    g = torch.Generator(device="cuda").manual_seed(nsplit)
-    x = torch.randn((n, 3, 5, 7, c), generator=g, device="cuda").to(torch.bfloat16)
-    w, b = torch.rand(c, generator=g, device="cuda") + 0.5, torch.randn(c, generator=g, device="cuda")
-    part = torch.rand((n, nsplit, groups, 3), generator=g, device="cuda")
-    part[..., 0] = torch.randint(0, 3, (n, nsplit, 1), generator=g, device="cuda") * 64.0
-    part[:, 0, :, 0] = 64.0
-    fin = gk.gn_finalize(part.reshape(-1), n, groups, nsplit)
-    want = gk.gn_apply(x, w, b, groups, 1e-5, True, [fin.data_ptr()])
-    got = gk.gn_apply(x, w, b, groups, 1e-5, True, [part.data_ptr()], nsplit=nsplit)
-    for a, e in zip(got, want):
-        assert torch.equal(a, e)
