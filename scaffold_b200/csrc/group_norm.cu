@@ -468,12 +468,32 @@ __global__ void __launch_bounds__(GN_THREADS, GN_WAVE) gn_bwd_dx_kernel(const Gn
   float* s_B = sm + p.C;        // [C] this rank's sum(dy' xhat)
   float* s_c1 = sm + 2 * p.C;   // [G]
   float* s_c2 = s_c1 + p.G;     // [G]
-  float* s_At = s_c2 + p.G;     // [C] all shards
+  float* s_At = s_c2 + p.G;     // [C] all shards, times the weight
   float* s_Bt = s_At + p.C;
   const int n = blockIdx.y;
   const int cg = p.C / p.G;
   if (!gn_wait_peers(p, 62)) return;
+  // What a thread needs of its own channels is read ahead of the collapse below: on a small tensor this prologue is most
+  // of the launch, and its phases are one L2 latency each.
+  const int tpv = p.C / 8;
+  const int vpb = GN_THREADS / tpv;
+  const int oct = threadIdx.x % tpv;
+  const int vl = threadIdx.x / tpv;
+  float a[8], c[8], mu[GP], rs[GP];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int ch = oct * 8 + i;
+    const int g = ch / cg;
+    const float m = p.mean[n * p.G + g], r = p.rstd[n * p.G + g];
+    a[i] = r * p.w[ch];
+    c[i] = p.b[ch] - m * a[i];
+    if (i % (8 / GP) == 0) {
+      mu[i / (8 / GP)] = m;
+      rs[i / (8 / GP)] = r;
+    }
+  }
   for (int ch = threadIdx.x; ch < p.C; ch += GN_THREADS) {
+    const float wc = p.w[ch];
     float At = 0.f, Bt = 0.f, A0 = 0.f, B0 = 0.f;
     for (int pi = 0; pi < p.n_parts; ++pi) {
       const float* base = p.parts[pi] + ((long long)n * p.nsplit * p.C + ch) * 2;
@@ -486,15 +506,15 @@ __global__ void __launch_bounds__(GN_THREADS, GN_WAVE) gn_bwd_dx_kernel(const Gn
       At += a;
       Bt += b;
     }
-    s_A[ch] = A0; s_B[ch] = B0; s_At[ch] = At; s_Bt[ch] = Bt;
+    s_A[ch] = A0; s_B[ch] = B0; s_At[ch] = wc * At; s_Bt[ch] = wc * Bt;
   }
   __syncthreads();
   for (int g = threadIdx.x; g < p.G; g += GN_THREADS) {
     float c1 = 0.f, c2 = 0.f;
     for (int j = 0; j < cg; ++j) {
       const int ch = g * cg + j;
-      c1 += p.w[ch] * s_At[ch];
-      c2 += p.w[ch] * s_Bt[ch];
+      c1 += s_At[ch];
+      c2 += s_Bt[ch];
     }
     s_c1[g] = c1 / p.group_elems;
     s_c2[g] = c2 / p.group_elems;
@@ -503,8 +523,8 @@ __global__ void __launch_bounds__(GN_THREADS, GN_WAVE) gn_bwd_dx_kernel(const Gn
   // dweight / dbias: this rank's share, summed over samples in index order
   if (blockIdx.x == 0 && blockIdx.y == 0 && p.dw != nullptr) {
     for (int ch = threadIdx.x; ch < p.C; ch += GN_THREADS) {
-      float a = 0.f, b = 0.f;
-      for (int nn = 0; nn < p.N; ++nn) {
+      float a = s_A[ch], b = s_B[ch];  // sample 0 is this block's
+      for (int nn = 1; nn < p.N; ++nn) {
         const float* base = p.parts[0] + ((long long)nn * p.nsplit * p.C + ch) * 2;
         for (int s = 0; s < p.nsplit; ++s) {
           a += base[(long long)s * p.C * 2];
@@ -515,25 +535,14 @@ __global__ void __launch_bounds__(GN_THREADS, GN_WAVE) gn_bwd_dx_kernel(const Gn
       p.dw[ch] = p.accumulate ? p.dw[ch] + b : b;
     }
   }
-  const int tpv = p.C / 8;
-  const int vpb = GN_THREADS / tpv;
-  const int oct = threadIdx.x % tpv;
-  const int vl = threadIdx.x / tpv;
   if (vl >= vpb) return;
   // dx = rstd (d w - c1 - xhat c2) = d a + (x - mean) q + r
-  float a[8], c[8], mu[GP], q[GP], r[GP];
+  float q[GP], r[GP];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int ch = oct * 8 + i;
-    const int g = ch / cg;
-    const float m = p.mean[n * p.G + g], rs = p.rstd[n * p.G + g];
-    a[i] = rs * p.w[ch];
-    c[i] = p.b[ch] - m * a[i];
-    if (i % (8 / GP) == 0) {
-      mu[i / (8 / GP)] = m;
-      q[i / (8 / GP)] = -rs * rs * s_c2[g];
-      r[i / (8 / GP)] = -rs * s_c1[g];
-    }
+  for (int i = 0; i < GP; ++i) {
+    const int g = (oct * 8 + i * (8 / GP)) / cg;
+    q[i] = -rs[i] * rs[i] * s_c2[g];
+    r[i] = -rs[i] * s_c1[g];
   }
   const long long base = (long long)n * p.S * p.C + oct * 8;
   auto body = [&](const uint4 rx, const uint4 rd, long long at) {

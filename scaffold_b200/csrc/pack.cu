@@ -188,6 +188,7 @@ __global__ void __launch_bounds__(256) pack_convT_kernel(const float* __restrict
   __shared__ __nv_bfloat16 t[PK_T * PT_LD];  // [ci][co * 8 + tap]
   const int ci0 = blockIdx.x * PK_T, co0 = blockIdx.y * PK_T;
   const int nci = min(PK_T, cin_pad - ci0), nco = min(PK_T, cout - co0);
+#pragma unroll 8
   for (int i = threadIdx.x; i < PK_T * PK_T * 8; i += 256) {
     const int ci = i / (PK_T * 8), j = i % (PK_T * 8);
     const bool in = ci0 + ci < cin && j < nco * 8;
@@ -195,14 +196,16 @@ __global__ void __launch_bounds__(256) pack_convT_kernel(const float* __restrict
   }
   __syncthreads();
   if (fwd) {
-    for (int i = threadIdx.x; i < PK_T * PK_T * 8; i += 256) {
+#pragma unroll 8
+  for (int i = threadIdx.x; i < PK_T * PK_T * 8; i += 256) {
       const int ci = i % PK_T, co = (i / PK_T) % PK_T, tap = i / (PK_T * PK_T);
       if (ci0 + ci < cin && co < nco)
         fwd[((long long)tap * cout + co0 + co) * cin + ci0 + ci] = t[ci * PT_LD + co * 8 + tap];
     }
   }
   if (dgrad) {
-    for (int i = threadIdx.x; i < PK_T * PK_T * 8; i += 256) {
+#pragma unroll 8
+  for (int i = threadIdx.x; i < PK_T * PK_T * 8; i += 256) {
       const int co = i % PK_T, ci = (i / PK_T) % PK_T, tap = i / (PK_T * PK_T);
       if (ci < nci && co < nco)
         dgrad[((long long)(tap >> 1) * cin_pad + ci0 + ci) * (2 * cout) + (tap & 1) * cout + co0 + co] =
