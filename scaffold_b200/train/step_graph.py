@@ -33,6 +33,15 @@ MAX_SHAPES = 4         # graphs per engine and kind of pass
 MAX_MAP_BYTES = 640 << 20
 
 
+def _watched() -> bool:
+    """True while something follows single operations or tensors (dispatch and function modes, saved-tensor hooks,
+    forward-mode AD, functorch transforms, tracing): it would see nothing of a replayed pass."""
+    return bool(torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
+                or torch._C._autograd._top_saved_tensors_default_hooks(True) is not None
+                or torch.autograd.forward_ad._current_level >= 0
+                or torch._C._functorch.maybe_current_level() is not None or torch._C._get_tracing_state() is not None)
+
+
 class _Fingerprint:
     """What a captured pass depends on besides the batch's values; ``holds()`` is a few hundred identity checks."""
 
@@ -154,7 +163,7 @@ class StepGraphs:
         widest = images.shape[0] * math.prod(images.shape[2:]) * model.base_width * 2
         return (widest <= MAX_MAP_BYTES and not model.checkpointing and not layout._aten_only[0]
                 and not torch.is_anomaly_enabled() and not perf._nvtx_enabled()
-                and not torch.nn.modules.module._has_any_global_hook() and torch._C._len_torch_dispatch_stack() == 0
+                and not torch.nn.modules.module._has_any_global_hook() and not _watched()
                 and not torch.cuda.is_current_stream_capturing())
 
     def get(self, engine, images, masks, train: bool) -> Optional[_Pass]:

@@ -102,3 +102,28 @@ def test_class_weights_are_read_at_replay_and_evaluation_follows_new_weights():
         for s, t in zip(a.eval_step(*batch), b.eval_step(*batch)):
             assert torch.equal(s, t), i
     assert _captured(a)
+
+
+@pytest.mark.parametrize("what", ["saved_tensors", "function_mode", "dual_level"])
+def test_an_observer_of_operations_sees_the_ordinary_pass(what):
+    from contextlib import nullcontext
+
+    from torch.overrides import TorchFunctionMode
+    class Mode(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    eng = _engine(True)
+    batch = _batch(0)
+    for _ in range(4):
+        eng.step(*batch)
+    assert _captured(eng)
+    packed = []
+    ctx = {"saved_tensors": lambda: torch.autograd.graph.saved_tensors_hooks(lambda t: (packed.append(1), t)[1], lambda t: t),
+           "function_mode": Mode, "dual_level": torch.autograd.forward_ad.dual_level}[what]
+    for manager, usable in ((ctx, False), (nullcontext, True)):
+        with manager():
+            assert (eng._graphs.get(eng, *batch, train=True) is not None) is usable
+    with ctx():
+        eng.step(*batch)
+    assert bool(packed) is (what == "saved_tensors")
