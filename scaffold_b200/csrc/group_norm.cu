@@ -112,20 +112,16 @@ __device__ __forceinline__ void stat_store(float* dst, const StatSums& a) {
 // L1 (the partials may have been written by other SMs during this launch).
 __device__ __forceinline__ StatSums stat_walk(const float* __restrict__ base, int G, int first, int step, int nsplit) {
   StatSums a{0.0, 0.0, 0.0};
-  int s = first;
-  for (; s + 7 * step < nsplit; s += 8 * step) {
+  for (int s = first; s < nsplit; s += 8 * step) {
     float e[8][3];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const float* q = base + (long long)(s + u * step) * G * 3;
-      e[u][0] = __ldcg(q); e[u][1] = __ldcg(q + 1); e[u][2] = __ldcg(q + 2);
+      if (s + u * step < nsplit) { e[u][0] = __ldcg(q); e[u][1] = __ldcg(q + 1); e[u][2] = __ldcg(q + 2); }
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) stat_add(a, e[u][0], e[u][1], e[u][2]);
-  }
-  for (; s < nsplit; s += step) {
-    const float* q = base + (long long)s * G * 3;
-    stat_add(a, __ldcg(q), __ldcg(q + 1), __ldcg(q + 2));
+    for (int u = 0; u < 8; ++u)
+      if (s + u * step < nsplit) stat_add(a, e[u][0], e[u][1], e[u][2]);
   }
   return a;
 }
@@ -151,11 +147,15 @@ __device__ __forceinline__ void stats_collapse_warp(const float* __restrict__ pa
 __device__ __forceinline__ void bwd_collapse_warp(const float* __restrict__ part, float* __restrict__ fin, int C,
                                                   int nsplit, int n, int c, int lane) {
   float a = 0.f, b = 0.f;
-#pragma unroll 8
-  for (int s = lane; s < nsplit; s += 32) {
-    const float2 e = __ldcg(reinterpret_cast<const float2*>(part + (((long long)n * nsplit + s) * C + c) * 2));
-    a += e.x;
-    b += e.y;
+  for (int s = lane; s < nsplit; s += 8 * 32) {
+    float2 e[8];  // eight in flight, the last ones too
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (s + u * 32 < nsplit)
+        e[u] = __ldcg(reinterpret_cast<const float2*>(part + (((long long)n * nsplit + s + u * 32) * C + c) * 2));
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (s + u * 32 < nsplit) { a += e[u].x; b += e[u].y; }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -588,6 +588,26 @@ __global__ void __launch_bounds__(GN_THREADS) gn_stats_finalize_kernel(const flo
   stats_collapse_warp(part, fin, G, nsplit, warp / G, warp % G, lane);
 }
 
+// The same collapse with a block per (n, g) beyond 32 partials: a lane's 16 partials were two trips to L2 and 16 dependent
+// double additions, a thread's 4 are one trip (512 partials 4.9 us a
+// launch, now 2.7).
+constexpr int GN_FIN_THREADS = 128;
+__global__ void __launch_bounds__(GN_FIN_THREADS) gn_stats_finalize_block_kernel(const float* __restrict__ part,
+                                                                                 float* __restrict__ fin, int G,
+                                                                                 int nsplit) {
+  __shared__ double s_w[GN_FIN_THREADS / 32][3];
+  const int n = blockIdx.x / G, g = blockIdx.x % G, warp = threadIdx.x >> 5;
+  const StatSums a = stat_warp_sum(stat_walk(part + ((long long)n * nsplit * G + g) * 3, G, threadIdx.x, GN_FIN_THREADS,
+                                             nsplit));
+  if ((threadIdx.x & 31) == 0) { s_w[warp][0] = a.n; s_w[warp][1] = a.s1; s_w[warp][2] = a.s2; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    StatSums t{0.0, 0.0, 0.0};
+    for (int w = 0; w < GN_FIN_THREADS / 32; ++w) { t.n += s_w[w][0]; t.s1 += s_w[w][1]; t.s2 += s_w[w][2]; }
+    stat_store(fin + ((long long)n * G + g) * 3, t);
+  }
+}
+
 // The same collapse for MANY partials per (n, g) (the per-warp partials a convolution's epilogue leaves: up to
 // 16K per sample). Bound: L2 latency and the sectors around 12-byte entries, so a cluster of eight CTAs shares one
 // (n, g): thread t of CTA r adds the partials r * 256 + t, + 2048, ..., each CTA adds its warps in order, and CTA 0
@@ -814,7 +834,10 @@ extern "C" int sb_gn_stats_finalize(const float* part, float* fin, int N, int G,
     sb_count_launch(1);
     return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
   }
-  gn_stats_finalize_kernel<<<(warps * 32 + GN_THREADS - 1) / GN_THREADS, GN_THREADS, 0, stream>>>(part, fin, N, G, nsplit);
+  if (nsplit > 32)
+    gn_stats_finalize_block_kernel<<<warps, GN_FIN_THREADS, 0, stream>>>(part, fin, G, nsplit);
+  else
+    gn_stats_finalize_kernel<<<(warps * 32 + GN_THREADS - 1) / GN_THREADS, GN_THREADS, 0, stream>>>(part, fin, N, G, nsplit);
   sb_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }
