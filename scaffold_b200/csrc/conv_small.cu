@@ -152,7 +152,10 @@ __global__ void __launch_bounds__(192, 1) conv_small_kernel(const __grid_constan
   }
 }
 
-// out[v][c] = bf16(bias[c] + sum_s ws[s][v][c]), channels routed to up to two destinations
+// out[v][c] = bf16(bias[c] + sum_s ws[s][v][c]), channels routed to up to two destinations. The slices are added in order,
+// SR_FLIGHT of them in flight: one after the other they were an L2 latency each (512 channels at 8^3: 8.2 us a
+// launch, now 5.7).
+constexpr int SR_FLIGHT = 6;
 struct SmallReduceParams {
   const float* ws;
   long long rows;  // N * D * 64 voxels
@@ -172,11 +175,21 @@ __global__ void __launch_bounds__(256) conv_small_reduce_kernel(const SmallReduc
     float f[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) f[e] = 0.f;
-    for (int s = 0; s < p.splits; ++s) {
-      const float4* src = reinterpret_cast<const float4*>(p.ws + ((long long)s * p.rows + v) * p.cout_pad + col);
-      const float4 a = src[0], b = src[1];
-      f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
-      f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
+    for (int s0 = 0; s0 < p.splits; s0 += SR_FLIGHT) {
+      float4 a[SR_FLIGHT], b[SR_FLIGHT];
+#pragma unroll
+      for (int u = 0; u < SR_FLIGHT; ++u)
+        if (s0 + u < p.splits) {
+          const float4* src = reinterpret_cast<const float4*>(p.ws + ((long long)(s0 + u) * p.rows + v) * p.cout_pad + col);
+          a[u] = __ldcs(src);
+          b[u] = __ldcs(src + 1);
+        }
+#pragma unroll
+      for (int u = 0; u < SR_FLIGHT; ++u)
+        if (s0 + u < p.splits) {
+          f[0] += a[u].x; f[1] += a[u].y; f[2] += a[u].z; f[3] += a[u].w;
+          f[4] += b[u].x; f[5] += b[u].y; f[6] += b[u].z; f[7] += b[u].w;
+        }
     }
     __nv_bfloat16* dst = nullptr;
     if (col < p.width0) {
