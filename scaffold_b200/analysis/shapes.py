@@ -145,6 +145,8 @@ class ConvProblem:
         if self.transposed:
             return {"fwd": "igemm(scatter)", "dgrad": "igemm(strided)", "wgrad": "wgrad(generic)"}[direction]
         if self.kernel == 1:
+            if direction == "dgrad" and k.cout in (16, 32) and k.cin <= 128 and not k.split_cin:
+                return "conv_point"  # (the forward pass has the head's bias)
             return "wgrad(generic)" if direction == "wgrad" else "igemm"
         big = w >= 16 and h >= 8
         rows_, kk_ = (k.cout, k.cin) if direction == "fwd" else (k.cin, k.cout)
