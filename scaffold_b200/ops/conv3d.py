@@ -35,7 +35,7 @@ from .layout import (EPOCH_CELL_ATTR, direct_grad_target, from_vm, notify_grad_w
 _GN_FROM_EPILOGUE = os.environ.get("SCAFFOLD_GN_FROM_EPILOGUE", "1") != "0"
 
 _PACK_REGISTRY: "weakref.WeakSet[_PackCache]" = weakref.WeakSet()
-_PACK_GENERATION = [0]  # counts the layouts that layers have asked for: a packing table built before is out of date
+_PACK_GENERATION = [0]  # counts new layouts and new owners of layouts: a packing table built before is out of date
 
 
 def _pack_members(cell) -> list:
@@ -110,6 +110,14 @@ def refresh_packs(flat) -> None:
             return
 
 
+def packed_weight(flat, cache):
+    """The parameter whose operand copies in ``cache`` :func:`repack_all` renews for ``flat``, or None."""
+    for c, w, *_ in flat.pack_plan.get("members", ()):
+        if c() is cache:
+            return w()
+    return None
+
+
 def pack_buffers(flat) -> list:
     """The operand buffers of :func:`repack_all`'s table (persistent: a captured pass reads them at their addresses)."""
     return [b for *_, bufs in flat.pack_plan.get("members", ()) for b in bufs.values()]
@@ -120,7 +128,7 @@ class _PackCache:
 
     def __init__(self):
         self._key = None
-        self._w_ref = None    # the parameter these copies belong to (set on first use)
+        self._w_ref = None    # the parameter these copies were made of
         self._real = {}       # source signature -> real channels per source
         self._tap_swap = 0    # tap-axis exchange the packs were made with (sharded runs, see Conv3d._tap_swap)
         self._vals = {}
@@ -132,6 +140,12 @@ class _PackCache:
         # strides / tap exchange: the same parameter may be read tap-transposed (sharded runs) or directly
         if tap_swap is not None:
             self._tap_swap = int(tap_swap)
+        if isinstance(w, torch.nn.Parameter) and (self._w_ref is None or self._w_ref() is not w):
+            # another parameter than the copies were made of (a copied module, load_state_dict(assign=True)), whatever
+            # its address and version
+            self._w_ref = weakref.ref(w)
+            self._key = None
+            _PACK_GENERATION[0] += 1
         key = (w.data_ptr(), w._version, w.device, weights_epoch(w), tuple(w.stride()), self._tap_swap)
         if key != self._key:
             self._key = key
@@ -145,6 +159,9 @@ class _PackCache:
         kernel launch, so a step packs each weight once.
         """
         self._sync(w, tap_swap)
+        if self._w_ref is not None and self not in _PACK_REGISTRY:  # first use, or the first one of a copied module
+            _PACK_REGISTRY.add(self)
+            _PACK_GENERATION[0] += 1
         sig = tuple(src_c)
         name = kind + ("_kd" if kd else "")
         if (name, sig) not in self._fresh:
@@ -152,9 +169,6 @@ class _PackCache:
                 self._asked.add((name, sig))
                 _PACK_GENERATION[0] += 1
             self._real[sig] = list(real_c)
-            if self._w_ref is None and isinstance(w, torch.nn.Parameter):
-                self._w_ref = weakref.ref(w)
-                _PACK_REGISTRY.add(self)
             group = [k for k in self._asked if k[1] == sig]
             want = {}
             co_pad, k_pad = ck.pad_channels(w.shape[0]), sum(sig)

@@ -105,6 +105,14 @@ class _Pass:
             c._vals = {}
         engine.flat.rebind_grads()
         c3.repack_all(engine.flat)
+        # ... so every layout that a layer uses has to be one that the optimizer step (and refresh_packs) renews
+        layouts = {}
+        for m in engine.model.modules():
+            if isinstance(m, c3.Conv3d):
+                c = m._cache
+                if c._asked and c3.packed_weight(engine.flat, c) is not m.weight:
+                    raise RuntimeError("a layer's operand copies are not the optimizer's to renew")
+                layouts[c] = set(c._asked), set(c._fresh), dict(c._bufs)
         self.packs = c3.pack_buffers(engine.flat)
         pool = torch.cuda.graph_pool_handle()
         self.forward_graph, self.backward_graph = torch.cuda.CUDAGraph(), None
@@ -124,9 +132,14 @@ class _Pass:
                 with torch.cuda.graph(self.backward_graph, pool=pool, capture_error_mode="thread_local"):
                     loss.backward()
                 self.back_launches = _lib.launch_count() - before
+            if any(c._asked != asked or c._bufs.keys() != bufs.keys() for c, (asked, _, bufs) in layouts.items()):
+                raise RuntimeError("a layer asked for a layout that the passes before had not")
         finally:
             for c in convs:
                 c._vals = {}  # these tensors live in the graph's memory
+            for c, (asked, fresh, bufs) in layouts.items():
+                c._asked, c._bufs = asked, bufs
+                c._fresh &= fresh  # packing that was recorded has not run
         self.out = out
         self.stream = torch.cuda.current_stream()
 

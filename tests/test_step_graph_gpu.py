@@ -127,3 +127,85 @@ def test_an_observer_of_operations_sees_the_ordinary_pass(what):
     with ctx():
         eng.step(*batch)
     assert bool(packed) is (what == "saved_tensors")
+
+
+@pytest.mark.parametrize("how", ["deepcopy", "assign"])
+def test_validation_of_a_copied_model_follows_its_weights(how):
+    """The operand copies of a model that was copied, or got new parameters, after a first pass."""
+    import copy
+
+    from scaffold_b200.models.unet import UNet
+    from scaffold_b200.ops.optim import FusedClipAdam
+    from scaffold_b200.train.engine import TrainEngine
+    dev = torch.device("cuda")
+
+    def make(graphs):
+        torch.manual_seed(3)
+        model = UNet(3, 5, layers=2, base_width=32).cuda()
+        TrainEngine(model, FusedClipAdam(model.parameters(), lr=1e-3), 5, dev).eval_step(*_batch(0))
+        if how == "deepcopy":
+            model = copy.deepcopy(model)
+        else:
+            model.load_state_dict({k: v.clone() for k, v in model.state_dict().items()}, assign=True)
+        eng = TrainEngine(model, FusedClipAdam(model.parameters(), lr=1e-3), 5, dev)
+        if not graphs:
+            eng._graphs.get = lambda *a, **k: None
+        return eng
+
+    a, b = make(True), make(False)
+    batch = _batch(1)
+    for i in range(12):
+        if i in (5, 8):
+            for e in (a, b):
+                e.step(*batch)
+        if i == 10:
+            for e in (a, b):
+                e.model.load_state_dict({k: v * 0.9 for k, v in e.model.state_dict().items()})
+        for s, t in zip(a.eval_step(*batch), b.eval_step(*batch)):
+            assert torch.equal(s, t), i
+    assert _captured(a) and not _captured(b)
+
+
+def test_copies_that_nothing_would_renew_keep_the_ordinary_pass():
+    from scaffold_b200.ops import conv3d as c3
+    a, b = _engine(True), _engine(False)
+    batch = _batch(1)
+    for e in (a, b):
+        e.eval_step(*batch)
+    conv = a.model.up_list[0].conv.double_conv[3]
+    c3._PACK_REGISTRY.discard(conv._cache)
+    conv._cache.conv3 = lambda w, *r: (type(conv._cache).conv3(conv._cache, w, *r),
+                                       c3._PACK_REGISTRY.discard(conv._cache))[0]
+    for i in range(8):
+        if i == 6:
+            for e in (a, b):
+                e.step(*batch)
+        for s, t in zip(a.eval_step(*batch), b.eval_step(*batch)):
+            assert torch.equal(s, t), i
+    assert not _captured(a)
+
+
+def test_a_failed_capture_leaves_no_copies_marked_fresh(monkeypatch):
+    """Packing that was recorded but never run must not count as done."""
+    a, b = _engine(True), _engine(False)
+    batch = _batch(1)
+    for e in (a, b):
+        for _ in range(2):
+            e.step(*batch)
+    ordinary = type(a).forward_loss
+
+    def failing(self, *args):
+        for m in self.model.modules():
+            if getattr(m, "_cache", None) is not None:
+                m._cache._fresh, m._cache._bufs = set(), {}   # the pass packs for itself
+        ordinary(self, *args)
+        raise RuntimeError("out of memory, say")
+
+    with monkeypatch.context() as m:
+        m.setattr(type(a), "forward_loss", failing)
+        stream = torch.cuda.current_stream()
+        assert a._graphs.get(a, *batch, train=True) is None
+        assert torch.cuda.current_stream() == stream
+    for _ in range(3):
+        assert torch.equal(a.step(*batch), b.step(*batch))
+        assert torch.equal(a.flat.data, b.flat.data)
