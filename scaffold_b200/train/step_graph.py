@@ -18,6 +18,7 @@ per engine. The memory is given back with the engine.
 from __future__ import annotations
 
 import math
+import weakref
 from typing import Optional
 
 import torch
@@ -165,6 +166,7 @@ class StepGraphs:
 
     def __init__(self):
         self._passes = {}   # key -> _Pass, or the number of ordinary passes seen, or None (cannot be captured)
+        self._model = None  # weak reference to the model that these passes are of
 
     @staticmethod
     def _usable(engine, images, masks) -> bool:
@@ -181,6 +183,9 @@ class StepGraphs:
 
     def get(self, engine, images, masks, train: bool) -> Optional[_Pass]:
         """The captured pass for this batch's shape, or None: run the ordinary pass."""
+        if self._model is None or self._model() is not engine.model:  # the engine has another model now
+            self._passes = {}
+            self._model = weakref.ref(engine.model)
         if images.dim() != 5 or not self._usable(engine, images, masks) or torch.is_grad_enabled() is not train:
             return None
         key = (train, tuple(images.shape), images.dtype, tuple(masks.shape), masks.dtype)

@@ -209,3 +209,29 @@ def test_a_failed_capture_leaves_no_copies_marked_fresh(monkeypatch):
     for _ in range(3):
         assert torch.equal(a.step(*batch), b.step(*batch))
         assert torch.equal(a.flat.data, b.flat.data)
+
+
+def test_another_model_in_the_engine_leaves_the_captured_passes():
+    import copy
+    a, b = _engine(True), _engine(False)
+    batch = _batch(4)
+    for _ in range(4):
+        for e in (a, b):
+            e.step(*batch)
+            e.eval_step(*batch)
+    assert len(_captured(a)) == 2
+    averaged = copy.deepcopy(a.model)
+    with torch.no_grad():
+        for p in averaged.parameters():
+            p.mul_(0.7)
+    models = a.model, b.model
+    a.model = b.model = averaged
+    for _ in range(5):
+        for s, t in zip(a.eval_step(*batch), b.eval_step(*batch)):
+            assert torch.equal(s, t)
+    a.model, b.model = models
+    for _ in range(4):
+        assert torch.equal(a.step(*batch), b.step(*batch))
+        for s, t in zip(a.eval_step(*batch), b.eval_step(*batch)):
+            assert torch.equal(s, t)
+    assert len(_captured(a)) == 2
