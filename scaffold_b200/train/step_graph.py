@@ -19,14 +19,20 @@ from __future__ import annotations
 
 import math
 import weakref
+from operator import eq, is_
+from types import FunctionType
 from typing import Optional
 
 import torch
+import torch.nn as nn
 
+from ..models import unet
 from ..models.unet import UNet
-from ..ops import _lib, conv_kernels as ck, layout, pool_kernels
+from ..ops import _lib, conv_kernels as ck, layout, loss as losses, pool_kernels
 from ..ops import conv3d as c3
+from ..ops.group_norm import GroupNorm
 from ..ops.optim import FusedClipAdam
+from ..ops.pool import MaxPool3d
 from ..utils import perf
 
 WARM_PASSES = 2        # ordinary passes over a shape before its capture (kernels set up, operand layouts known)
@@ -43,47 +49,74 @@ def _watched() -> bool:
                 or torch._C._functorch.maybe_current_level() is not None or torch._C._get_tracing_state() is not None)
 
 
+# The modules whose passes are known to be kernels and nothing else. Any other one (a dropout in an Identity's place, a
+# subclass) may keep state of its own in Python.
+_MODULES = (UNet, unet.DoubleConv, unet.Down, unet.Up, unet.OutConv, unet._FirstConvSequential, c3.Conv3d,
+            c3.ConvTranspose3d, GroupNorm, MaxPool3d, nn.Sequential, nn.ModuleList, nn.Identity, nn.Upsample)
+_ENGINE_STEPS = ("to_device", "_autocast", "forward_loss", "_eval_pass")
+
+
+def _functions(engine) -> list:
+    """The functions that a pass runs, wherever they could be replaced for all instances."""
+    return [t.forward for t in _MODULES] + [getattr(type(engine), n) for n in _ENGINE_STEPS] + [
+        UNet.forward_padded_logits, UNet.features, UNet._run, unet.Down.forward_with_skip, unet.Down._after_pool,
+        c3.Conv3d.forward_padded, c3.Conv3d._cuda_forward, ck.conv_same, ck.conv_wgrad, ck.convT_fwd, ck.convT_dgrad,
+        losses.segmentation_loss_fused, losses.hard_dice_fused]
+
+
+def _replaced_steps(engine) -> bool:
+    """True for an engine whose steps are not TrainEngine's: a subclass, or functions of its own."""
+    from .engine import TrainEngine
+    t = type(engine)
+    return any(n in engine.__dict__ or (t is not TrainEngine and getattr(t, n) is not getattr(TrainEngine, n))
+               for n in _ENGINE_STEPS)
+
+
 class _Fingerprint:
-    """What a captured pass depends on besides the batch's values; ``holds()`` is a few hundred identity checks."""
+    """What a captured pass depends on besides the batch's values; ``holds()`` is some thousand identity checks."""
 
     def __init__(self, engine):
         modules = list(engine.model.modules())
-        self._dicts = [(d, tuple(d.items())) for m in modules for d in (m._parameters, m._buffers, m._modules)]
+        # every attribute of every module: settings, mode, a forward or a compiled call of its own, ... (dicts compare
+        # their values by identity first; tensors are looked at by identity alone)
+        self._dicts = [d for m in modules for d in (m.__dict__, m._modules)]
+        self._were = [dict(d) for d in self._dicts]
+        self._tensors = [d for m in modules for d in (m._parameters, m._buffers)]
+        self._named = self._items(self._tensors)
         self._hooks = [h for m in modules for h in (m._forward_hooks, m._forward_pre_hooks, m._backward_hooks,
                                                     m._backward_pre_hooks)]
         self._params = [(p, p.data_ptr(), p.requires_grad) for p in engine.model.parameters()]
-        self._modules = modules
+        self._known = all(type(m) in _MODULES and m._compiled_call_impl is None
+                          and not any(isinstance(getattr(type(m), n, None), FunctionType) for n in m.__dict__)
+                          for m in modules)
+        self._code = _functions(engine)
         self._settings = self._read(engine)
 
-    def _read(self, engine):
-        out = [m.training for m in self._modules]
-        for m in self._modules:
-            d = m.__dict__
-            if "eps" in d:  # GroupNorm
-                out += (d["eps"], d["num_groups"], d["activation"], d["_spatial"])
-            elif "kernel_size" in d:  # convolutions, pooling
-                out += (d["kernel_size"], d["stride"], d["padding"], d.get("gn_groups_hint"), d.get("_spatial"))
+    @staticmethod
+    def _read(engine):
         cw = engine.class_weights
-        out += (engine.amp, engine.n_classes, id(cw), 0 if cw is None else cw.data_ptr(), engine.model.checkpointing,
-                engine.model._spatial, id(engine.model.forward_padded_logits.__func__), engine.flat.data.data_ptr(),
-                engine.flat.grad.data_ptr(), ck.PAIR_CONV, c3._GN_FROM_EPILOGUE, pool_kernels._USE_INDEX,
-                ck.conv_same, ck.conv_wgrad, ck.convT_fwd, ck.convT_dgrad)
-        return out
+        return (engine.amp, engine.n_classes, id(cw), 0 if cw is None else cw.data_ptr(), engine.flat.data.data_ptr(),
+                engine.flat.grad.data_ptr(), ck.PAIR_CONV, c3._GN_FROM_EPILOGUE, pool_kernels._USE_INDEX)
 
     def holds(self, engine) -> bool:
-        for h in self._hooks:
-            if h:
+        if not self._known or any(self._hooks):
+            return False
+        try:
+            if not all(map(eq, self._dicts, self._were)):
                 return False
-        for d, items in self._dicts:
-            if len(d) != len(items):
-                return False
-            for k, v in items:
-                if d.get(k) is not v:
-                    return False
+        except RuntimeError:  # a tensor in an attribute that was another one: it has no truth value
+            return False
+        now = self._items(self._tensors)
+        if len(now) != len(self._named) or not all(map(is_, now, self._named)):
+            return False
         for p, ptr, needs in self._params:
             if p.data_ptr() != ptr or p.requires_grad is not needs or p._backward_hooks or p._post_accumulate_grad_hooks:
                 return False
-        return self._settings == self._read(engine)
+        return self._settings == self._read(engine) and self._code == _functions(engine)
+
+    @staticmethod
+    def _items(dicts) -> list:
+        return [v for d in dicts for kv in d.items() for v in kv]
 
 
 class _Pass:
@@ -173,7 +206,7 @@ class StepGraphs:
         model = engine.model
         if not (engine.cuda and engine.fused_loss and engine.flat is not None and type(model) is UNet
                 and isinstance(engine.optimizer, FusedClipAdam) and engine.reducer.world == 1
-                and engine.spatial is None and model._spatial is None):
+                and engine.spatial is None and model._spatial is None and not _replaced_steps(engine)):
             return False
         widest = images.shape[0] * math.prod(images.shape[2:]) * model.base_width * 2
         return (widest <= MAX_MAP_BYTES and not model.checkpointing and not layout._aten_only[0]
@@ -209,7 +242,8 @@ class StepGraphs:
         if sum(isinstance(p, _Pass) and k[0] == train for k, p in self._passes.items()) >= MAX_SHAPES:
             return None
         probe = _Fingerprint(engine)
-        if not probe.holds(engine):  # hooks are set
+        if not probe.holds(engine):  # hooks are set, or a module is not one of the model's own: look again later
+            self._passes[key] = 0
             return None
         try:
             self._passes[key] = _Pass(engine, images, masks, train)

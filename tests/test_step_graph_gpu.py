@@ -235,3 +235,65 @@ def test_another_model_in_the_engine_leaves_the_captured_passes():
         for s, t in zip(a.eval_step(*batch), b.eval_step(*batch)):
             assert torch.equal(s, t)
     assert len(_captured(a)) == 2
+
+
+def _counting(fn, seen):
+    def call(*args, **kwargs):
+        seen.append(1)
+        return fn(*args, **kwargs)
+    return call
+
+
+@pytest.mark.parametrize("what", ["block", "head", "padded", "features", "forward_loss", "eval_pass", "to_device"])
+@pytest.mark.parametrize("when", ["before", "after"])
+def test_a_replaced_function_runs_on_every_pass(what, when):
+    eng = _engine(True)
+    batch = _batch(1)
+    owner, name = {"block": (eng.model.down_list[1], "forward"), "head": (eng.model.up_list[-1].conv, "forward_padded"),
+                   "padded": (eng.model, "forward_padded_logits"), "features": (eng.model, "features"),
+                   "forward_loss": (eng, "forward_loss"), "eval_pass": (eng, "_eval_pass"),
+                   "to_device": (eng, "to_device")}[what]
+
+    def passes(n):
+        for _ in range(n):
+            eng.eval_step(*batch)
+    if when == "after":
+        passes(4)
+        assert len(_captured(eng)) == 1
+    seen = []
+    setattr(owner, name, _counting(getattr(owner, name), seen))   # a plain function on the instance
+    passes(5)
+    assert len(seen) == 5
+    delattr(owner, name)
+    passes(4)
+    assert len(seen) == 5 and len(_captured(eng)) == 1
+
+
+@pytest.mark.parametrize("setting", ["compiled", "dilation", "attribute", "class_function", "submodule", "subclass"])
+def test_what_a_pass_depends_on_ends_the_replays(setting, monkeypatch):
+    from scaffold_b200.ops import conv3d as c3
+    eng = _engine(True)
+    batch = _batch(1)
+    for _ in range(4):
+        eng.eval_step(*batch)
+    assert _captured(eng)
+    conv = eng.model.down_list[1].maxpool_conv[1].double_conv
+    if setting == "compiled":
+        conv[0]._compiled_call_impl = conv[0]._call_impl   # what Module.compile() sets
+    elif setting == "dilation":
+        conv[0].dilation = (2, 2, 2)
+    elif setting == "attribute":
+        conv[1].num_groups = 4
+    elif setting == "class_function":
+        monkeypatch.setattr(c3.Conv3d, "_cuda_forward", _counting(c3.Conv3d._cuda_forward, []))
+    elif setting == "submodule":
+        conv[2] = torch.nn.Dropout3d(0.5)
+    else:
+        class Mine(type(eng)):
+            def forward_loss(self, *args):
+                return super().forward_loss(*args)
+        eng.__class__ = Mine
+    assert eng._graphs.get(eng, *batch, train=False) is None
+    if setting in ("submodule", "subclass", "compiled"):   # ... and there are none of such a model
+        with torch.no_grad():
+            assert all(eng._graphs.get(eng, *batch, train=False) is None for _ in range(5))
