@@ -126,8 +126,7 @@ class _Pass:
         dev = engine.device
         self.images = torch.empty(images.shape, dtype=images.dtype, device=dev)
         self.masks = torch.empty(masks.shape, dtype=masks.dtype, device=dev)
-        self.images.copy_(images)
-        self.masks.copy_(masks)
+        self._load(images, masks)
         self.fingerprint = _Fingerprint(engine)
         self.class_weights = engine.class_weights  # the kernels read it at its address: keep it alive
         convs = [c for m in engine.model.modules() for c in (getattr(m, "_cache", None), getattr(m, "_cache_b", None))
@@ -177,14 +176,18 @@ class _Pass:
         self.out = out
         self.stream = torch.cuda.current_stream()
 
+    @torch.no_grad()
+    def _load(self, images, masks):
+        self.images.copy_(images, non_blocking=True)
+        self.masks.copy_(masks, non_blocking=True)
+
     def forward(self, engine, images, masks):
         stream = torch.cuda.current_stream()
         if stream != self.stream:  # the buffers are the graph's: a pass on another stream comes after the last one
             stream.wait_stream(self.stream)
             self.stream = stream
         c3.refresh_packs(engine.flat)
-        self.images.copy_(images, non_blocking=True)
-        self.masks.copy_(masks, non_blocking=True)
+        self._load(images, masks)
         self.forward_graph.replay()
         _lib.lib().sb_count_launch(self.launches)
         return tuple(t.clone() for t in self.out)
@@ -220,6 +223,8 @@ class StepGraphs:
             self._passes = {}
             self._model = weakref.ref(engine.model)
         if images.dim() != 5 or not self._usable(engine, images, masks) or torch.is_grad_enabled() is not train:
+            return None
+        if images.requires_grad:  # the caller wants the gradient of the batch itself (and its first layer takes another path)
             return None
         key = (train, tuple(images.shape), images.dtype, tuple(masks.shape), masks.dtype)
         seen = self._passes.get(key, 0)

@@ -297,3 +297,30 @@ def test_what_a_pass_depends_on_ends_the_replays(setting, monkeypatch):
     if setting in ("submodule", "subclass", "compiled"):   # ... and there are none of such a model
         with torch.no_grad():
             assert all(eng._graphs.get(eng, *batch, train=False) is None for _ in range(5))
+
+
+@pytest.mark.parametrize("captured_first", [False, True])
+def test_a_batch_that_needs_a_gradient_gets_it(captured_first):
+    a, b = _engine(True), _engine(False)
+    for _ in range(4 if captured_first else 0):
+        for e in (a, b):
+            e.step(*_batch(0))
+    for i in range(5):
+        grads = []
+        for e in (a, b):
+            x, y = _batch(i)
+            x.requires_grad_()
+            e.step(x, y)
+            grads.append(x.grad)
+        assert grads[0] is not None and torch.equal(*grads)
+    for _ in range(5):   # the ordinary batches around it are replayed, from buffers that are no part of a graph
+        assert torch.equal(a.step(*_batch(9)), b.step(*_batch(9)))
+    assert len(_captured(a)) == 1
+    static = a._graphs._passes[_captured(a)[0]].images
+    assert static.is_leaf and not static.requires_grad
+    assert torch.equal(a.flat.data, b.flat.data)
+    x, y = _batch(3)
+    for i in range(8):
+        x.requires_grad_(i % 2 == 0)
+        assert torch.equal(a.eval_step(x, y)[0], b.eval_step(x, y)[0])
+    assert len(_captured(a)) == 2
