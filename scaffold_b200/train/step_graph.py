@@ -224,6 +224,8 @@ class StepGraphs:
             self._model = weakref.ref(engine.model)
         if images.dim() != 5 or not self._usable(engine, images, masks) or torch.is_grad_enabled() is not train:
             return None
+        if torch.is_inference_mode_enabled():  # buffers made in it could not be written outside of it
+            return None
         if images.requires_grad:  # the caller wants the gradient of the batch itself (and its first layer takes another path)
             return None
         key = (train, tuple(images.shape), images.dtype, tuple(masks.shape), masks.dtype)

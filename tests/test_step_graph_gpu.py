@@ -324,3 +324,18 @@ def test_a_batch_that_needs_a_gradient_gets_it(captured_first):
         x.requires_grad_(i % 2 == 0)
         assert torch.equal(a.eval_step(x, y)[0], b.eval_step(x, y)[0])
     assert len(_captured(a)) == 2
+
+
+def test_validation_inside_and_outside_of_inference_mode():
+    a, b = _engine(True), _engine(False)
+    batch = _batch(2)
+    for i in range(14):
+        with torch.inference_mode(i < 4 or i % 3 == 0):
+            got, want = a.eval_step(*batch), b.eval_step(*batch)
+            assert [t.is_inference() for t in got] == [t.is_inference() for t in want]
+            for s, t in zip(got, want):
+                assert torch.equal(s, t), i
+        if i == 8:
+            for e in (a, b):
+                e.step(*batch)
+    assert len(_captured(a)) == 1
