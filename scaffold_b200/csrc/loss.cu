@@ -225,11 +225,12 @@ __global__ void __launch_bounds__(256) loss_finalize_kernel(const float* __restr
 }
 
 // From the sums of all shards: dice[N][C] and, when asked for, the loss and what its gradient needs.
-//   out[3]: ce + (1 - fg), ce, fg (mean foreground Dice)
+//   loss[1] = ce + (1 - fg), ce[1], fg[1] (mean foreground Dice)
 //   coef[N][2][C]: alpha, beta of d(-fg)/dp_c (zero for class 0 and for a class that is absent on both sides), den[1]
 // One block: N * C is a few dozen values; in torch operations the same arithmetic is some thirty launches.
 __global__ void __launch_bounds__(256) loss_head_kernel(const float* __restrict__ sums, int N, int C,
-                                                        float* __restrict__ dice, float* __restrict__ out,
+                                                        float* __restrict__ dice, float* __restrict__ loss,
+                                                        float* __restrict__ ce_out, float* __restrict__ fg_out,
                                                         float* __restrict__ coef, float* __restrict__ den_out) {
   __shared__ float red[3][8];
   const int K = 3 * C + 2, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(256) loss_head_kernel(const float* __restrict_
       coef[((long long)n * 2 + 1) * C + c] = on ? (inter2 + LOSS_EPS) / (m * u * u) : 0.f;
     }
   }
-  if (out == nullptr) return;
+  if (loss == nullptr) return;
   for (int n = threadIdx.x; n < N; n += 256) {
     num += sums[(long long)n * K + 3 * C];
     den += sums[(long long)n * K + 3 * C + 1];
@@ -266,9 +267,9 @@ __global__ void __launch_bounds__(256) loss_head_kernel(const float* __restrict_
     den = fmaxf(den, 1.1920929e-7f);  // the smallest fp32 step above 1, as clamp_min(finfo.eps)
     fg /= m;
     const float ce = num / den;
-    out[0] = ce + (1.f - fg);
-    out[1] = ce;
-    out[2] = fg;
+    loss[0] = ce + (1.f - fg);
+    ce_out[0] = ce;
+    fg_out[0] = fg;
     den_out[0] = den;
   }
 }
@@ -393,12 +394,14 @@ extern "C" int sb_loss_sums(const void* logits, const void* labels, int label_ki
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }
 
-// dice[N][C]; out[3] = loss, ce, fg; coef[N][2][C]; den[1] (out, coef and den together, or all null)
-extern "C" int sb_loss_head(const float* sums, int N, int C, float* dice, float* out, float* coef, float* den,
-                            cudaStream_t stream) {
-  if (N < 1 || C < 1 || (out == nullptr) != (coef == nullptr) || (out == nullptr) != (den == nullptr))
-    return SB_ERR_SHAPE;
-  loss_head_kernel<<<1, 256, 0, stream>>>(sums, N, C, dice, out, coef, den);
+// dice[N][C]; loss[1], ce[1], fg[1], coef[N][2][C] and den[1] together, or all null
+extern "C" int sb_loss_head(const float* sums, int N, int C, float* dice, float* loss, float* ce, float* fg, float* coef,
+                            float* den, cudaStream_t stream) {
+  if (N < 1 || C < 1) return SB_ERR_SHAPE;
+  const void* all[5] = {loss, ce, fg, coef, den};
+  for (const void* p : all)
+    if ((p == nullptr) != (loss == nullptr)) return SB_ERR_SHAPE;
+  loss_head_kernel<<<1, 256, 0, stream>>>(sums, N, C, dice, loss, ce, fg, coef, den);
   sb_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }

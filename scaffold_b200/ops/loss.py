@@ -29,7 +29,7 @@ from . import _lib
 _P = C.c_void_p
 _lib.register("sb_loss_blocks", [C.c_longlong], C.c_int)
 _lib.register("sb_loss_sums", [_P, _P, C.c_int, _P, _P, _P, C.c_int, C.c_longlong, C.c_int, C.c_int, C.c_int, _P, _P])
-_lib.register("sb_loss_head", [_P, C.c_int, C.c_int, _P, _P, _P, _P, _P])
+_lib.register("sb_loss_head", [_P, C.c_int, C.c_int, _P, _P, _P, _P, _P, _P, _P])
 _lib.register("sb_loss_grad", [_P, _P, C.c_int, _P, _P, _P, _P, _P, C.c_int, C.c_longlong, C.c_int, C.c_int, _P, _P])
 
 FUSED_MAX_CLASSES = 32  # widest head of csrc/loss.cu (LOSS_MAXC); wider heads take the PyTorch formula
@@ -133,15 +133,15 @@ class _FusedLossFn(torch.autograd.Function):
             spatial.all_reduce_sum(sums)
         n = sums.shape[0]
         dev = sums.device
-        out = torch.empty(3, dtype=torch.float32, device=dev)  # loss, ce, fg
+        loss, ce, fg = (torch.empty((), dtype=torch.float32, device=dev) for _ in range(3))
         coef = torch.empty((n, 2, c), dtype=torch.float32, device=dev)
         den = torch.empty(1, dtype=torch.float32, device=dev)
-        _lib.check(_lib.lib().sb_loss_head(sums.data_ptr(), n, c, None, out.data_ptr(), coef.data_ptr(),
-                                           den.data_ptr(), _lib.stream_ptr()), "sb_loss_head")
+        _lib.check(_lib.lib().sb_loss_head(sums.data_ptr(), n, c, None, loss.data_ptr(), ce.data_ptr(), fg.data_ptr(),
+                                           coef.data_ptr(), den.data_ptr(), _lib.stream_ptr()), "sb_loss_head")
         ctx.save_for_backward(logits_vm, labels, coef, den)
         ctx.cw, ctx.c = cw, c
         ctx.mark_non_differentiable(labels)
-        return out[0], out[1], out[2]
+        return loss, ce, fg
 
     @staticmethod
     def backward(ctx, g, _gce, _gfg):
@@ -174,8 +174,8 @@ def hard_dice_fused(logits_vm: torch.Tensor, labels: torch.Tensor, n_classes: in
     if spatial is not None and spatial.size > 1:
         spatial.all_reduce_sum(sums)
     dice = torch.empty((sums.shape[0], c), dtype=torch.float32, device=sums.device)
-    _lib.check(_lib.lib().sb_loss_head(sums.data_ptr(), sums.shape[0], c, dice.data_ptr(), None, None, None,
-                                       _lib.stream_ptr()), "sb_loss_head")
+    _lib.check(_lib.lib().sb_loss_head(sums.data_ptr(), sums.shape[0], c, dice.data_ptr(), None, None, None, None,
+                                       None, _lib.stream_ptr()), "sb_loss_head")
     return dice
 
 

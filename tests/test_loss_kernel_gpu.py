@@ -46,3 +46,21 @@ def test_hard_dice_matches_the_formula(classes, shape):
     got = L.hard_dice_fused(logits, labels, classes)
     ref = L.hard_dice_reference(logits[..., :classes].permute(0, 4, 1, 2, 3).float(), labels, classes)
     torch.testing.assert_close(got, ref, rtol=2e-7, atol=0)  # counts are exact; one quotient in fp32
+
+
+def test_the_loss_can_be_changed_in_place():
+    """The three results are tensors of their own, as the formula's are (gradient accumulation: ``loss /= n``)."""
+    from scaffold_b200.ops import loss as L
+    g = torch.Generator(device="cuda").manual_seed(1)
+    logits = torch.randn((2, 4, 5, 6, 16), generator=g, device="cuda").to(torch.bfloat16)
+    labels = torch.randint(0, 5, (2, 4, 5, 6), generator=g, device="cuda", dtype=torch.int16)
+    a, b = logits.clone().requires_grad_(), logits.clone().requires_grad_()
+    loss, ce, fg = L.segmentation_loss_fused(a, labels, 5, None)
+    values = float(ce), float(fg)
+    loss /= 4
+    loss.mul_(3.0).add_(1.0)
+    loss.backward()
+    ref, *_ = L.segmentation_loss_fused(b, labels, 5, None)
+    (ref / 4 * 3.0 + 1.0).backward()
+    assert torch.equal(loss, ref / 4 * 3.0 + 1.0) and torch.equal(a.grad, b.grad)
+    assert (float(ce), float(fg)) == values and not (loss._is_view() or ce._is_view() or fg._is_view())
