@@ -106,7 +106,7 @@ __device__ __forceinline__ void stat_store(float* dst, const StatSums& a) {
   const double m2 = a.s2 - a.s1 * mean;
   dst[0] = (float)a.n;
   dst[1] = (float)mean;
-  dst[2] = (float)(m2 > 0.0 ? m2 : 0.0);
+  dst[2] = (float)(m2 < 0.0 ? 0.0 : m2);  // a NaN stays one: an overflow has to show in what follows
 }
 // The sums of partials first, first + step, ... of (n, g) (`base`: partial 0), eight partials in flight. Loads bypass
 // L1 (the partials may have been written by other SMs during this launch).

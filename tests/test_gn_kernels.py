@@ -149,3 +149,39 @@ def test_finalize_pools_partials_like_fp64(nsplit):
     ref = torch.stack([tot, mean, (m2 + n * (m - mean[:, None]) ** 2).sum(1)], -1)
     # sums in double, results rounded once to fp32: 2^-24, doubled for the subtraction in M2
     torch.testing.assert_close(got, ref, rtol=2 ** -22, atol=1e-3)
+
+
+@pytest.mark.parametrize("nsplit", [1, 32, 33, 1024, 1025])
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+def test_finalize_keeps_what_is_not_finite(nsplit, bad):
+    """A partial over an infinity has that mean and a NaN for M2; its group's variance is NaN, as the formula's is."""
+    from scaffold_b200.ops import gn_kernels as gk
+    part = torch.ones((2, nsplit, 8, 3), device="cuda")
+    part[1, nsplit // 2, 3, 1], part[1, nsplit // 2, 3, 2] = bad, float("nan")
+    got = gk.gn_finalize(part.reshape(-1), 2, 8, nsplit).view(2, 8, 3)
+    expect = torch.zeros((2, 8), dtype=torch.bool, device="cuda")
+    expect[1, 3] = True
+    assert torch.equal(got[..., 2].isnan(), expect) and torch.equal(~got[..., 1].isfinite(), expect)
+
+
+@pytest.mark.parametrize("dims", [(4, 5, 6), (24, 24, 24)])
+@pytest.mark.parametrize("through", ["statistics", "convolution"])
+def test_an_infinite_activation_makes_its_group_nan(dims, through):
+    from scaffold_b200.ops.conv3d import Conv3d
+    from scaffold_b200.ops.group_norm import GroupNorm
+    torch.manual_seed(0)
+    x = torch.randn((2, 64, *dims), device="cuda").to(torch.bfloat16).to(memory_format=torch.channels_last_3d)
+    norm = GroupNorm(8, 64, activation="relu").cuda()
+    conv = Conv3d(64, 64, 3, padding=1, bias=False).cuda()
+    conv.gn_groups_hint = 8
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        if through == "convolution":
+            conv.weight[17] = 3e38   # its output overflows where the inputs add up
+            x[1] = x[1].abs() * 100
+            x[0] = 0
+            y = norm(conv(x))
+        else:
+            x[1, 17, 1, 2, 3] = float("inf")
+            y = norm(x)
+    assert y[1, 16:24].isnan().all() and not y[0].isnan().any()
+    assert not y[1, :16].isnan().any() and not y[1, 24:].isnan().any()
