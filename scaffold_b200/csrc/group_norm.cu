@@ -135,13 +135,22 @@ __device__ __forceinline__ StatSums stat_warp_sum(StatSums a) {
   return a;
 }
 
-// One warp collapses the `nsplit` partials of (n, g) in a fixed order (lane-strided, then xor shuffles): the separate
-// finalize kernel and the last-block tail of the statistics kernel run exactly this, so both give the same bits.
+// One warp collapses the `nsplit` partials of (n, g): up to 32 of them one per lane, more as GN_FIN_WARPS strands (32
+// lanes each, partials strand * 32 + lane, + 128, ...) whose sums it adds in order. The separate finalize launch gives
+// each strand a warp of its own (gn_stats_finalize_block_kernel) and takes the same sums in the same order, so it and
+// the last-block tail of the statistics kernel give the same bits.
 // 592 partials, kernel time: 13 us as a chain of Chan merges (one L2 latency and one division each).
+constexpr int GN_FIN_WARPS = 4;
 __device__ __forceinline__ void stats_collapse_warp(const float* __restrict__ part, float* __restrict__ fin, int G,
                                                     int nsplit, int n, int g, int lane) {
-  const StatSums a = stat_warp_sum(stat_walk(part + ((long long)n * nsplit * G + g) * 3, G, lane, 32, nsplit));
-  if (lane == 0) stat_store(fin + ((long long)n * G + g) * 3, a);
+  const float* base = part + ((long long)n * nsplit * G + g) * 3;
+  StatSums t{0.0, 0.0, 0.0};
+  const int strands = nsplit > 32 ? GN_FIN_WARPS : 1;
+  for (int w = 0; w < strands; ++w) {
+    const StatSums a = stat_warp_sum(stat_walk(base, G, w * 32 + lane, strands * 32, nsplit));
+    t.n += a.n; t.s1 += a.s1; t.s2 += a.s2;
+  }
+  if (lane == 0) stat_store(fin + ((long long)n * G + g) * 3, t);
 }
 
 __device__ __forceinline__ void bwd_collapse_warp(const float* __restrict__ part, float* __restrict__ fin, int C,
@@ -576,7 +585,7 @@ __global__ void __launch_bounds__(GN_THREADS, GN_WAVE) gn_bwd_dx_kernel(const Gn
 
 // ----------------------------------------------------------------------------
 // finalize: collapse the per-split partials of one rank into a single entry per
-// (n, g) / (n, c), in parallel (one warp per output, fixed merge tree), so the
+// (n, g) / (n, c), in parallel and in a fixed order, so the
 // streaming kernels start from O(1) statistics instead of walking every split.
 // ----------------------------------------------------------------------------
 __global__ void __launch_bounds__(GN_THREADS) gn_stats_finalize_kernel(const float* __restrict__ part,
@@ -588,14 +597,13 @@ __global__ void __launch_bounds__(GN_THREADS) gn_stats_finalize_kernel(const flo
   stats_collapse_warp(part, fin, G, nsplit, warp / G, warp % G, lane);
 }
 
-// The same collapse with a block per (n, g) beyond 32 partials: a lane's 16 partials were two trips to L2 and 16 dependent
-// double additions, a thread's 4 are one trip (512 partials 4.9 us a
-// launch, now 2.7).
-constexpr int GN_FIN_THREADS = 128;
+// The same collapse with a block per (n, g), a warp per strand, beyond 32 partials: a lane's 16 partials were two trips
+// to L2 and 16 dependent double additions, a thread's 4 are one trip (512 partials 4.9 us a launch, now 2.7).
+constexpr int GN_FIN_THREADS = 32 * GN_FIN_WARPS;
 __global__ void __launch_bounds__(GN_FIN_THREADS) gn_stats_finalize_block_kernel(const float* __restrict__ part,
                                                                                  float* __restrict__ fin, int G,
                                                                                  int nsplit) {
-  __shared__ double s_w[GN_FIN_THREADS / 32][3];
+  __shared__ double s_w[GN_FIN_WARPS][3];
   const int n = blockIdx.x / G, g = blockIdx.x % G, warp = threadIdx.x >> 5;
   const StatSums a = stat_warp_sum(stat_walk(part + ((long long)n * nsplit * G + g) * 3, G, threadIdx.x, GN_FIN_THREADS,
                                              nsplit));
@@ -603,7 +611,7 @@ __global__ void __launch_bounds__(GN_FIN_THREADS) gn_stats_finalize_block_kernel
   __syncthreads();
   if (threadIdx.x == 0) {
     StatSums t{0.0, 0.0, 0.0};
-    for (int w = 0; w < GN_FIN_THREADS / 32; ++w) { t.n += s_w[w][0]; t.s1 += s_w[w][1]; t.s2 += s_w[w][2]; }
+    for (int w = 0; w < GN_FIN_WARPS; ++w) { t.n += s_w[w][0]; t.s1 += s_w[w][1]; t.s2 += s_w[w][2]; }
     stat_store(fin + ((long long)n * G + g) * 3, t);
   }
 }
@@ -829,7 +837,8 @@ extern "C" int sb_gn_share(const float* fin, long long count, void* const* dst, 
 // fin: [N][G][3] (stats) / [N][C][2] (bwd) -- the single-split form the apply / dx kernels merge
 extern "C" int sb_gn_stats_finalize(const float* part, float* fin, int N, int G, int nsplit, cudaStream_t stream) {
   const int warps = N * G;
-  if (nsplit > 1024) {  // a warp per output would walk more than 32 partials per lane: a cluster per output instead
+  // a warp per output up to 32 partials, a block of four up to 1024 (8 per thread, all in flight), a cluster beyond
+  if (nsplit > 1024) {
     gn_stats_finalize_wide_kernel<<<warps * GN_WIDE_CLUSTER, GN_THREADS, 0, stream>>>(part, fin, N, G, nsplit);
     sb_count_launch(1);
     return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;

@@ -90,10 +90,13 @@ def test_gn_two_shards_equal_whole_volume():
     assert (got - whole.float()).abs().max().item() <= 2 ** -6
 
 
-@pytest.mark.parametrize("shape,groups", [((2, 16, 32, 32, 64), 8), ((1, 8, 8, 8, 1024), 8), ((3, 5, 9, 7, 32), 4)])
+@pytest.mark.parametrize("shape,groups", [((2, 16, 32, 32, 64), 8), ((1, 8, 8, 8, 1024), 8), ((3, 5, 9, 7, 32), 4),
+                                          ((1, 8, 8, 16, 64), 8), ((1, 1, 24, 44, 64), 8), ((4, 8, 16, 16, 256), 8),
+                                          ((1, 32, 32, 32, 64), 8)])
 def test_last_block_collapse_equals_the_separate_finalize_launch(shape, groups, monkeypatch):
     """The statistics kernels can collapse their partials in the block that finishes last; the result must be the
-    bits of the separate finalize launch (same merge tree), forward and backward."""
+    bits of the separate finalize launch (same order of the sums), forward and backward. The shapes have 5 to 592
+    partials per output, 32 and 33 (one warp, four warps) among them."""
     from scaffold_b200.ops import _lib, gn_kernels as gk
     g = torch.Generator(device="cuda").manual_seed(21)
     x = torch.randn(shape, generator=g, device="cuda").to(torch.bfloat16)
@@ -131,10 +134,10 @@ def test_last_block_collapse_equals_the_separate_finalize_launch(shape, groups, 
     assert torch.equal(again, outs[0][0])
 
 
-@pytest.mark.parametrize("nsplit", [1, 31, 592, 1024, 1025, 2049, 16384])
+@pytest.mark.parametrize("nsplit", [1, 31, 32, 33, 128, 129, 592, 1024, 1025, 2049, 16384])
 def test_finalize_pools_partials_like_fp64(nsplit):
-    """Both collapse kernels (a warp per output up to 1024 partials, a cluster of eight CTAs beyond), empty partials and
-    a mean of a hundred standard deviations included."""
+    """All three collapse kernels (a warp per output up to 32 partials, a block up to 1024, a cluster of eight CTAs
+    beyond), empty partials and a mean of a hundred standard deviations included."""
     from scaffold_b200.ops import gn_kernels as gk
     g = torch.Generator(device="cuda").manual_seed(nsplit)
     part = torch.empty((2, nsplit, 8, 3), device="cuda")
