@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(256) loss_head_kernel(const float* __restrict_
   if (threadIdx.x == 0) {
     fg = num = den = 0.f;
     for (int w = 0; w < 8; ++w) { fg += red[0][w]; num += red[1][w]; den += red[2][w]; }
-    den = fmaxf(den, 1.1920929e-7f);  // the smallest fp32 step above 1, as clamp_min(finfo.eps)
+    den = den < 1.1920929e-7f ? 1.1920929e-7f : den;  // the fp32 step above 1, as clamp_min(finfo.eps): a NaN stays one
     fg /= m;
     const float ce = num / den;
     loss[0] = ce + (1.f - fg);

@@ -56,11 +56,25 @@ def test_the_loss_can_be_changed_in_place():
     labels = torch.randint(0, 5, (2, 4, 5, 6), generator=g, device="cuda", dtype=torch.int16)
     a, b = logits.clone().requires_grad_(), logits.clone().requires_grad_()
     loss, ce, fg = L.segmentation_loss_fused(a, labels, 5, None)
-    values = float(ce), float(fg)
+    values = float(ce.detach()), float(fg.detach())
     loss /= 4
     loss.mul_(3.0).add_(1.0)
     loss.backward()
     ref, *_ = L.segmentation_loss_fused(b, labels, 5, None)
     (ref / 4 * 3.0 + 1.0).backward()
     assert torch.equal(loss, ref / 4 * 3.0 + 1.0) and torch.equal(a.grad, b.grad)
-    assert (float(ce), float(fg)) == values and not (loss._is_view() or ce._is_view() or fg._is_view())
+    assert (float(ce.detach()), float(fg.detach())) == values and not (loss._is_view() or ce._is_view() or fg._is_view())
+
+
+def test_a_nan_class_weight_shows_in_every_gradient():
+    """The cross-entropy's denominator is NaN then, for the voxels of the other classes too."""
+    from scaffold_b200.ops import loss as L
+    g = torch.Generator(device="cuda").manual_seed(1)
+    logits = torch.randn((2, 4, 5, 6, 16), generator=g, device="cuda").to(torch.bfloat16).requires_grad_()
+    labels = torch.randint(0, 5, (2, 4, 5, 6), generator=g, device="cuda", dtype=torch.int16)
+    weights = torch.ones(5, device="cuda")
+    weights[2] = float("nan")
+    loss, ce, fg = L.segmentation_loss_fused(logits, labels, 5, weights)
+    loss.backward()
+    assert loss.isnan() and ce.isnan() and fg.isfinite()
+    assert logits.grad[..., :5].isnan().all()
