@@ -215,9 +215,9 @@ def _pack_point(w: torch.Tensor, src_c: Sequence[int], real_c: Sequence[int], dg
     return (ck.pack_weight_dgrad if dgrad else ck.pack_weight_fwd)(_pad_in_channels(w, src_c, real_c))
 
 
-def _bias_grad(gy: torch.Tensor, n_out: int, bias) -> Optional[torch.Tensor]:
+def _bias_grad(ctx, gy: torch.Tensor, n_out: int, bias) -> Optional[torch.Tensor]:
     """Bias gradient for autograd, or None when it went straight into the flat gradient buffer."""
-    direct = direct_grad_target(bias)
+    direct = direct_grad_target(bias, ctx)
     gb = ck.bias_grad(gy, n_out, into=direct)
     if direct is None:
         return gb
@@ -289,7 +289,7 @@ class _ConvSameFn(torch.autograd.Function):
                     gxs[i] = o
         gw = gb = None
         if ctx.needs_input_grad[0]:
-            direct = direct_grad_target(ctx.wparam) if list(src_c) == list(real_c) else None
+            direct = direct_grad_target(ctx.wparam, ctx) if list(src_c) == list(real_c) else None
             if direct is not None:
                 # the ordered split-K reduce adds straight into the parameter's slice of the flat gradient buffer
                 ck.conv_wgrad(gy, list(xs), ks, direct, accumulate=True, x_off=ctx.in_off, tap_swap=ctx.tap_swap)
@@ -308,7 +308,7 @@ class _ConvSameFn(torch.autograd.Function):
                     o += sc
                 gw = torch.cat(parts, 1).contiguous()
         if ctx.has_bias and ctx.needs_input_grad[1]:
-            gb = _bias_grad(gy, weight.shape[0], ctx.bparam)
+            gb = _bias_grad(ctx, gy, weight.shape[0], ctx.bparam)
         return (gw, gb, None, None, None, *gxs)
 
 
@@ -338,7 +338,7 @@ class _StemFn(torch.autograd.Function):
         gy = gy.contiguous()
         gw = gb = None
         if ctx.needs_input_grad[0]:
-            direct = direct_grad_target(ctx.wparam)
+            direct = direct_grad_target(ctx.wparam, ctx)
             if direct is not None:
                 ck.conv_wgrad(gy, [xs], 3, direct, accumulate=True, stem=True)
                 notify_grad_written(ctx.wparam)
@@ -346,7 +346,7 @@ class _StemFn(torch.autograd.Function):
                 gw = torch.empty(weight.shape, dtype=torch.float32, device=weight.device)
                 ck.conv_wgrad(gy, [xs], 3, gw, stem=True)
         if ctx.bparam is not None and ctx.needs_input_grad[1]:
-            gb = _bias_grad(gy, weight.shape[0], ctx.bparam)
+            gb = _bias_grad(ctx, gy, weight.shape[0], ctx.bparam)
         return gw, gb, None, None
 
 
@@ -394,7 +394,7 @@ class _ConvHaloFn(torch.autograd.Function):
                     gxs[i] = o
         gw = None
         if ctx.needs_input_grad[0]:
-            direct = direct_grad_target(ctx.wparam)
+            direct = direct_grad_target(ctx.wparam, ctx)
             if direct is not None:
                 ck.conv_wgrad(gy, list(xs), 3, direct, accumulate=True, x_halo=ctx.halo_saved, tap_swap=ctx.tap_swap)
                 notify_grad_written(ctx.wparam)
@@ -529,7 +529,7 @@ class _ConvTFn(torch.autograd.Function):
             wd = mod._cache.get(weight, "both", lambda w: ck.pack_convT(w, True, True))[1]
             gx = ck.convT_dgrad(gy, wd, x.shape[4])
         if ctx.needs_input_grad[0]:
-            direct = direct_grad_target(ctx.wparam)
+            direct = direct_grad_target(ctx.wparam, ctx)
             if direct is not None:
                 ck.conv_wgrad(gy, [x], 2, direct, accumulate=True)
                 notify_grad_written(ctx.wparam)
@@ -537,7 +537,7 @@ class _ConvTFn(torch.autograd.Function):
                 gw = torch.empty(weight.shape, dtype=torch.float32, device=weight.device)  # contiguous whatever the parameter layout
                 ck.conv_wgrad(gy, [x], 2, gw)
         if ctx.has_bias and ctx.needs_input_grad[1]:
-            gb = _bias_grad(gy, gy.shape[4], ctx.bparam)
+            gb = _bias_grad(ctx, gy, gy.shape[4], ctx.bparam)
         return gw, gb, None, gx
 
 

@@ -48,7 +48,7 @@ class _GnFn(torch.autograd.Function):
         if spatial is None:
             into = None
             if ctx.needs_input_grad[1] and ctx.needs_input_grad[2]:
-                into = tuple(direct_grad_target(p) for p in ctx.params)
+                into = tuple(direct_grad_target(p, ctx) for p in ctx.params)
                 if any(t is None for t in into):
                     into = None
             dx, dw, db = gk.gn_backward(gy, x, w32, b32, mean, rstd, groups, eps, relu, into=into)

@@ -87,20 +87,34 @@ def weights_epoch(w=None):
 
 
 # Parameters whose ``.grad`` is a view into a flat gradient buffer (set up by the fused optimizer) are marked
-# with this attribute; the convolution backward passes then add their weight gradient straight into that view
-# (no temporary tensor, no autograd accumulation kernel) and tell the listeners below that it is there.
+# with this attribute; the convolution and GroupNorm backward passes then add their parameters' gradients straight into
+# those views (no temporary tensor, no autograd accumulation kernel) and tell the listeners below that they are there.
 FLAT_GRAD_ATTR = "_sb_flat_grad"
 _grad_written_listeners = []
 
 
-def direct_grad_target(param):
-    """The flat-buffer gradient view of ``param`` when the kernels may accumulate into it directly, else None."""
+def _autograd_accumulates(ctx, param) -> bool:
+    """Whether the running backward pass adds a gradient to ``param.grad`` that ``ctx``'s node returns for it: not when
+    the caller asked for other tensors' gradients (``backward(inputs=...)``), nor when for this one's as a result
+    (``autograd.grad``)."""
+    for node, _ in ctx.next_functions:
+        if getattr(node, "variable", None) is param:
+            try:
+                return torch._C._will_engine_execute_node(node)
+            except RuntimeError:  # the parameter is one of autograd.grad()'s inputs
+                return False
+    return False
+
+
+def direct_grad_target(param, ctx):
+    """The flat-buffer gradient view of ``param`` when the kernels may accumulate into it directly, else None. ``ctx`` is
+    the autograd node in whose backward pass this is asked."""
     if not getattr(param, FLAT_GRAD_ATTR, False) or param._backward_hooks:
         return None  # a hook on the parameter wants to see its gradient: autograd's own accumulation
     g = param.grad
     if g is None or g.dtype != torch.float32 or not g.is_contiguous() or g.shape != param.shape:
         return None
-    return g
+    return g if _autograd_accumulates(ctx, param) else None
 
 
 def add_grad_written_listener(fn) -> None:

@@ -27,17 +27,36 @@ def test_direct_gradients_accumulate_like_autograd(n, edge):
     flat = copy.deepcopy(plain)
     FusedClipAdam(flat.parameters()).attach()
     x = torch.randn((n, 32, *edge), device="cuda").to(torch.bfloat16).to(memory_format=torch.channels_last_3d)
-    seen = []
+    seen, added = [], []
     handle = flat[2].weight.register_hook(lambda g: seen.append(g.clone()))
+    for p in (flat[2].bias, flat[3].bias, flat[1].weight):
+        p.register_post_accumulate_grad_hook(lambda p: added.append(p))
     for k in range(2):  # the second pass adds to the first: twice the gradient, exactly
         for net in (plain, flat):
             _run(net, x).float().square().mean().backward()
         if k == 0:
             handle.remove()
+    assert len(added) == 6  # a post-accumulate hook runs after a direct write as well
     assert len(seen) == 1 and seen[0].shape == flat[2].weight.shape  # a hooked parameter keeps autograd's path
     for (name, p), q in zip(plain.named_parameters(), flat.parameters()):
         # the same kernels in the same order; only the reduction that adds into an existing value may round once more
         torch.testing.assert_close(q.grad, p.grad, rtol=2 ** -22, atol=0, msg=name)
+
+
+@pytest.mark.parametrize("name", ["0.weight", "0.bias", "1.weight", "2.weight", "2.bias", "3.weight", "3.bias"])
+def test_gradients_asked_for_by_name_are_returned(name):
+    """autograd.grad() of a flat optimizer's parameter, and backward(inputs=...) without it, leave its .grad alone."""
+    from scaffold_b200.ops.optim import FusedClipAdam
+    plain = _net(0)
+    flat = copy.deepcopy(plain)
+    FusedClipAdam(flat.parameters()).attach()
+    x = torch.randn((2, 32, 4, 6, 8), device="cuda").to(torch.bfloat16).to(memory_format=torch.channels_last_3d)
+    loss = lambda net, t: _run(net, t).float().square().mean()  # noqa: E731
+    want, got = (torch.autograd.grad(loss(net, x), [dict(net.named_parameters())[name]])[0] for net in (plain, flat))
+    assert torch.equal(got, want)
+    x.requires_grad_()
+    loss(flat, x).backward(inputs=[x])
+    assert x.grad.any() and all(not p.grad.any() for p in flat.parameters())
 
 
 def test_a_step_renews_its_own_operand_copies_only():
