@@ -187,10 +187,15 @@ class _Pass:
             stream.wait_stream(self.stream)
             self.stream = stream
         c3.refresh_packs(engine.flat)
-        self._load(images, masks)
-        self.forward_graph.replay()
+        # the regions of the ordinary pass; the loss is part of the graph, so its host time counts as the prediction's
+        with perf.region("image_to_device"):
+            self._load(images, masks)
+        with perf.region("predict"):
+            self.forward_graph.replay()
+        with perf.region("calculate_loss"):
+            out = tuple(t.clone() for t in self.out)
         _lib.lib().sb_count_launch(self.launches)
-        return tuple(t.clone() for t in self.out)
+        return out
 
     def backward(self):
         self.backward_graph.replay()

@@ -339,3 +339,20 @@ def test_validation_inside_and_outside_of_inference_mode():
             for e in (a, b):
                 e.step(*batch)
     assert len(_captured(a)) == 1
+
+
+def test_replayed_passes_count_in_the_region_totals():
+    from scaffold_b200.utils import perf
+    totals = []
+    for graphs in (True, False):
+        eng = _engine(graphs)
+        before = {k: v["count"] for k, v in perf.region_totals().items()}
+        for i in range(6):
+            eng.step(*_batch(i))
+            eng.eval_step(*_batch(i))
+        assert len(_captured(eng)) == 2 * graphs
+        totals.append({k: v["count"] - before.get(k, 0) for k, v in perf.region_totals().items()})
+    # a capture runs the pass's Python once more
+    for name, extra in (("image_to_device", 0), ("predict", 2), ("calculate_loss", 2), ("backward", 0),
+                        ("step_and_update", 0)):
+        assert totals[0][name] == totals[1][name] + extra, name
