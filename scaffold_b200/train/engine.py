@@ -85,6 +85,15 @@ class TrainEngine:
                                                              self.spatial)
             return loss, ce, fg, logits
 
+    def _with_room(self, fn):
+        """``fn()``, and once more when it ran out of memory that the captured passes keep."""
+        try:
+            return fn()
+        except torch.OutOfMemoryError:
+            if not self._graphs.release():
+                raise
+        return fn()
+
     # -- the step ------------------------------------------------------------------
     def step(self, images: torch.Tensor, masks: torch.Tensor, loss_host: Optional[torch.Tensor] = None) -> torch.Tensor:
         """One optimizer step; returns the loss as a device scalar.
@@ -95,10 +104,10 @@ class TrainEngine:
         """
         graph = self._graphs.get(self, images, masks, train=True)
         if graph is None:
-            images, masks = self.to_device(images, masks)
+            images, masks = self._with_room(lambda: self.to_device(images, masks))
         self.optimizer.zero_grad(set_to_none=self.flat is None)
         if graph is None:
-            loss, ce, fg, _ = self.forward_loss(images, masks)
+            loss, ce, fg, _ = self._with_room(lambda: self.forward_loss(images, masks))
         else:
             loss, ce, fg = graph.forward(self, images, masks)
         if loss_host is not None and self.cuda:
@@ -112,7 +121,19 @@ class TrainEngine:
             self._loss_host = loss_host
         with region("backward"):
             if graph is None:
-                loss.backward()
+                try:
+                    loss.backward()
+                    again = False
+                except torch.OutOfMemoryError:
+                    again = self._graphs.release()
+                    if not again:
+                        raise
+                if again:  # half of the gradients are there: from the start, with the captured passes' memory
+                    ce, fg = ce.detach(), fg.detach()
+                    self.optimizer.zero_grad(set_to_none=self.flat is None)
+                    loss = None
+                    loss = self.forward_loss(images, masks)[0]
+                    loss.backward()
             else:
                 graph.backward()
         with region("step_and_update"):
@@ -140,7 +161,7 @@ class TrainEngine:
         graph = self._graphs.get(self, images, masks, train=False)
         if graph is not None:
             return graph.forward(self, images, masks)
-        return self._eval_pass(*self.to_device(images, masks))
+        return self._with_room(lambda: self._eval_pass(*self.to_device(images, masks)))
 
     def _eval_pass(self, images: torch.Tensor, masks: torch.Tensor):
         loss, ce, fg, logits = self.forward_loss(images, masks)

@@ -13,7 +13,8 @@ the results out of them, so inputs may live anywhere and results are the caller'
 
 Limits: batches whose widest feature map is at most ``MAX_MAP_BYTES`` (2 x 128 cubed x 64 channels), since the graph
 keeps the memory of one pass's activations and larger batches gain less than 1 %; at most ``MAX_SHAPES`` batch shapes
-per engine. The memory is given back with the engine.
+per engine, and ``1 / MEMORY_SHARE`` of the device's memory. The memory is given back with the engine, when a pass is
+found out of date, and when an ordinary pass of the engine runs out of memory.
 """
 from __future__ import annotations
 
@@ -38,6 +39,7 @@ from ..utils import perf
 WARM_PASSES = 2        # ordinary passes over a shape before its capture (kernels set up, operand layouts known)
 MAX_SHAPES = 4         # graphs per engine and kind of pass
 MAX_MAP_BYTES = 640 << 20
+MEMORY_SHARE = 8       # an engine's graphs together keep at most 1 / this of the device's memory
 
 
 def _watched() -> bool:
@@ -175,6 +177,9 @@ class _Pass:
                 c._fresh &= fresh  # packing that was recorded has not run
         self.out = out
         self.stream = torch.cuda.current_stream()
+        # what the graphs keep: their pool, the buffers of the batch
+        self.bytes = sum(s["total_size"] for s in torch.cuda.memory_snapshot() if tuple(s["segment_pool_id"]) == tuple(pool))
+        self.bytes += sum(t.numel() * t.element_size() for t in (self.images, self.masks))
 
     @torch.no_grad()
     def _load(self, images, masks):
@@ -238,8 +243,9 @@ class StepGraphs:
         if isinstance(seen, _Pass):
             if seen.fingerprint.holds(engine):
                 return seen
-            seen = 0  # the model was changed: start over
-            self._passes[key] = seen
+            # the model was changed: start over, and keep no memory for the other shapes' passes either
+            self._passes = {k: 0 if k[0] == train and isinstance(p, _Pass) else p for k, p in self._passes.items()}
+            seen = 0
         if seen is None:
             return None
         if seen < WARM_PASSES:
@@ -251,18 +257,33 @@ class StepGraphs:
         if not owned:  # a parameter outside the optimizer: nothing would renew its operand copies
             self._passes[key] = None
             return None
-        if sum(isinstance(p, _Pass) and k[0] == train for k, p in self._passes.items()) >= MAX_SHAPES:
+        kept = {k: p for k, p in self._passes.items() if isinstance(p, _Pass)}
+        room = torch.cuda.get_device_properties(engine.device).total_memory // MEMORY_SHARE
+        room -= sum(p.bytes for p in kept.values())
+        if sum(k[0] == train for k in kept) >= MAX_SHAPES or room <= 0:
             return None
         probe = _Fingerprint(engine)
         if not probe.holds(engine):  # hooks are set, or a module is not one of the model's own: look again later
             self._passes[key] = 0
             return None
         try:
-            self._passes[key] = _Pass(engine, images, masks, train)
+            new = _Pass(engine, images, masks, train)
+            if new.bytes > room:
+                raise RuntimeError(f"its {new.bytes >> 20} MB are over the limit")
+            self._passes[key] = new
         except RuntimeError as exc:  # no memory for the graph's buffers, or an operation that cannot be captured
             import logging
             logging.getLogger("scaffold").warning("the %s pass stays uncaptured: %s", "training" if train else
                                                   "validation", str(exc).splitlines()[0])
-            self._passes[key] = None
+            self._passes[key] = new = None
             torch.cuda.synchronize()
         return self._passes[key]
+
+    def release(self) -> bool:
+        """Give the memory of all captured passes back; False when there was none."""
+        held = any(isinstance(p, _Pass) for p in self._passes.values())
+        self._passes = {k: None if isinstance(p, _Pass) else p for k, p in self._passes.items()}
+        if held:
+            torch.cuda.synchronize()
+            torch.cuda.empty_cache()
+        return held

@@ -356,3 +356,56 @@ def test_replayed_passes_count_in_the_region_totals():
     for name, extra in (("image_to_device", 0), ("predict", 2), ("calculate_loss", 2), ("backward", 0),
                         ("step_and_update", 0)):
         assert totals[0][name] == totals[1][name] + extra, name
+
+
+def test_captured_passes_keep_a_bounded_share_of_the_memory(monkeypatch):
+    from scaffold_b200.train import step_graph as sg
+    a, b = _engine(True), _engine(False)
+    for i in range(4):
+        a.step(*_batch(i)), b.step(*_batch(i))
+    (key,) = _captured(a)
+    kept = a._graphs._passes[key].bytes
+    x, _ = _batch(0)
+    maps = x.shape[0] * 32 * x[0, 0].numel() * 2    # the widest map is one of many that backward needs
+    assert 8 * maps < kept < 1 << 30
+    total = torch.cuda.get_device_properties(0).total_memory
+    monkeypatch.setattr(sg, "MEMORY_SHARE", total // (kept + (1 << 20)))   # room for this one, not for two
+    for i in range(5):
+        assert torch.equal(a.step(*_batch(i, n=4)), b.step(*_batch(i, n=4)))
+    assert _captured(a) == [key]
+    assert torch.equal(a.step(*_batch(9)), b.step(*_batch(9))) and torch.equal(a.flat.data, b.flat.data)
+
+
+@pytest.mark.parametrize("where", ["forward", "backward", "validation"])
+def test_an_ordinary_pass_that_runs_out_of_memory_gets_that_of_the_captured_ones(where):
+    """The allocator's error is made on the host, once, in an ordinary pass of another shape."""
+    a, b = _engine(True), _engine(False)
+    for i in range(4):
+        a.step(*_batch(i)), b.step(*_batch(i))
+    assert _captured(a)
+    failures = []
+
+    def fail_once(*args):
+        if not failures:
+            failures.append(1)
+            raise torch.OutOfMemoryError("out of memory")
+
+    if where == "backward":
+        handle = a.model.down_list[0].double_conv[1].weight.register_hook(fail_once)   # near the end of backward
+        assert torch.equal(a.step(*_batch(9, n=1)), b.step(*_batch(9, n=1)))
+        handle.remove()
+    else:
+        handle = a.model.up_list[0].register_forward_hook(fail_once)
+        if where == "forward":
+            assert torch.equal(a.step(*_batch(9, n=1)), b.step(*_batch(9, n=1)))
+        else:
+            for s, t in zip(a.eval_step(*_batch(9, n=1)), b.eval_step(*_batch(9, n=1))):
+                assert torch.equal(s, t)
+        handle.remove()
+    assert failures and not _captured(a)
+    assert torch.equal(a.flat.grad, b.flat.grad) and torch.equal(a.flat.data, b.flat.data)
+    failures.clear()
+    handle = a.model.up_list[0].register_forward_hook(fail_once)
+    with pytest.raises(torch.OutOfMemoryError):   # nothing left to give back
+        a.step(*_batch(9, n=1))
+    handle.remove()
