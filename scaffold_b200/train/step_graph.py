@@ -191,6 +191,8 @@ class _Pass:
         if stream != self.stream:  # the buffers are the graph's: a pass on another stream comes after the last one
             stream.wait_stream(self.stream)
             self.stream = stream
+            self.images.record_stream(stream)  # made on another one, and dropped whenever the pass is
+            self.masks.record_stream(stream)
         c3.refresh_packs(engine.flat)
         # the regions of the ordinary pass; the loss is part of the graph, so its host time counts as the prediction's
         with perf.region("image_to_device"):

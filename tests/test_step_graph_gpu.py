@@ -409,3 +409,26 @@ def test_an_ordinary_pass_that_runs_out_of_memory_gets_that_of_the_captured_ones
     with pytest.raises(torch.OutOfMemoryError):   # nothing left to give back
         a.step(*_batch(9, n=1))
     handle.remove()
+
+
+def test_a_pass_dropped_while_another_stream_replays_it_keeps_its_buffers():
+    a, b = _engine(True), _engine(False)
+    batch = _batch(1, edge=(32, 32, 32))
+    for e in (a, b):
+        for _ in range(4):
+            want = e.eval_step(*batch)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    static = a._graphs._passes[_captured(a)[0]].images
+    size = static.numel()
+    with torch.cuda.stream(side):
+        for _ in range(20):
+            got = a.eval_step(*batch)
+    address = static.data_ptr()
+    del static
+    a._graphs.__init__()            # dropped with replays pending
+    reused = torch.full((size,), 1e9, device="cuda")   # the default stream's next allocation of that size
+    assert reused.data_ptr() != address or side.query()
+    side.synchronize()
+    for s, t in zip(got, want):
+        assert torch.equal(s, t)
