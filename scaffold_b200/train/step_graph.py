@@ -19,6 +19,7 @@ found out of date, and when an ordinary pass of the engine runs out of memory.
 from __future__ import annotations
 
 import math
+import threading
 import weakref
 from operator import eq, is_
 from types import FunctionType
@@ -39,6 +40,7 @@ from ..utils import perf
 WARM_PASSES = 2        # ordinary passes over a shape before its capture (kernels set up, operand layouts known)
 MAX_SHAPES = 4         # graphs per engine and kind of pass
 MAX_MAP_BYTES = 640 << 20
+_CAPTURES = threading.Lock()  # torch captures on one stream of the process
 MEMORY_SHARE = 8       # an engine's graphs together keep at most 1 / this of the device's memory
 
 
@@ -126,6 +128,7 @@ class _Pass:
 
     def __init__(self, engine, images, masks, train: bool):
         dev = engine.device
+        self._lock = threading.Lock()
         self.images = torch.empty(images.shape, dtype=images.dtype, device=dev)
         self.masks = torch.empty(masks.shape, dtype=masks.dtype, device=dev)
         self._load(images, masks)
@@ -187,6 +190,10 @@ class _Pass:
         self.masks.copy_(masks, non_blocking=True)
 
     def forward(self, engine, images, masks):
+        with self._lock:  # one set of buffers: threads take turns, each on its own stream behind the last one's
+            return self._forward(engine, images, masks)
+
+    def _forward(self, engine, images, masks):
         stream = torch.cuda.current_stream()
         if stream != self.stream:  # the buffers are the graph's: a pass on another stream comes after the last one
             stream.wait_stream(self.stream)
@@ -215,6 +222,7 @@ class StepGraphs:
     def __init__(self):
         self._passes = {}   # key -> _Pass, or the number of ordinary passes seen, or None (cannot be captured)
         self._model = None  # weak reference to the model that these passes are of
+        self._lock = threading.Lock()
 
     @staticmethod
     def _usable(engine, images, masks) -> bool:
@@ -231,6 +239,10 @@ class StepGraphs:
 
     def get(self, engine, images, masks, train: bool) -> Optional[_Pass]:
         """The captured pass for this batch's shape, or None: run the ordinary pass."""
+        with self._lock:
+            return self._get(engine, images, masks, train)
+
+    def _get(self, engine, images, masks, train):
         if self._model is None or self._model() is not engine.model:  # the engine has another model now
             self._passes = {}
             self._model = weakref.ref(engine.model)
@@ -269,7 +281,8 @@ class StepGraphs:
             self._passes[key] = 0
             return None
         try:
-            new = _Pass(engine, images, masks, train)
+            with _CAPTURES:
+                new = _Pass(engine, images, masks, train)
             if new.bytes > room:
                 raise RuntimeError(f"its {new.bytes >> 20} MB are over the limit")
             self._passes[key] = new
@@ -283,8 +296,9 @@ class StepGraphs:
 
     def release(self) -> bool:
         """Give the memory of all captured passes back; False when there was none."""
-        held = any(isinstance(p, _Pass) for p in self._passes.values())
-        self._passes = {k: None if isinstance(p, _Pass) else p for k, p in self._passes.items()}
+        with self._lock:
+            held = any(isinstance(p, _Pass) for p in self._passes.values())
+            self._passes = {k: None if isinstance(p, _Pass) else p for k, p in self._passes.items()}
         if held:
             torch.cuda.synchronize()
             torch.cuda.empty_cache()

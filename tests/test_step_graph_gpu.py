@@ -432,3 +432,26 @@ def test_a_pass_dropped_while_another_stream_replays_it_keeps_its_buffers():
     side.synchronize()
     for s, t in zip(got, want):
         assert torch.equal(s, t)
+
+
+def test_threads_validate_their_own_batches():
+    from concurrent.futures import ThreadPoolExecutor
+    a, b = _engine(True), _engine(False)
+    batches = [_batch(i) for i in range(4)]
+    for _ in range(4):
+        a.eval_step(*batches[0])
+    assert _captured(a)
+    want = [b.eval_step(*x) for x in batches]
+    torch.cuda.synchronize()
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            out = [a.eval_step(*batches[i]) for _ in range(40)]
+            torch.cuda.current_stream().synchronize()
+        return out
+    with ThreadPoolExecutor(4) as pool:
+        got = list(pool.map(work, range(4)))
+    for i in range(4):
+        for out in got[i]:
+            for s, t in zip(out, want[i]):
+                assert torch.equal(s, t)
