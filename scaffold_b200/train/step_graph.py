@@ -224,6 +224,9 @@ class StepGraphs:
         self._model = None  # weak reference to the model that these passes are of
         self._lock = threading.Lock()
 
+    def __reduce__(self):  # a copy of the engine has captured nothing yet
+        return StepGraphs, ()
+
     @staticmethod
     def _usable(engine, images, masks) -> bool:
         model = engine.model

@@ -455,3 +455,13 @@ def test_threads_validate_their_own_batches():
         for out in got[i]:
             for s, t in zip(out, want[i]):
                 assert torch.equal(s, t)
+
+
+def test_a_copied_engine_starts_without_captured_passes():
+    import copy
+    a = _engine(True)
+    for i in range(4):
+        a.eval_step(*_batch(i))
+    assert _captured(a)
+    c = copy.deepcopy(a._graphs)
+    assert c is not a._graphs and not c._passes and _captured(a)
