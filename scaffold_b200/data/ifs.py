@@ -89,11 +89,15 @@ def _to_host(t: torch.Tensor) -> np.ndarray:
     while step < largest and 8 * step <= size:
         step *= 2
     step //= t.element_size()
+    try:
+        ring = [torch.empty(step, dtype=t.dtype, pin_memory=True)
+                for _ in range(min(_STAGE_BUFFERS, -(-t.numel() // step)))]
+    except RuntimeError:  # no more page-locked memory on this host
+        return t.cpu().numpy()
     src = t.contiguous().view(-1)
     out = np.empty(tuple(t.shape), dtype=torch.empty(0, dtype=t.dtype).numpy().dtype)
     dst = torch.from_numpy(out).view(-1)
     spans = [(a, min(a + step, src.numel())) for a in range(0, src.numel(), step)]
-    ring = [torch.empty(step, dtype=t.dtype, pin_memory=True) for _ in range(min(_STAGE_BUFFERS, len(spans)))]
     done = [torch.cuda.Event() for _ in ring]
     with torch.cuda.device(t.device):
         for i in range(len(spans) + len(ring) - 1):

@@ -61,3 +61,19 @@ def test_staged_copy_to_host_is_the_tensor(chunks, monkeypatch):
         n = max(1, int(chunks * 4096 / torch.empty(0, dtype=dtype).element_size()) // 2)
         t = (torch.arange(3 * n, device="cuda") % 30011).to(dtype).view(n, 3)[:, 1:]  # not contiguous
         np.testing.assert_array_equal(ifs._to_host(t), t.cpu().numpy())
+
+
+def test_results_reach_the_host_without_page_locked_memory(monkeypatch):
+    import torch
+
+    from scaffold_b200.data import ifs
+    make = torch.empty
+
+    def refusing(*args, **kwargs):
+        if kwargs.get("pin_memory"):
+            raise RuntimeError("out of page-locked memory")
+        return make(*args, **kwargs)
+    t = torch.arange(1 << 20, device="cuda")
+    want = t.cpu().numpy()
+    monkeypatch.setattr(torch, "empty", refusing)
+    np.testing.assert_array_equal(ifs._to_host(t), want)
