@@ -586,18 +586,23 @@ static int finish_and_launch(IgemmParams& p, int cout_rows, cudaStream_t stream)
   if (p.splits < 1) p.splits = 1;
   p.k_per_split = cdiv(kiters, p.splits);
   if (p.splits > 1) p.ocols = 0;
-  p.bias_n = p.ocols > 0 && p.bias ? (p.scatter ? p.sc_cout : p.width0) : 0;
-  // dynamic shared memory behind the stages: staging buffers (8 of 32 rows), bias
-  const int extra = 8 * 64 * p.ocols + (p.bias_n ? ((cout_rows * 4 + 127) / 128) * 128 : 0);
   // Two CTAs per SM when there are tiles for them and three stages fit in half the shared memory (two where the
   // staging buffers take their share and the whole reduction is at most two steps): the second CTA's MMAs and epilogue
   // fill the first one's waits (each CTA allocates 256 of the 512 TMEM columns).
   const int half = g_smem_limit / 2 - 2048;
-  const int need = p.ocols > 0 && kiters <= 2 ? 2 : 3;
-  const bool dual = p.num_tiles * p.splits > g_sm_count && (half - 1024 - extra) / p.stage_bytes >= need;
-  int st = ((dual ? half : g_smem_limit) - 1024 - extra) / p.stage_bytes;
+  int extra = 0, st = 0;
+  bool dual = false;
+  for (;; p.ocols = 0) {
+    // behind the stages: staging buffers (8 of 32 rows), and the bias as far as columns read it
+    p.bias_n = p.ocols > 0 && p.bias ? (p.scatter ? p.sc_cout : p.width0) : 0;
+    extra = 8 * 64 * p.ocols + (p.bias_n ? (((p.scatter ? p.sc_cout : cout_rows) * 4 + 127) / 128) * 128 : 0);
+    const int need = p.ocols > 0 && kiters <= 2 ? 2 : 3;
+    dual = p.num_tiles * p.splits > g_sm_count && (half - 1024 - extra) / p.stage_bytes >= need;
+    st = ((dual ? half : g_smem_limit) - 1024 - extra) / p.stage_bytes;
+    if (st >= 2) break;
+    if (p.ocols == 0) return SB_ERR_SHAPE;  // with a bias too wide to stage: stores from registers
+  }
   if (st > MAX_STAGES) st = MAX_STAGES;
-  if (st < 2) return SB_ERR_SHAPE;
   p.stages = st;
   p.stg_off = st * p.stage_bytes;
   p.bias_off = p.stg_off + 8 * 64 * p.ocols;
@@ -682,8 +687,9 @@ extern "C" int sb_conv_gn_splits(const SbConvArgs* a) {
   return conv_plane3_gn_splits(a);
 }
 
-// force_plain: 0 = automatic (k = 1 from 16 or 32 channels; 8 x 8 plane kernel; the two-SM pair kernel for wide outputs given tap-ordered
-// weights only; kd-fused or plane-walk kernel when the shape is eligible; else this file's generic kernel),
+// force_plain: 0 = automatic (k = 1 from 16 or 32 channels; 8 x 8 plane kernel; the two-SM pair kernel for wide outputs
+// given tap-ordered weights only; kd-fused or plane-walk kernel when the shape is eligible; else this file's generic
+// kernel),
 // 1 = generic kernel one tap per load, 2 = generic kernel with the w-shift reuse, 3 = generic kernel with the
 // (h, w)-shift reuse, 4 = automatic without the pair kernel.
 extern "C" int sb_conv_fwd(const SbConvArgs* a, cudaStream_t stream) {
@@ -842,7 +848,8 @@ extern "C" int sb_convT_fwd(const SbConvTArgs* a, cudaStream_t stream) {
   p.inv_cout = (uint32_t)(0xffffffffu / (uint32_t)a->cout + 1u);
   p.inv_2cout = (uint32_t)(0xffffffffu / (2u * (uint32_t)a->cout) + 1u);
   p.status = a->status;
-  p.ocols = a->dst_ld == a->cout && (reinterpret_cast<uintptr_t>(a->dst) & 15) == 0
+  // (inv_2cout divides exactly while column * 2 cout < 2^32)
+  p.ocols = a->dst_ld == a->cout && (reinterpret_cast<uintptr_t>(a->dst) & 15) == 0 && a->cout < 16384
                 ? store_columns(p.BN, 2 * a->cout) : 0;
   for (int o = 0; p.ocols > 0 && o < 4; ++o) {
     const long long C = a->cout, W2 = 2LL * a->W, H2 = 2LL * a->H, D2 = 2LL * a->D;

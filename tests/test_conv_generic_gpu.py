@@ -48,7 +48,8 @@ def test_pointwise(dims, cin, cout, with_bias):
 
 @pytest.mark.parametrize("dims,cin,cout", [
     ((1, 1, 1, 1), 32, 16), ((1, 3, 5, 7), 64, 32), ((2, 5, 3, 9), 96, 48), ((1, 2, 9, 17), 128, 64),
-    ((2, 3, 4, 33), 32, 16), ((1, 2, 3, 5), 16, 8), ((1, 2, 2, 150), 256, 128)])
+    ((2, 3, 4, 33), 32, 16), ((1, 2, 3, 5), 16, 8), ((1, 2, 2, 150), 256, 128), ((1, 1, 2, 3), 16, 6144),
+    ((1, 1, 2, 3), 16, 20000)])
 @pytest.mark.parametrize("with_bias", [False, True])
 def test_transposed(dims, cin, cout, with_bias):
     from scaffold_b200.ops import _lib, conv_kernels as ck
