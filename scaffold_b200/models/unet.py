@@ -65,9 +65,9 @@ class DoubleConv(nn.Module):
 
 
 def _observed(m: nn.Module) -> bool:
-    """True when someone would notice that ``m`` is not called: a hook, or a forward of its own."""
+    """True when someone would notice that ``m`` is not called: a hook, or a forward or a compiled call of its own."""
     return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
-                or "forward" in m.__dict__)
+                or "forward" in m.__dict__ or m._compiled_call_impl is not None)
 
 
 class Down(nn.Module):
@@ -119,6 +119,14 @@ class Up(nn.Module):
         dev = x2.device.type
         dtype = torch.get_autocast_dtype(dev) if dev in ("cpu", "cuda") and torch.is_autocast_enabled(dev) else x2.dtype
         return self.conv(torch.cat([x2.to(dtype), x1.to(dtype)], dim=1))
+
+
+    def reads_skip_only(self) -> bool:
+        """True when nothing but the block's first convolution sees the skip tensor (a hook may change it in place, or
+        wait for its whole gradient)."""
+        seq = self.conv.double_conv if type(self) is Up and type(self.conv) is DoubleConv else None
+        return (type(seq) is _FirstConvSequential and type(seq[0]) is Conv3d
+                and not any(_observed(m) for m in (self, self.conv, seq, seq[0])))
 
 
 class OutConv(nn.Module):
@@ -188,9 +196,10 @@ class UNet(nn.Module):
         if x.is_cuda and not x.is_contiguous():
             x = x.contiguous()  # the input staging kernel reads a dense NCDHW tensor
         skips = [self._run(self.down_list[0], x)]
+        plain = not self.checkpointing and type(self)._run is UNet._run and "_run" not in self.__dict__
         for i in range(1, self.layers + 1):
-            block = self.down_list[i]
-            if self.checkpointing or not isinstance(block, Down):
+            block, reader = self.down_list[i], self.up_list[self.layers - i]
+            if not (plain and isinstance(block, Down) and isinstance(reader, Up) and reader.reads_skip_only()):
                 skips.append(self._run(block, skips[-1]))
             else:
                 out, skips[-1] = block.forward_with_skip(skips[-1])

@@ -49,3 +49,46 @@ def test_a_hook_on_a_passed_by_module_keeps_its_call(dims, where):
     assert seen
     for a, b in zip(fused, separate):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("where", ["block", "double", "sequence", "convolution"])
+def test_a_hook_that_changes_the_skip_tensor_may_do_so(where):
+    """In place, as on any module's input; and the gradient that it waits for is the whole one."""
+    from scaffold_b200.models.unet import UNet
+    torch.manual_seed(0)
+    net = UNet(3, 4, layers=2, base_width=16).cuda()
+    x = torch.rand((1, 3, 16, 16, 32), device="cuda")
+    up = net.up_list[1]   # reads the first block's output
+    mod = {"block": up, "double": up.conv, "sequence": up.conv.double_conv, "convolution": up.conv.double_conv[0]}[where]
+    whole, inside = [], []
+
+    def outer(m, args, out):
+        out.register_hook(lambda g: whole.append(g.clone()))
+
+    def inner(m, args):
+        skip = args[1] if where == "block" else args[0][0]
+        skip.register_hook(lambda g: inside.append(g.clone()))
+        with torch.no_grad():
+            skip.mul_(0.5)
+        return None
+    handles = [net.down_list[0].register_forward_hook(outer), mod.register_forward_pre_hook(inner)]
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        net(x).float().square().mean().backward()
+    for h in handles:
+        h.remove()
+    assert len(whole) == len(inside) == 1 and torch.equal(whole[0], inside[0])
+
+
+def test_a_run_of_its_own_is_called_for_every_block():
+    from scaffold_b200.models.unet import UNet
+
+    class Counting(UNet):
+        calls = 0
+
+        def _run(self, block, *inputs):
+            self.calls += 1
+            return super()._run(block, *inputs)
+    net = Counting(3, 4, layers=2, base_width=16).cuda()
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        net(torch.rand((1, 3, 16, 16, 32), device="cuda")).sum().backward()
+    assert net.calls == 3 + 3   # three encoder blocks, two decoder blocks, the head
