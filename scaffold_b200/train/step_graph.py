@@ -284,7 +284,8 @@ class StepGraphs:
             self._passes[key] = 0
             return None
         try:
-            with _CAPTURES:
+            # (the caller's stream is current again whatever ends a capture)
+            with _CAPTURES, torch.cuda.stream(torch.cuda.current_stream()):
                 new = _Pass(engine, images, masks, train)
             if new.bytes > room:
                 raise RuntimeError(f"its {new.bytes >> 20} MB are over the limit")

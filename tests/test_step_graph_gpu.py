@@ -465,3 +465,22 @@ def test_a_copied_engine_starts_without_captured_passes():
     assert _captured(a)
     c = copy.deepcopy(a._graphs)
     assert c is not a._graphs and not c._passes and _captured(a)
+
+
+@pytest.mark.parametrize("train", [True, False])
+def test_a_pass_that_reads_a_value_on_the_host_stays_uncaptured(train, monkeypatch):
+    """The runtime refuses the synchronisation and ends the capture; the engine goes on with ordinary passes."""
+    a, b = _engine(True), _engine(False)
+    ordinary = type(a).forward_loss
+
+    def reading(self, *args):
+        out = ordinary(self, *args)
+        float(out[0].detach())
+        return out
+    monkeypatch.setattr(type(a), "forward_loss", reading)
+    stream = torch.cuda.current_stream()
+    for i in range(6):
+        batch = _batch(i)
+        got, want = (e.step(*batch) if train else e.eval_step(*batch)[0] for e in (a, b))
+        assert torch.equal(got, want) and torch.cuda.current_stream() == stream, i
+    assert not _captured(a) and torch.equal(a.flat.data, b.flat.data)
