@@ -78,7 +78,7 @@ __device__ __forceinline__ void adam_one(float& p, float g, float& m, float& v, 
 // the serial norm, 476 us now (5.3 TB/s over the step's 2.5 GB).
 __global__ void __launch_bounds__(OPT_THREADS) adam_kernel(float* __restrict__ p, const float* __restrict__ g,
                                                            float* __restrict__ m, float* __restrict__ v, long long n,
-                                                           float lr, float b1, float b2, float eps, float bc1,
+                                                           int vec, float lr, float b1, float b2, float eps, float bc1,
                                                            float bc2_sqrt, float max_norm,
                                                            const float* __restrict__ norm, float grad_scale) {
   float coef = grad_scale;
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(OPT_THREADS) adam_kernel(float* __restrict__ p
     coef *= c < 1.f ? c : 1.f;
   }
   const AdamCoef k{lr / bc1, b1, b2, eps, bc2_sqrt, coef};
-  const long long n4 = n / 4, stride = (long long)gridDim.x * OPT_THREADS;
+  const long long n4 = vec ? n / 4 : 0, stride = (long long)gridDim.x * OPT_THREADS;
   float4* p4 = reinterpret_cast<float4*>(p);
   const float4* g4 = reinterpret_cast<const float4*>(g);
   float4* m4 = reinterpret_cast<float4*>(m);
@@ -119,8 +119,8 @@ __global__ void __launch_bounds__(OPT_THREADS) adam_kernel(float* __restrict__ p
       }
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x < (int)(n - n4 * 4)) {
-    const long long j = n4 * 4 + threadIdx.x;
+  // what the vectors leave over: up to three elements, or all of them when a buffer does not start on 16 bytes
+  for (long long j = n4 * 4 + (long long)blockIdx.x * OPT_THREADS + threadIdx.x; j < n; j += stride) {
     float pj = p[j], mj = m[j], vj = v[j];
     adam_one(pj, g[j], mj, vj, k);
     p[j] = pj; m[j] = mj; v[j] = vj;
@@ -150,13 +150,12 @@ extern "C" int sb_grad_norm(const float* g, long long n, float* partials, float*
 extern "C" int sb_adam_step(float* p, const float* g, float* m, float* v, long long n, float lr, float b1, float b2,
                             float eps, int step, float max_norm, const float* norm, float grad_scale,
                             cudaStream_t stream) {
-  if (((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(m) |
-        reinterpret_cast<uintptr_t>(v)) & 15) != 0)
-    return SB_ERR_ALIGN;
+  const int vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(m) |
+                    reinterpret_cast<uintptr_t>(v)) & 15) == 0;
   const float bc1 = 1.f - powf(b1, (float)step);
   const float bc2_sqrt = sqrtf(1.f - powf(b2, (float)step));
   const int blocks = sb_opt_blocks(n);
-  adam_kernel<<<blocks, OPT_THREADS, 0, stream>>>(p, g, m, v, n, lr, b1, b2, eps, bc1, bc2_sqrt, max_norm, norm,
+  adam_kernel<<<blocks, OPT_THREADS, 0, stream>>>(p, g, m, v, n, vec, lr, b1, b2, eps, bc1, bc2_sqrt, max_norm, norm,
                                                   grad_scale);
   sb_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;

@@ -31,3 +31,26 @@ def test_adam_tail_and_norm(n):
     assert torch.equal(p[n:].double(), q[n:])  # nothing behind the end is touched
     assert ((p[:n].double() - q[:n]).abs() <= 2e-6 * q[:n].abs() + 1e-4 * (q[:n] - p[:n].double()).abs() + 5e-6
             * (1 + (mm[:n] / vv[:n] ** 0.5).abs())).all()
+
+
+@pytest.mark.parametrize("n", [1, 5, 70001])
+def test_adam_on_buffers_off_the_vectors_alignment(n):
+    """As on aligned ones, but for the multiply-adds that the compiler fuses in one loop and not in the other: each
+    moment has two of them and the parameter one more, of terms below 1 (2^-24 each); the step's quotient carries the
+    moments' relative errors, 4 roundings of 2^-24, times a step of at most 0.2."""
+    from scaffold_b200.ops import _lib
+    import scaffold_b200.ops.optim  # noqa: F401  (registers the entry points)
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    bufs = [torch.rand(n, generator=gen, device="cuda") for _ in range(4)]
+    lib, s = _lib.lib(), _lib.stream_ptr()
+    outs = []
+    for shift in (0, 1):
+        own = [torch.full((n + 2,), 7.0, device="cuda") for _ in bufs]
+        views = [o[shift:shift + n].copy_(b) for o, b in zip(own, bufs)]
+        p, g, m, v = (t.data_ptr() for t in views)
+        assert lib.sb_adam_step(p, g, m, v, n, 1e-2, 0.9, 0.999, 1e-8, 3, -1.0, None, 1.0, s) == 0
+        torch.cuda.synchronize()
+        assert all((o[:shift] == 7).all() and (o[shift + n:] == 7).all() for o in own)
+        outs.append([t.clone() for t in views])
+    for a, b in zip(*outs):
+        torch.testing.assert_close(a, b, rtol=0, atol=2 ** -21)
