@@ -108,19 +108,20 @@ __device__ __forceinline__ void stat_store(float* dst, const StatSums& a) {
   dst[1] = (float)mean;
   dst[2] = (float)(m2 < 0.0 ? 0.0 : m2);  // a NaN stays one: an overflow has to show in what follows
 }
-// The sums of partials first, first + step, ... of (n, g) (`base`: partial 0), eight partials in flight. Loads bypass
+// The sums of partials first, first + step, ... of (n, g) (`base`: partial 0), FLIGHT partials in flight. Loads bypass
 // L1 (the partials may have been written by other SMs during this launch).
+template <int FLIGHT>
 __device__ __forceinline__ StatSums stat_walk(const float* __restrict__ base, int G, int first, int step, int nsplit) {
   StatSums a{0.0, 0.0, 0.0};
-  for (int s = first; s < nsplit; s += 8 * step) {
-    float e[8][3];
+  for (int s = first; s < nsplit; s += FLIGHT * step) {
+    float e[FLIGHT][3];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
+    for (int u = 0; u < FLIGHT; ++u) {
       const float* q = base + (long long)(s + u * step) * G * 3;
       if (s + u * step < nsplit) { e[u][0] = __ldcg(q); e[u][1] = __ldcg(q + 1); e[u][2] = __ldcg(q + 2); }
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
+    for (int u = 0; u < FLIGHT; ++u)
       if (s + u * step < nsplit) stat_add(a, e[u][0], e[u][1], e[u][2]);
   }
   return a;
@@ -147,7 +148,9 @@ __device__ __forceinline__ void stats_collapse_warp(const float* __restrict__ pa
   StatSums t{0.0, 0.0, 0.0};
   const int strands = nsplit > 32 ? GN_FIN_WARPS : 1;
   for (int w = 0; w < strands; ++w) {
-    const StatSums a = stat_warp_sum(stat_walk(base, G, w * 32 + lane, strands * 32, nsplit));
+    // (five in flight: all of a lane's share of 592, and with eight the statistics kernel takes 80 registers instead of
+    // 64, so one block per SM less: 75 us more for ten launches at 3 x 35x32x28 voxels of 16 channels)
+    const StatSums a = stat_warp_sum(stat_walk<5>(base, G, w * 32 + lane, strands * 32, nsplit));
     t.n += a.n; t.s1 += a.s1; t.s2 += a.s2;
   }
   if (lane == 0) stat_store(fin + ((long long)n * G + g) * 3, t);
@@ -605,7 +608,7 @@ __global__ void __launch_bounds__(GN_FIN_THREADS) gn_stats_finalize_block_kernel
                                                                                  int nsplit) {
   __shared__ double s_w[GN_FIN_WARPS][3];
   const int n = blockIdx.x / G, g = blockIdx.x % G, warp = threadIdx.x >> 5;
-  const StatSums a = stat_warp_sum(stat_walk(part + ((long long)n * nsplit * G + g) * 3, G, threadIdx.x, GN_FIN_THREADS,
+  const StatSums a = stat_warp_sum(stat_walk<8>(part + ((long long)n * nsplit * G + g) * 3, G, threadIdx.x, GN_FIN_THREADS,
                                              nsplit));
   if ((threadIdx.x & 31) == 0) { s_w[warp][0] = a.n; s_w[warp][1] = a.s1; s_w[warp][2] = a.s2; }
   __syncthreads();
@@ -628,7 +631,7 @@ __global__ void __cluster_dims__(GN_WIDE_CLUSTER, 1, 1) __launch_bounds__(GN_THR
   __shared__ double s_cta[3];
   const int out = blockIdx.x / GN_WIDE_CLUSTER, rank = blockIdx.x % GN_WIDE_CLUSTER;
   const int n = out / G, g = out % G, warp = threadIdx.x >> 5;
-  const StatSums a = stat_warp_sum(stat_walk(part + ((long long)n * nsplit * G + g) * 3, G,
+  const StatSums a = stat_warp_sum(stat_walk<8>(part + ((long long)n * nsplit * G + g) * 3, G,
                                              rank * GN_THREADS + threadIdx.x, GN_WIDE_CLUSTER * GN_THREADS, nsplit));
   if ((threadIdx.x & 31) == 0) { s_w[warp][0] = a.n; s_w[warp][1] = a.s1; s_w[warp][2] = a.s2; }
   __syncthreads();

@@ -196,7 +196,8 @@ class UNet(nn.Module):
         if x.is_cuda and not x.is_contiguous():
             x = x.contiguous()  # the input staging kernel reads a dense NCDHW tensor
         skips = [self._run(self.down_list[0], x)]
-        plain = not self.checkpointing and type(self)._run is UNet._run and "_run" not in self.__dict__
+        plain = (torch.is_grad_enabled() and not self.checkpointing and type(self)._run is UNet._run
+                 and "_run" not in self.__dict__)
         for i in range(1, self.layers + 1):
             block, reader = self.down_list[i], self.up_list[self.layers - i]
             if not (plain and isinstance(block, Down) and isinstance(reader, Up) and reader.reads_skip_only()):

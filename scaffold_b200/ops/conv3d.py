@@ -129,6 +129,7 @@ class _PackCache:
     def __init__(self):
         self._key = None
         self._w_ref = None    # the parameter these copies were made of
+        self._listed = False  # in _PACK_REGISTRY as that parameter's
         self._real = {}       # source signature -> real channels per source
         self._tap_swap = 0    # tap-axis exchange the packs were made with (sharded runs, see Conv3d._tap_swap)
         self._vals = {}
@@ -140,11 +141,12 @@ class _PackCache:
         # strides / tap exchange: the same parameter may be read tap-transposed (sharded runs) or directly
         if tap_swap is not None:
             self._tap_swap = int(tap_swap)
-        if isinstance(w, torch.nn.Parameter) and (self._w_ref is None or self._w_ref() is not w):
+        if (self._w_ref is None or self._w_ref() is not w) and isinstance(w, torch.nn.Parameter):
             # another parameter than the copies were made of (a copied module, load_state_dict(assign=True)), whatever
             # its address and version
             self._w_ref = weakref.ref(w)
             self._key = None
+            self._listed = False
             _PACK_GENERATION[0] += 1
         key = (w.data_ptr(), w._version, w.device, weights_epoch(w), tuple(w.stride()), self._tap_swap)
         if key != self._key:
@@ -159,9 +161,9 @@ class _PackCache:
         kernel launch, so a step packs each weight once.
         """
         self._sync(w, tap_swap)
-        if self._w_ref is not None and self not in _PACK_REGISTRY:  # first use, or the first one of a copied module
+        if not self._listed and self._w_ref is not None:  # first use, or the first one of a copied module
             _PACK_REGISTRY.add(self)
-            _PACK_GENERATION[0] += 1
+            self._listed = True
         sig = tuple(src_c)
         name = kind + ("_kd" if kd else "")
         if (name, sig) not in self._fresh:

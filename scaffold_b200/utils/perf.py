@@ -61,6 +61,12 @@ def end_code_region(name: str) -> None:
         nv.range_pop()
 
 
+def count_region(name: str, seconds: float) -> None:
+    """One visit of a region that the caller has timed itself (no NVTX range)."""
+    _totals[name] += seconds
+    _counts[name] += 1
+
+
 @contextmanager
 def region(name: str):
     begin_code_region(name)
