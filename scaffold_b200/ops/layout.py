@@ -106,15 +106,15 @@ def _autograd_accumulates(ctx, param) -> bool:
     return False
 
 
-def direct_grad_target(param, ctx):
+def direct_grad_target(param, ctx=None):
     """The flat-buffer gradient view of ``param`` when the kernels may accumulate into it directly, else None. ``ctx`` is
-    the autograd node in whose backward pass this is asked."""
+    the autograd node in whose backward pass this is asked; without one nothing is known of the pass."""
     if not getattr(param, FLAT_GRAD_ATTR, False) or param._backward_hooks:
         return None  # a hook on the parameter wants to see its gradient: autograd's own accumulation
     g = param.grad
     if g is None or g.dtype != torch.float32 or not g.is_contiguous() or g.shape != param.shape:
         return None
-    return g if _autograd_accumulates(ctx, param) else None
+    return g if ctx is None or _autograd_accumulates(ctx, param) else None
 
 
 def add_grad_written_listener(fn) -> None:
