@@ -19,7 +19,7 @@ from ..ops.layout import AMP_DTYPE
 from ..ops.optim import FusedClipAdam
 from ..parallel.ddp import GradReducer
 from ..utils.perf import region
-from .step_graph import StepGraphs
+from .step_graph import StepGraphs, remember_functions
 
 
 class TrainEngine:
@@ -171,3 +171,6 @@ class TrainEngine:
         else:
             dice = L.hard_dice_reference(logits.float(), masks, self.n_classes, self.spatial)
         return loss, dice
+
+
+remember_functions(TrainEngine)

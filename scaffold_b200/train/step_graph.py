@@ -62,12 +62,21 @@ _MODULES = (UNet, unet.DoubleConv, unet.Down, unet.Up, unet.OutConv, unet._First
 _ENGINE_STEPS = ("to_device", "_autocast", "forward_loss", "_eval_pass")
 
 
-def _functions(engine) -> list:
+def _functions(engine_type) -> list:
     """The functions that a pass runs, wherever they could be replaced for all instances."""
-    return [t.forward for t in _MODULES] + [getattr(type(engine), n) for n in _ENGINE_STEPS] + [
+    return [t.forward for t in _MODULES] + [getattr(engine_type, n) for n in _ENGINE_STEPS] + [
         UNet.forward_padded_logits, UNet.features, UNet._run, unet.Down.forward_with_skip, unet.Down._after_pool,
         c3.Conv3d.forward_padded, c3.Conv3d._cuda_forward, ck.conv_same, ck.conv_wgrad, ck.convT_fwd, ck.convT_dgrad,
         losses.segmentation_loss_fused, losses.hard_dice_fused]
+
+
+def remember_functions(engine_type) -> None:
+    """Called where the engine is defined: a pass with other functions than these is not captured. (One that, say, reads
+    a value on the host ends a capture with an error that torch's allocator does not quite recover from.)"""
+    _OWN_FUNCTIONS[:] = _functions(engine_type)
+
+
+_OWN_FUNCTIONS: list = []
 
 
 def _replaced_steps(engine) -> bool:
@@ -97,7 +106,6 @@ class _Fingerprint:
         self._known = all(type(m) in _MODULES and m._compiled_call_impl is None
                           and not any(isinstance(getattr(type(m), n, None), FunctionType) for n in m.__dict__)
                           for m in modules)
-        self._code = _functions(engine)
         self._settings = self._read(engine)
 
     @staticmethod
@@ -121,7 +129,7 @@ class _Fingerprint:
         if ([p.data_ptr() for p in ps] != self._ptrs or [p.requires_grad for p in ps] != self._needs
                 or any([p._backward_hooks or p._post_accumulate_grad_hooks for p in ps])):
             return False
-        return self._settings == self._read(engine) and self._code == _functions(engine)
+        return self._settings == self._read(engine) and _functions(type(engine)) == _OWN_FUNCTIONS
 
 
 class _Pass:

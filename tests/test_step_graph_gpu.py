@@ -201,8 +201,10 @@ def test_a_failed_capture_leaves_no_copies_marked_fresh(monkeypatch):
         ordinary(self, *args)
         raise RuntimeError("out of memory, say")
 
+    from scaffold_b200.train import step_graph as sg
     with monkeypatch.context() as m:
         m.setattr(type(a), "forward_loss", failing)
+        m.setattr(sg, "_OWN_FUNCTIONS", sg._functions(type(a)))
         stream = torch.cuda.current_stream()
         assert a._graphs.get(a, *batch, train=True) is None
         assert torch.cuda.current_stream() == stream
@@ -468,19 +470,23 @@ def test_a_copied_engine_starts_without_captured_passes():
 
 
 @pytest.mark.parametrize("train", [True, False])
-def test_a_pass_that_reads_a_value_on_the_host_stays_uncaptured(train, monkeypatch):
-    """The runtime refuses the synchronisation and ends the capture; the engine goes on with ordinary passes."""
+def test_a_pass_that_reads_a_value_on_the_host_is_never_captured(train, monkeypatch):
+    """A capture would end with an error there. A function put in the engine's own place on the class could do so."""
     a, b = _engine(True), _engine(False)
     ordinary = type(a).forward_loss
+    seen = []
 
     def reading(self, *args):
         out = ordinary(self, *args)
-        float(out[0].detach())
+        seen.append(float(out[0].detach()))
         return out
-    monkeypatch.setattr(type(a), "forward_loss", reading)
-    stream = torch.cuda.current_stream()
-    for i in range(6):
-        batch = _batch(i)
-        got, want = (e.step(*batch) if train else e.eval_step(*batch)[0] for e in (a, b))
-        assert torch.equal(got, want) and torch.cuda.current_stream() == stream, i
-    assert not _captured(a) and torch.equal(a.flat.data, b.flat.data)
+    with monkeypatch.context() as m:
+        m.setattr(type(a), "forward_loss", reading)
+        for i in range(6):
+            batch = _batch(i)
+            got, want = (e.step(*batch) if train else e.eval_step(*batch)[0] for e in (a, b))
+            assert torch.equal(got, want) and not _captured(a) and len(seen) == 2 * (i + 1)
+    for i in range(4):
+        got, want = (e.step(*_batch(i)) if train else e.eval_step(*_batch(i))[0] for e in (a, b))
+        assert torch.equal(got, want)
+    assert _captured(a) and torch.equal(a.flat.data, b.flat.data)
