@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(256) pack_convT_kernel(const float* __restrict
   __syncthreads();
   if (fwd) {
 #pragma unroll 8
-  for (int i = threadIdx.x; i < PK_T * PK_T * 8; i += 256) {
+    for (int i = threadIdx.x; i < PK_T * PK_T * 8; i += 256) {
       const int ci = i % PK_T, co = (i / PK_T) % PK_T, tap = i / (PK_T * PK_T);
       if (ci0 + ci < cin && co < nco)
         fwd[((long long)tap * cout + co0 + co) * cin + ci0 + ci] = t[ci * PT_LD + co * 8 + tap];
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(256) pack_convT_kernel(const float* __restrict
   }
   if (dgrad) {
 #pragma unroll 8
-  for (int i = threadIdx.x; i < PK_T * PK_T * 8; i += 256) {
+    for (int i = threadIdx.x; i < PK_T * PK_T * 8; i += 256) {
       const int co = i % PK_T, ci = (i / PK_T) % PK_T, tap = i / (PK_T * PK_T);
       if (ci < nci && co < nco)
         dgrad[((long long)(tap >> 1) * cin_pad + ci0 + ci) * (2 * cout) + (tap & 1) * cout + co0 + co] =

@@ -219,10 +219,10 @@ __global__ void __launch_bounds__(256) maxpool2_bwd_idx_kernel(const __nv_bfloat
   }
 }
 
-// zero the planes a floor-mode pool never reads (odd extents), or copy `add` there. One thread per 8 channels of a voxel: as one thread per
-// voxel with 2-byte stores, 2 x 11 x 15 x 19 voxels of 256 channels took 67 us.
-__global__ void __launch_bounds__(256) maxpool2_bwd_tail_kernel(__nv_bfloat16* gx,
-                                                                const __nv_bfloat16* __restrict__ add, int N, int D, int H, int W, int C) {
+// zero the planes a floor-mode pool never reads (odd extents), or copy `add` there. One thread per 8 channels of a
+// voxel: as one thread per voxel with 2-byte stores, 2 x 11 x 15 x 19 voxels of 256 channels took 67 us.
+__global__ void __launch_bounds__(256) maxpool2_bwd_tail_kernel(__nv_bfloat16* gx, const __nv_bfloat16* __restrict__ add,
+                                                                int N, int D, int H, int W, int C) {
   const int C8 = C / 8;
   const long long total = (long long)N * D * H * W * C8;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
