@@ -1,8 +1,7 @@
 """CUDA graphs of the training and validation passes of a :class:`TrainEngine`.
 
-A step of a small network is bound by its launches: at scale 5 (32 cubed, base width 64) some 200 launches cost about
-25 us of host time each while the kernels need 1.4 ms together, and even at scale 7 the gaps between launches are
-4 % of the step. After a few ordinary passes over batches of one shape the engine therefore captures that pass and
+A step of a small network is bound by its launches: at scale 5 (32 cubed, base width 64) an ordinary step takes 4.2 ms
+and a replayed one 1.0, and even at scale 7 and base width 32 the gaps between launches are 3 % of the step. After a few ordinary passes over batches of one shape the engine therefore captures that pass and
 replays it: one graph for forward and loss, one for backward (so that the loss can be copied to the host between the
 two). The optimizer's update, whose learning rate and step count change from step to step, stays outside.
 
@@ -11,8 +10,9 @@ at has changed: the same parameters at the same addresses, the same modules with
 them (see :class:`_Fingerprint`). Otherwise the ordinary pass runs. The batch is copied into the graph's own buffers,
 the results out of them, so inputs may live anywhere and results are the caller's to keep.
 
-Limits: batches whose widest feature map is at most ``MAX_MAP_BYTES`` (2 x 128 cubed x 64 channels), since the graph
-keeps the memory of one pass's activations and larger batches gain less than 1 %; at most ``MAX_SHAPES`` batch shapes
+Limits: batches whose widest feature map is at most ``MAX_MAP_BYTES``, since the graph keeps the memory of one pass's
+activations (2 x 128 cubed x 64 channels gains 1.0 to 1.7 % for 7.4 GB, 2 x 160 cubed 1.0 to 1.8 % for 14.4 GB, 256
+cubed nothing for 29.5 GB; the limit stands above the first); at most ``MAX_SHAPES`` batch shapes
 per engine, and ``1 / MEMORY_SHARE`` of the device's memory. The memory is given back with the engine, when a pass is
 found out of date, and when an ordinary pass of the engine runs out of memory.
 """
@@ -72,11 +72,21 @@ def _functions(engine_type) -> list:
 
 def remember_functions(engine_type) -> None:
     """Called where the engine is defined: a pass with other functions than these is not captured. (One that, say, reads
-    a value on the host ends a capture with an error that torch's allocator does not quite recover from.)"""
+    a value on the host ends a capture with an error, see ``_capture_failed``.)"""
     _OWN_FUNCTIONS[:] = _functions(engine_type)
 
 
 _OWN_FUNCTIONS: list = []
+
+
+def _capture_failed(device, rng_state) -> None:
+    """An error of the runtime inside a capture leaves torch's generator of the device in its capture state, where every
+    later use of it raises: it gets a state of its own again, the one from before the capture."""
+    torch.cuda.synchronize(device)
+    index = torch.cuda.current_device() if device.index is None else device.index
+    fresh = torch.Generator(device=device)
+    fresh.set_state(rng_state)
+    torch.cuda.default_generators[index].graphsafe_set_state(fresh)
 
 
 def _replaced_steps(engine) -> bool:
@@ -295,6 +305,7 @@ class StepGraphs:
         if not probe.holds(engine):  # hooks are set, or a module is not one of the model's own: look again later
             self._passes[key] = 0
             return None
+        rng_state = torch.cuda.get_rng_state(engine.device)
         try:
             # (the caller's stream is current again whatever ends a capture)
             with _CAPTURES, torch.cuda.stream(torch.cuda.current_stream()):
@@ -307,7 +318,7 @@ class StepGraphs:
             logging.getLogger("scaffold").warning("the %s pass stays uncaptured: %s", "training" if train else
                                                   "validation", str(exc).splitlines()[0])
             self._passes[key] = new = None
-            torch.cuda.synchronize()
+            _capture_failed(engine.device, rng_state)
         return self._passes[key]
 
     def release(self) -> bool:

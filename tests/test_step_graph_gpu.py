@@ -490,3 +490,33 @@ def test_a_pass_that_reads_a_value_on_the_host_is_never_captured(train, monkeypa
         got, want = (e.step(*_batch(i)) if train else e.eval_step(*_batch(i))[0] for e in (a, b))
         assert torch.equal(got, want)
     assert _captured(a) and torch.equal(a.flat.data, b.flat.data)
+
+
+def test_an_error_of_the_runtime_inside_a_capture_leaves_the_device_usable(monkeypatch):
+    """The stream, the random numbers, the allocator and later captures (the synchronisation is refused, nothing runs)."""
+    from scaffold_b200.train import step_graph as sg
+    a, b = _engine(True), _engine(False)
+    for i in range(2):
+        a.step(*_batch(i)), b.step(*_batch(i))
+    ordinary = type(a).forward_loss
+
+    def reading(self, *args):
+        out = ordinary(self, *args)
+        float(out[0].detach())
+        return out
+    torch.cuda.manual_seed(7)
+    want = torch.rand(5, device="cuda"), torch.rand(5, device="cuda")
+    torch.cuda.manual_seed(7)
+    got = [torch.rand(5, device="cuda")]
+    stream = torch.cuda.current_stream()
+    with monkeypatch.context() as m:
+        m.setattr(type(a), "forward_loss", reading)
+        m.setattr(sg, "_OWN_FUNCTIONS", sg._functions(type(a)))
+        assert torch.equal(a.step(*_batch(2)), b.step(*_batch(2)))
+    assert torch.cuda.current_stream() == stream and not _captured(a)
+    got.append(torch.rand(5, device="cuda"))
+    assert all(torch.equal(g, w) for g, w in zip(got, want))
+    torch.cuda.empty_cache()
+    for i in range(5):   # another shape is still captured
+        assert torch.equal(a.step(*_batch(i, n=1)), b.step(*_batch(i, n=1)))
+    assert len(_captured(a)) == 1 and torch.equal(a.flat.data, b.flat.data)
